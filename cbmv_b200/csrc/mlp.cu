@@ -1,6 +1,6 @@
 // BF16 tensor-core kernels of the learned matching-probability classifier
 // (the MLP surrogate of the reference's random forest, test.py:603-620):
-// a general C = A * B^T GEMM on tcgen05 used by the trainer.
+// a general C = A * B^T GEMM on tcgen05, and the trainer's two kernels.
 //
 // Every CTA computes a 128-row x N tile: the K dimension streams through
 // shared memory in 64-wide, 128-byte-swizzled chunks (umma.cuh), one thread
@@ -128,193 +128,542 @@ extern "C" int cbmv_gemm_bf16(const uint16_t* A, const uint16_t* B, float* C, in
 }
 
 // ====================================================================
-// MLP: 20 -> 128 -> 128 -> 64 -> 1, ReLU, sigmoid output.
+// Training: 20 -> 128 -> 128 -> 64 -> 1, GELU or ReLU, sigmoid output.
 // Parameter vector (float32, host order):
 //   cap[20] mu[20] inv_sd[20]        input transform x' = (min(x,cap)-mu)*inv_sd
 //   W1[128x20] b1[128] W2[128x128] b2[128] W3[64x128] b3[64] w4[64] b4[1]
-// Training keeps float32 master weights (Adam) and bfloat16 copies for the
-// tensor cores: W1b [128x64] (K zero-padded), W2b, W3b, and the transposes
-// W1T [64x128], W2T, W3T [128x64] used by the input-gradient GEMMs.
+// float32 master weights (Adam), bfloat16 GEMM operands, float32
+// accumulation.
+//
+// Two launches.  A batch of 8192 is 1.3 GFLOP on 0.7 MB of samples, so
+// nothing but latency bounds it: as 24 launches with every intermediate in
+// HBM it took 7.99 ms, 6.5 of it in the bias gradients (one block, one
+// thread per column walking the whole batch) and 1.3 in GEMMs whose one or
+// two CTAs staged the batch as their K dimension.
+//
+// mlp_train_kernel runs forward and backward of 128-sample tiles; the
+// activations of a tile never leave the SM between layers:
+//   shared memory  the bf16 weights (64 KB), the tile's X0, A1, A2 and dS3;
+//                  dS2 and dS1 take the place of A2 and A1 once the MMAs that
+//                  read those have completed
+//   tensor memory  the accumulator [128 x 128] and the f16 arguments of the
+//                  two 128-wide activations (what their derivatives need)
+// The input gradients contract over a layer's outputs by reading the same
+// K-major weight tiles as MN-major operands (umma.cuh, sw128_desc_mn).  The
+// bias gradients are column sums of the float32 deltas, reduced over a
+// warp's 32 rows by a 31-step exchange per 32 columns.
+//
+// mlp_wgrad_kernel forms the weight gradients, contractions over the batch,
+// from the operand tiles the first kernel stored as they were (bulk copies
+// both ways, swizzle included): eight CTAs own a 64 x 64 block of dW1, dW2
+// or dW3^T each and stream the tiles through a ring of stages.  A block is
+// one accumulator chain in sample order: partial sums in the first kernel
+// would be quicker (33 us in all at 8192) but move the gradients by the
+// rounding of a single chain, 6e-5 relative at 32768.  It is bound by what
+// one SM takes in, 32 KB per tile at 0.44 us.
+// Measured, forward and backward of one batch: 34 us at 128 samples, 59 us
+// at 8192 (7.99 ms before), 156 us at 32768.
+// All sums have a fixed order, so a batch gives the same gradients every time.
 // ====================================================================
 namespace cbmv {
 namespace {
 
+constexpr int kTrainThreads = 256;  // two threads per tile row, each half of the columns
+// a CTA's share of the sums over the samples: db1, db2, db3, dw4, db4, loss
+constexpr int kSums = kH1 + kH2 + 2 * kH3 + 2;
 
-#define GS(i, n) for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += (int64_t)gridDim.x * blockDim.x)
+// shared memory: the operand tiles of one 128-sample tile, in the order
+// they are stored for the weight gradients, then the weights
+constexpr uint32_t kAtom = 128 * 128;  // one SW128 atom of 128 rows x 64 columns
+constexpr uint32_t kTX0 = 0, kTA1 = kTX0 + kAtom, kTA2 = kTA1 + 2 * kAtom, kTD3 = kTA2 + 2 * kAtom,
+                   kTW1 = kTD3 + kAtom, kTW2 = kTW1 + kAtom, kTW3 = kTW2 + 2 * kAtom, kTEnd = kTW3 + kAtom;
+constexpr size_t kSmTrain = 1024 + kTEnd;
+// the stored image of a tile: X0, A1, A2, dS3, dS2, dS1
+constexpr uint32_t kID2 = kTD3 + kAtom, kID1 = kID2 + 2 * kAtom, kImage = kID1 + 2 * kAtom;
+// tensor-memory columns
+constexpr uint32_t kCAcc = 0, kCS1 = 128, kCS2 = 192, kTrainCols = 256;
 
-// raw features [B,20] -> normalised bf16 [B,64] (zero padded) and its transpose [64,B]
-__global__ void mlp_prep_kernel(const float* __restrict__ X, int B, const float* __restrict__ P,
-                                uint16_t* __restrict__ X0, uint16_t* __restrict__ X0T) {
-  GS(t, (int64_t)B * kK1) {
-    const int b = (int)(t / kK1), k = (int)(t % kK1);
-    float v = 0.0f;
-    if (k < kF) v = (fminf(X[(int64_t)b * kF + k], P[k]) - P[kF + k]) * P[2 * kF + k];
-    const uint16_t h = to_bf16(v);
-    X0[t] = h;
-    X0T[(int64_t)k * B + b] = h;
-  }
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+  const __nv_bfloat162 x = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&x);
 }
 
-// S = Z + b; A = act(S) as bf16 [B,N] and [N,B]; Af = act(S) float (optional)
-__global__ void mlp_bias_act_kernel(const float* __restrict__ Z, const float* __restrict__ bias, int B,
-                                    int N, int act, float* __restrict__ S, uint16_t* __restrict__ A,
-                                    uint16_t* __restrict__ AT, float* __restrict__ Af) {
-  GS(t, (int64_t)B * N) {
-    const int b = (int)(t / N), n = (int)(t % N);
-    const float s = Z[t] + bias[n];
-    S[t] = s;
-    const float a = act_t(act, s, nullptr);
-    if (A) A[t] = to_bf16(a);
-    if (AT) AT[(int64_t)n * B + b] = to_bf16(a);
-    if (Af) Af[t] = a;
-  }
+// eight consecutive float32 weights -> one 16-byte chunk of a K-major tile
+__device__ __forceinline__ void stage8(unsigned char* dst, const float* __restrict__ src) {
+  const float4 a = __ldg(reinterpret_cast<const float4*>(src)), b = __ldg(reinterpret_cast<const float4*>(src) + 1);
+  *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
 }
 
-// output layer, loss and the first backward step, one warp per sample:
-// z = A3 . w4 + b4, p = sigmoid(z), loss_i = BCE; dz = (p - y) / B;
-// dS3 = dz * w4 * act'(S3) -> bf16 [B,64] and [64,B]; per-sample dz and
-// dz*A3 kept for the (ordered) reductions of dw4 / db4.
-__global__ void mlp_head_kernel(const float* __restrict__ A3f, const float* __restrict__ S3,
-                                const float* __restrict__ y, const float* __restrict__ P, int B, int act,
-                                float* __restrict__ loss_i, float* __restrict__ dz,
-                                float* __restrict__ dw4_i, uint16_t* __restrict__ dS3,
-                                uint16_t* __restrict__ dS3T, float* __restrict__ dS3f) {
-  const int lane = threadIdx.x & 31;
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < B; b += warps) {
-    const float* a = A3f + (int64_t)b * kH3;
-    float z = a[lane] * P[kOffW4 + lane] + a[lane + 32] * P[kOffW4 + lane + 32];
-    for (int o = 16; o; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-    z += P[kOffB4];
-    const float p = 1.0f / (1.0f + expf(-z));
-    const float yy = y[b];
-    // BCE with logits, stable form
-    const float l = fmaxf(z, 0.0f) - z * yy + log1pf(expf(-fabsf(z)));
-    const float g = (p - yy) / (float)B;
-    if (lane == 0) {
-      loss_i[b] = l / (float)B;
-      dz[b] = g;
-    }
-    for (int k = lane; k < kH3; k += 32) {
-      float dg;
-      act_t(act, S3[(int64_t)b * kH3 + k], &dg);
-      const float d = g * P[kOffW4 + k] * dg;
-      dS3[(int64_t)b * kH3 + k] = to_bf16(d);
-      dS3T[(int64_t)k * B + b] = to_bf16(d);
-      dS3f[(int64_t)b * kH3 + k] = d;
-      dw4_i[(int64_t)b * kH3 + k] = g * a[k];
-    }
+// The activation of two pre-activations as bf16, and in *s what its
+// derivative needs, as two f16 values: the GELU's argument, the ReLU's 0/1.
+template <int ACT>
+__device__ __forceinline__ uint32_t train_act(float a, float b, uint32_t* s, float2* f = nullptr) {
+  float2 v;
+  __half2 arg;
+  if (ACT == CBMV_ACT_GELU) {
+    arg = gelu_arg(a, b);
+    v = __half22float2(gelu_f16x2(arg));
+  } else {
+    v = make_float2(a > 0.0f ? a : 0.0f, b > 0.0f ? b : 0.0f);
+    arg = __floats2half2_rn(a > 0.0f ? 1.0f : 0.0f, b > 0.0f ? 1.0f : 0.0f);
   }
+  *s = *reinterpret_cast<const uint32_t*>(&arg);
+  if (f) *f = v;
+  return pack_bf16(v.x, v.y);
 }
 
-// dS = dA * act'(S) -> bf16 [B,N], [N,B] and float [B,N]
-__global__ void mlp_dact_kernel(const float* __restrict__ dA, const float* __restrict__ S, int B, int N, int act,
-                                 uint16_t* __restrict__ dS, uint16_t* __restrict__ dST,
-                                 float* __restrict__ dSf) {
-  GS(t, (int64_t)B * N) {
-    const int b = (int)(t / N), n = (int)(t % N);
-    float dg;
-    act_t(act, S[t], &dg);
-    const float d = dA[t] * dg;
-    dS[t] = to_bf16(d);
-    dST[(int64_t)n * B + b] = to_bf16(d);
-    dSf[t] = d;
-  }
+template <int ACT>
+__device__ __forceinline__ float2 train_grad(uint32_t s) {
+  const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&s));
+  return ACT == CBMV_ACT_GELU ? make_float2(gelu_grad(x.x), gelu_grad(x.y)) : x;
 }
 
-// column sums of a float [B,N] matrix in a fixed order (deterministic):
-// out[n] = sum over b of M[b,n]; one thread per column, sequential over b
-// in 8 interleaved partial sums added in order.
-__global__ void mlp_colsum_kernel(const float* __restrict__ M, int B, int N, float* __restrict__ out) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int b = 0; b < B; b += 8)
+// Sums over the warp's lanes of 32 values each: lane l receives the sum of
+// v[l].  Every step exchanges one half of the remaining values (31 shuffles).
+__device__ __forceinline__ float warp_colsum(float (&v)[32], int lane) {
 #pragma unroll
-    for (int j = 0; j < 8; j++)
-      if (b + j < B) s[j] += M[(int64_t)(b + j) * N + n];
-  out[n] = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+  for (int o = 16; o; o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < o; i++) {
+      const float send = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  return v[0];
 }
 
-// Adam on float32 masters from the gathered gradient vector g (same order
-// as the parameters, norm part excluded), then refresh the bf16 copies.
-__global__ void mlp_adam_kernel(float* __restrict__ P, float* __restrict__ m, float* __restrict__ v,
-                                const float* __restrict__ g, float lr, float b1, float b2, float eps,
-                                float bc1, float bc2, float wd) {
-  GS(i, (int64_t)(kNParams - kNormN)) {
-    const int j = (int)i + kNormN;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const bool is_weight = (j >= kOffW1 && j < kOffB1) || (j >= kOffW2 && j < kOffB2) ||
-                           (j >= kOffW3 && j < kOffB3) || (j >= kOffW4 && j < kOffB4);
-    float p = P[j];
-    if (is_weight) p -= lr * wd * p;
-    P[j] = p - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+template <int ACT>
+__global__ void __launch_bounds__(kTrainThreads, 1)
+    mlp_train_kernel(const float* __restrict__ X, const float* __restrict__ y, const float* __restrict__ P, int B,
+                     unsigned char* __restrict__ images, float* __restrict__ sums, int* __restrict__ status) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  __shared__ float s_nrm[kNormN], s_b1[kH1], s_b2[kH2], s_b3[kH3], s_w4[kH3];
+  __shared__ float s_b4;
+  __shared__ float s_red[4][kSums];
+  __shared__ uint64_t bar;
+  __shared__ uint32_t tmem_base;
+  const int tid = threadIdx.x, lane = tid & 31, quad = (tid >> 5) & 3, half = tid >> 7, row = tid & 127;
+
+  if (tid < 32) umma::tmem_alloc(&tmem_base, kTrainCols);
+  if (tid == 0) umma::mbar_init(&bar, 1);
+  // weights, K-major; columns of X0 and W1 beyond the 20 features are zero
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  for (int q = tid; q < kH1 * 4; q += kTrainThreads) {
+    const int r = q >> 2, k = (q & 3) * 8;
+    unsigned char* dst = base + kTW1 + umma::sw128_offset(128, r, k);
+    if (k + 8 <= kF) {
+      stage8(dst, P + kOffW1 + r * kF + k);
+    } else {
+      const float* w = P + kOffW1 + r * kF + k;
+      *reinterpret_cast<uint4*>(dst) = k < kF ? make_uint4(pack_bf16(w[0], w[1]), pack_bf16(w[2], w[3]), 0u, 0u) : zero;
+    }
   }
+  for (int q = tid; q < kH2 * 16; q += kTrainThreads) {
+    const int r = q >> 4, k = (q & 15) * 8;
+    stage8(base + kTW2 + umma::sw128_offset(128, r, k), P + kOffW2 + r * kH1 + k);
+  }
+  for (int q = tid; q < kH3 * 16; q += kTrainThreads) {
+    const int r = q >> 4, k = (q & 15) * 8;
+    stage8(base + kTW3 + umma::sw128_offset(64, r, k), P + kOffW3 + r * kH2 + k);
+  }
+  for (int j = 4 * half; j < 4 * half + 4; j++)
+    if (j >= 4) *reinterpret_cast<uint4*>(base + kTX0 + umma::sw128_offset(128, row, 8 * j)) = zero;
+  if (tid < kNormN) s_nrm[tid] = P[tid];
+  if (tid < kH1) s_b1[tid] = P[kOffB1 + tid];
+  if (tid < kH2) s_b2[tid] = P[kOffB2 + tid];
+  if (tid < kH3) s_b3[tid] = P[kOffB3 + tid];
+  if (tid < kH3) s_w4[tid] = P[kOffW4 + tid];
+  if (tid == 0) s_b4 = P[kOffB4];
+  umma::fence_async_smem();
+  umma::tc_fence_before();
+  __syncthreads();
+  umma::tc_fence_after();
+
+  const uint32_t tm = tmem_base, tlane = tm + ((uint32_t)(quad * 32) << 16);
+  const uint32_t sb = umma::smem_u32(base);
+  const int r7s = (row & 7) << 4;
+  // 16-byte chunk holding columns c .. c+7 of this thread's row of a 128-row tile
+  auto chunk = [&](uint32_t tile, int c) {
+    return reinterpret_cast<uint4*>(base + tile + (c >> 6) * kAtom + (row >> 3) * 1024 + (row & 7) * 128 +
+                                    ((((c & 63) >> 3) << 4) ^ r7s));
+  };
+  uint32_t phase = 0;
+  bool ok = true;
+  auto handoff = [&]() {  // the threads' shared- and tensor-memory accesses before the next MMAs
+    umma::fence_async_smem();
+    umma::tc_fence_before();
+    __syncthreads();
+    umma::tc_fence_after();
+  };
+  // the leader waits for the MMAs, another warp's first thread for its stores
+  // to have read the tiles that are overwritten next
+  constexpr int kStorer = 32;
+  auto wait = [&]() {
+    if (tid == kStorer) umma::bulk_wait_read();
+    const int r = __syncthreads_and(tid == 0 ? umma::mbar_wait(&bar, phase, kWaitLimit) : 1);
+    phase ^= 1u;
+    umma::tc_fence_after();
+    return r != 0;
+  };
+  // column sums of this CTA's tiles (warp `quad` of either half): db1 and
+  // db2 columns 64*half + 32*i + lane, db3 and dw4 column 32*half + lane
+  float db1[2] = {0, 0}, db2[2] = {0, 0}, db3 = 0.0f, dw4 = 0.0f, db4 = 0.0f, loss = 0.0f;
+
+  // hidden layer: accumulator + bias -> activation (bf16 tile) and its argument (f16, tensor memory)
+  auto forward = [&](const float* bias, uint32_t tile, uint32_t args) {
+#pragma unroll
+    for (int c0 = 0; c0 < 64; c0 += 16) {
+      const int c = 64 * half + c0;
+      uint32_t v[16], s[8], a[8];
+      umma::tmem_ld16_issue(tlane + kCAcc + c, v);
+      umma::tmem_ld16_wait(v);
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+        a[i] = train_act<ACT>(__uint_as_float(v[2 * i]) + bias[c + 2 * i], __uint_as_float(v[2 * i + 1]) + bias[c + 2 * i + 1], &s[i]);
+      *chunk(tile, c) = make_uint4(a[0], a[1], a[2], a[3]);
+      *chunk(tile, c + 8) = make_uint4(a[4], a[5], a[6], a[7]);
+      umma::tmem_st8(tlane + args + c / 2, s);
+    }
+    umma::tmem_st_wait();
+  };
+  // dS = dA * act'(S) -> bf16 tile, and its column sums
+  auto backward = [&](uint32_t tile, uint32_t args, float* db) {
+#pragma unroll
+    for (int b = 0; b < 2; b++) {
+      const int c = 64 * half + 32 * b;
+      float d[32];
+      {
+        uint32_t v[32], s[16];
+        umma::tmem_ld32_issue(tlane + kCAcc + c, v);
+        umma::tmem_ld16_issue(tlane + args + c / 2, s);
+        umma::tmem_ld32_wait(v);
+        umma::tmem_ld16_wait(s);
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+          const float2 g = train_grad<ACT>(s[i]);
+          d[2 * i] = __uint_as_float(v[2 * i]) * g.x;
+          d[2 * i + 1] = __uint_as_float(v[2 * i + 1]) * g.y;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        *chunk(tile, c + 8 * i) = make_uint4(pack_bf16(d[8 * i], d[8 * i + 1]), pack_bf16(d[8 * i + 2], d[8 * i + 3]),
+                                             pack_bf16(d[8 * i + 4], d[8 * i + 5]), pack_bf16(d[8 * i + 6], d[8 * i + 7]));
+      db[b] += warp_colsum(d, lane);
+    }
+  };
+  constexpr uint32_t id128 = umma::idesc_bf16(128, 128), id64 = umma::idesc_bf16(128, 64);
+
+  const int tiles = B / 128;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    unsigned char* image = images + (size_t)tile * kImage;
+    auto store = [&](uint32_t at, uint32_t smem, uint32_t bytes) {
+      if (tid == kStorer) umma::bulk_store(image + at, sb + smem, bytes);
+    };
+    const int64_t b = (int64_t)tile * 128 + row;
+    float x[16];
+    const int k0 = 16 * half;
+#pragma unroll
+    for (int k = 0; k < 16; k++) x[k] = k0 + k < kF ? X[b * kF + k0 + k] : 0.0f;
+    const float yy = y[b];
+    // 1. normalised bf16 inputs
+#pragma unroll
+    for (int k = 0; k < 16; k++)
+      if (k0 + k < kF) x[k] = (fminf(x[k], s_nrm[k0 + k]) - s_nrm[kF + k0 + k]) * s_nrm[2 * kF + k0 + k];
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+      *chunk(kTX0, k0 + 8 * j) = make_uint4(pack_bf16(x[8 * j], x[8 * j + 1]), pack_bf16(x[8 * j + 2], x[8 * j + 3]),
+                                            pack_bf16(x[8 * j + 4], x[8 * j + 5]), pack_bf16(x[8 * j + 6], x[8 * j + 7]));
+    handoff();
+    store(kTX0, kTX0, kAtom);
+    // 2. layer 1 (K = 32)
+    if (tid == 0) {
+      const uint64_t da = umma::sw128_desc(sb + kTX0), dw = umma::sw128_desc(sb + kTW1);
+      umma::mma_bf16(tm + kCAcc, da, dw, id128, false);
+      umma::mma_bf16(tm + kCAcc, da + 2, dw + 2, id128, true);
+      umma::mma_commit(&bar);
+    }
+    if (!(ok = wait())) break;
+    forward(s_b1, kTA1, kCS1);
+    handoff();
+    store(kTA1, kTA1, 2 * kAtom);
+    // 3. layer 2
+    if (tid == 0) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const uint32_t o = (k >> 2) * kAtom + (k & 3) * 32;
+        umma::mma_bf16(tm + kCAcc, umma::sw128_desc(sb + kTA1 + o), umma::sw128_desc(sb + kTW2 + o), id128, k > 0);
+      }
+      umma::mma_commit(&bar);
+    }
+    if (!(ok = wait())) break;
+    forward(s_b2, kTA2, kCS2);
+    handoff();
+    store(kTA2, kTA2, 2 * kAtom);
+    // 4. layer 3
+    if (tid == 0) {
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        umma::mma_bf16(tm + kCAcc, umma::sw128_desc(sb + kTA2 + (k >> 2) * kAtom + (k & 3) * 32),
+                       umma::sw128_desc(sb + kTW3 + (k >> 2) * 64 * 128 + (k & 3) * 32), id64, k > 0);
+      umma::mma_commit(&bar);
+    }
+    if (!(ok = wait())) break;
+    // 5. output layer, loss, dS3 = dz w4 act'(S3).  Both threads of a row
+    //    form the whole dot product (in the order of a 32-lane exchange over
+    //    fma(a[l], w[l], a[l+32] w[l+32])); each forms its half of dS3.
+    {
+      float t[32], a3[32];
+      uint32_t s3[16];
+#pragma unroll
+      for (int p = 1; p >= 0; p--)
+#pragma unroll
+        for (int c = 0; c < 32; c += 16) {
+          uint32_t v[16];
+          umma::tmem_ld16_issue(tlane + kCAcc + 32 * p + c, v);
+          umma::tmem_ld16_wait(v);
+#pragma unroll
+          for (int i = 0; i < 8; i++) {
+            const int n = 32 * p + c + 2 * i;
+            uint32_t s;
+            float2 f;
+            train_act<ACT>(__uint_as_float(v[2 * i]) + s_b3[n], __uint_as_float(v[2 * i + 1]) + s_b3[n + 1], &s, &f);
+            t[c + 2 * i] = p == 1 ? f.x * s_w4[n] : fmaf(f.x, s_w4[n], t[c + 2 * i]);
+            t[c + 2 * i + 1] = p == 1 ? f.y * s_w4[n + 1] : fmaf(f.y, s_w4[n + 1], t[c + 2 * i + 1]);
+            if (p == half) {
+              s3[(c + 2 * i) / 2] = s;
+              a3[c + 2 * i] = f.x;
+              a3[c + 2 * i + 1] = f.y;
+            }
+          }
+        }
+#pragma unroll
+      for (int o = 16; o; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < o; i++) t[i] += t[i + o];
+      const float z = t[0] + s_b4;
+      const float prob = 1.0f / (1.0f + expf(-z));
+      // BCE with logits, stable form
+      const float l = fmaxf(z, 0.0f) - z * yy + log1pf(expf(-fabsf(z)));
+      const float g = (prob - yy) / (float)B;
+      loss += l / (float)B;
+      db4 += g;
+      float d[32];
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        const float2 dg = train_grad<ACT>(s3[i]);
+        d[2 * i] = g * s_w4[32 * half + 2 * i] * dg.x;
+        d[2 * i + 1] = g * s_w4[32 * half + 2 * i + 1] * dg.y;
+        a3[2 * i] *= g;
+        a3[2 * i + 1] *= g;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        *chunk(kTD3, 32 * half + 8 * i) =
+            make_uint4(pack_bf16(d[8 * i], d[8 * i + 1]), pack_bf16(d[8 * i + 2], d[8 * i + 3]),
+                       pack_bf16(d[8 * i + 4], d[8 * i + 5]), pack_bf16(d[8 * i + 6], d[8 * i + 7]));
+      db3 += warp_colsum(d, lane);
+      dw4 += warp_colsum(a3, lane);
+    }
+    handoff();
+    store(kTD3, kTD3, kAtom);
+    // 6. dA2 = dS3 W3; dS2 takes A2's place
+    if (tid == 0) {
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        umma::mma_bf16(tm + kCAcc, umma::sw128_desc(sb + kTD3 + 32 * k), umma::sw128_desc_mn(sb + kTW3 + 2048 * k, 64),
+                       id128 | umma::kTransposeB, k > 0);
+      umma::mma_commit(&bar);
+    }
+    if (!(ok = wait())) break;
+    backward(kTA2, kCS2, db2);
+    handoff();
+    store(kID2, kTA2, 2 * kAtom);
+    // 7. dA1 = dS2 W2; dS1 takes A1's place
+    if (tid == 0) {
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        umma::mma_bf16(tm + kCAcc, umma::sw128_desc(sb + kTA2 + (k >> 2) * kAtom + (k & 3) * 32),
+                       umma::sw128_desc_mn(sb + kTW2 + 2048 * k, 128), id128 | umma::kTransposeB, k > 0);
+      umma::mma_commit(&bar);
+    }
+    if (!(ok = wait())) break;
+    backward(kTA1, kCS1, db1);
+    handoff();
+    store(kID1, kTA1, 2 * kAtom);
+  }
+  if (!ok && tid == 0) {
+    // a wait gave up: record it and let the MMAs in flight finish (bounded)
+    // before their memory is freed
+    atomicExch(status, 1);
+    umma::mbar_wait(&bar, phase ^ 1u, kWaitLimit);
+  }
+  // the four warps of a half cover the tile's rows: their column sums added in order
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    s_red[quad][64 * half + 32 * i + lane] = db1[i];
+    s_red[quad][kH1 + 64 * half + 32 * i + lane] = db2[i];
+  }
+  s_red[quad][kH1 + kH2 + 32 * half + lane] = db3;
+  s_red[quad][kH1 + kH2 + kH3 + 32 * half + lane] = dw4;
+  if (half == 0) {
+    for (int k = 16; k; k >>= 1) {
+      db4 += __shfl_xor_sync(0xffffffffu, db4, k);
+      loss += __shfl_xor_sync(0xffffffffu, loss, k);
+    }
+    if (lane == 0) {
+      s_red[quad][kSums - 2] = db4;
+      s_red[quad][kSums - 1] = loss;
+    }
+  }
+  if (tid == kStorer) umma::bulk_wait();
+  umma::tc_fence_before();
+  __syncthreads();
+  for (int i = tid; i < kSums; i += kTrainThreads)
+    sums[(size_t)blockIdx.x * kSums + i] = ((s_red[0][i] + s_red[1][i]) + s_red[2][i]) + s_red[3][i];
+  if (tid < 32) umma::tmem_dealloc(tm, kTrainCols);
 }
 
-__global__ void mlp_pack_kernel(const float* __restrict__ P, uint16_t* __restrict__ W1b,
-                                uint16_t* __restrict__ W1T, uint16_t* __restrict__ W2b,
-                                uint16_t* __restrict__ W2T, uint16_t* __restrict__ W3b,
-                                uint16_t* __restrict__ W3T) {
-  GS(t, (int64_t)kH1 * kK1) {  // W1b [128,64], W1T [64,128]
-    const int n = (int)(t / kK1), k = (int)(t % kK1);
-    const uint16_t h = to_bf16(k < kF ? P[kOffW1 + n * kF + k] : 0.0f);
-    W1b[t] = h;
-    W1T[(int64_t)k * kH1 + n] = h;
+struct AdamStep {
+  float *P, *m, *v;
+  float lr, b1, b2, eps, bc1, bc2, wd;
+};
+
+// What becomes of gradient g of parameter j (kNormN <= j < kNParams): Adam
+// with decoupled weight decay (STEP) or a place in `grads`.
+template <bool STEP>
+__device__ __forceinline__ void finish_grad(const AdamStep& a, float* __restrict__ grads, int j, float g) {
+  const int i = j - kNormN;
+  if (!STEP) {
+    grads[i] = g;
+    return;
   }
-  GS(t, (int64_t)kH2 * kH1) {  // W2b [128,128], W2T
-    const int n = (int)(t / kH1), k = (int)(t % kH1);
-    const uint16_t h = to_bf16(P[kOffW2 + t]);
-    W2b[t] = h;
-    W2T[(int64_t)k * kH2 + n] = h;
-  }
-  GS(t, (int64_t)kH3 * kH2) {  // W3b [64,128], W3T [128,64]
-    const int n = (int)(t / kH2), k = (int)(t % kH2);
-    const uint16_t h = to_bf16(P[kOffW3 + t]);
-    W3b[t] = h;
-    W3T[(int64_t)k * kH3 + n] = h;
-  }
+  const float mi = a.b1 * a.m[i] + (1.0f - a.b1) * g;
+  const float vi = a.b2 * a.v[i] + (1.0f - a.b2) * g * g;
+  a.m[i] = mi;
+  a.v[i] = vi;
+  const bool is_weight = (j >= kOffW1 && j < kOffB1) || (j >= kOffW2 && j < kOffB2) ||
+                         (j >= kOffW3 && j < kOffB3) || (j >= kOffW4 && j < kOffB4);
+  float p = a.P[j];
+  if (is_weight) p -= a.lr * a.wd * p;
+  a.P[j] = p - a.lr * (mi / a.bc1) / (sqrtf(vi / a.bc2) + a.eps);
 }
 
-// gather the gradients into parameter order (dW1 [128,64] -> first 20 cols,
-// dW3 arrives transposed [128,64]).
-__global__ void mlp_gather_grad_kernel(const float* __restrict__ dW1, const float* __restrict__ db1,
-                                       const float* __restrict__ dW2, const float* __restrict__ db2,
-                                       const float* __restrict__ dW3T, const float* __restrict__ db3,
-                                       const float* __restrict__ dw4, const float* __restrict__ db4,
-                                       float* __restrict__ g) {
-  GS(i, (int64_t)(kNParams - kNormN)) {
-    const int j = (int)i + kNormN;
-    float v;
-    if (j < kOffB1) { const int q = j - kOffW1; v = dW1[(q / kF) * kK1 + q % kF]; }
-    else if (j < kOffW2) v = db1[j - kOffB1];
-    else if (j < kOffB2) v = dW2[j - kOffW2];
-    else if (j < kOffW3) v = db2[j - kOffB2];
-    else if (j < kOffB3) { const int q = j - kOffW3; v = dW3T[(q % kH2) * kH3 + q / kH2]; }
-    else if (j < kOffW4) v = db3[j - kOffB3];
-    else if (j < kOffB4) v = dw4[j - kOffW4];
-    else v = db4[0];
-    g[i] = v;
+constexpr int kWgradThreads = 128, kWgradStages = 6, kWgradBlocks = 8;
+constexpr uint32_t kStageBytes = 2 * kAtom;
+constexpr size_t kSmWgrad = 1024 + kWgradStages * kStageBytes;
+constexpr int kSumBlocks = (kSums + kWgradThreads - 1) / kWgradThreads;
+
+// Blocks 0..7: a 64 x 64 block of a weight gradient each, D[m][n] = sum over
+// the samples of U[b][m] V[b][n] with U, V one 64-column atom of the stored
+// operands; the further blocks: the sums over the training kernel's CTAs.
+template <bool STEP>
+__global__ void __launch_bounds__(kWgradThreads, 1)
+    mlp_wgrad_kernel(const unsigned char* __restrict__ images, int tiles, const float* __restrict__ sums, int ctas,
+                     AdamStep a, float* __restrict__ grads, float* __restrict__ loss, int* __restrict__ status) {
+  const int r = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (r >= kWgradBlocks) {
+    const int i = (r - kWgradBlocks) * kWgradThreads + tid;
+    if (i >= kSums) return;
+    float g = 0.0f;
+#pragma unroll 8
+    for (int c = 0; c < ctas; c++) g += sums[(size_t)c * kSums + i];
+    if (i == kSums - 1) {
+      if (loss) *loss = g;
+      return;
+    }
+    finish_grad<STEP>(a, grads,
+                      i < kH1               ? kOffB1 + i
+                      : i < kH1 + kH2       ? kOffB2 + i - kH1
+                      : i < kH1 + kH2 + kH3 ? kOffB3 + i - kH1 - kH2
+                                            : kOffW4 + i - kH1 - kH2 - kH3,  // w4, then b4
+                      g);
+    return;
   }
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  const uint32_t sb = (umma::smem_u32(smem_raw) + 1023u) & ~1023u;
+  __shared__ uint64_t full[kWgradStages], empty[kWgradStages], done;
+  __shared__ uint32_t tmem_base;
+  __shared__ int s_fail;
+  if (tid < 32) umma::tmem_alloc(&tmem_base, 64);
+  if (tid == 0) {
+    for (int i = 0; i < kWgradStages; i++) {
+      umma::mbar_init(&full[i], 1);
+      umma::mbar_init(&empty[i], 1);
+    }
+    umma::mbar_init(&done, 1);
+    s_fail = 0;
+  }
+  umma::tc_fence_before();
+  __syncthreads();
+  umma::tc_fence_after();
+  const uint32_t tm = tmem_base;
+  const uint32_t u = r < 4 ? kID2 + (r & 1) * kAtom : r < 6 ? kTA2 + (r - 4) * kAtom : kID1 + (r - 6) * kAtom;
+  const uint32_t v = r < 4 ? kTA1 + (r >> 1) * kAtom : r < 6 ? kTD3 : kTX0;
+  if (tid == 0) {  // producer
+    for (int t = 0; t < tiles; t++) {
+      const int s = t % kWgradStages, n = t / kWgradStages;
+      if (n > 0 && !umma::mbar_wait(&empty[s], (uint32_t)(n - 1) & 1u, kWaitLimit)) {
+        s_fail = 1;
+        break;
+      }
+      const unsigned char* image = images + (size_t)t * kImage;
+      umma::mbar_expect_tx(&full[s], kStageBytes);
+      umma::bulk_load(sb + s * kStageBytes, image + u, kAtom, &full[s]);
+      umma::bulk_load(sb + s * kStageBytes + kAtom, image + v, kAtom, &full[s]);
+    }
+  } else if (tid == 32) {  // MMAs, in sample order
+    constexpr uint32_t id = umma::idesc_bf16(64, 64) | umma::kTransposeA | umma::kTransposeB;
+    bool ok = true;
+    for (int t = 0; t < tiles && ok; t++) {
+      const int s = t % kWgradStages, n = t / kWgradStages;
+      ok = umma::mbar_wait(&full[s], (uint32_t)n & 1u, kWaitLimit);
+      if (!ok) break;
+      umma::tc_fence_after();
+      const uint32_t at = sb + s * kStageBytes;
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        umma::mma_bf16(tm, umma::sw128_desc_mn(at + 2048 * k, 128), umma::sw128_desc_mn(at + kAtom + 2048 * k, 128), id,
+                       t > 0 || k > 0);
+      umma::mma_commit(&empty[s]);
+    }
+    umma::mma_commit(&done);
+    if (!umma::mbar_wait(&done, 0, kWaitLimit) || !ok) s_fail = 1;
+  }
+  __syncthreads();
+  umma::tc_fence_after();
+  if (s_fail) {
+    // record it and let the copies in flight land (bounded) before the CTA ends
+    if (tid == 0) {
+      atomicExch(status, 1);
+      for (int s = 0; s < kWgradStages && s < tiles; s++)
+        umma::mbar_wait(&full[s], (uint32_t)((tiles - 1 - s) / kWgradStages) & 1u, kWaitLimit);
+    }
+  } else {
+    // row m of a 64-row accumulator: lane m % 16 of the tensor-memory quarter m / 16
+    const int m = 16 * warp + lane;
+    for (int c = 0; c < 64; c += 16) {
+      float g[16];
+      umma::tmem_ld16(tm + ((uint32_t)(warp * 32) << 16) + c, g);
+      if (lane < 16) {
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+          const int n = c + i;
+          if (r < 4) finish_grad<STEP>(a, grads, kOffW2 + (64 * (r & 1) + m) * kH1 + 64 * (r >> 1) + n, g[i]);
+          else if (r < 6) finish_grad<STEP>(a, grads, kOffW3 + n * kH2 + 64 * (r - 4) + m, g[i]);
+          else if (n < kF) finish_grad<STEP>(a, grads, kOffW1 + (64 * (r - 6) + m) * kF + n, g[i]);
+        }
+      }
+      __syncwarp();
+    }
+  }
+  umma::tc_fence_before();
+  __syncthreads();
+  if (tid < 32) umma::tmem_dealloc(tm, 64);
 }
 
-__global__ void sum_kernel(const float* __restrict__ a, int n, float* __restrict__ out) {
-  // one warp, fixed order per lane then a fixed tree
-  float s = 0.0f;
-  for (int i = threadIdx.x; i < n; i += 32) s += a[i];
-  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (threadIdx.x == 0) *out = s;
-}
-
-}  // namespace
-}  // namespace cbmv
-
-
-namespace {
 size_t carve_mlp(cbmv_mlp* n, char* base) {
   size_t off = 0;
   auto take = [&](size_t bytes) -> void* {
@@ -323,53 +672,38 @@ size_t carve_mlp(cbmv_mlp* n, char* base) {
     off += bytes;
     return p;
   };
-  const size_t B = (size_t)n->B;
-  using namespace cbmv;
   n->P = (float*)take(sizeof(float) * kNParams);
   n->m = (float*)take(sizeof(float) * kNParams);
   n->v = (float*)take(sizeof(float) * kNParams);
-  n->g = (float*)take(sizeof(float) * kNParams);
-  n->W1b = (uint16_t*)take(2 * kH1 * kK1);
-  n->W1T = (uint16_t*)take(2 * kH1 * kK1);
-  n->W2b = (uint16_t*)take(2 * kH2 * kH1);
-  n->W2T = (uint16_t*)take(2 * kH2 * kH1);
-  n->W3b = (uint16_t*)take(2 * kH3 * kH2);
-  n->W3T = (uint16_t*)take(2 * kH3 * kH2);
-  n->X0 = (uint16_t*)take(2 * B * kK1);
-  n->X0T = (uint16_t*)take(2 * B * kK1);
-  n->A1 = (uint16_t*)take(2 * B * kH1);
-  n->A1T = (uint16_t*)take(2 * B * kH1);
-  n->A2 = (uint16_t*)take(2 * B * kH2);
-  n->A2T = (uint16_t*)take(2 * B * kH2);
-  n->dS3 = (uint16_t*)take(2 * B * kH3);
-  n->dS3T = (uint16_t*)take(2 * B * kH3);
-  n->dS2 = (uint16_t*)take(2 * B * kH2);
-  n->dS2T = (uint16_t*)take(2 * B * kH2);
-  n->dS1 = (uint16_t*)take(2 * B * kH1);
-  n->dS1T = (uint16_t*)take(2 * B * kH1);
-  n->Z = (float*)take(4 * B * 128);
-  n->S1 = (float*)take(4 * B * kH1);
-  n->S2 = (float*)take(4 * B * kH2);
-  n->S3 = (float*)take(4 * B * kH3);
-  n->A3f = (float*)take(4 * B * kH3);
-  n->dA = (float*)take(4 * B * 128);
-  n->dSf = (float*)take(4 * B * 128);
-  n->loss_i = (float*)take(4 * B);
-  n->dz = (float*)take(4 * B);
-  n->dw4_i = (float*)take(4 * B * kH3);
-  n->dW1 = (float*)take(4 * kH1 * kK1);
-  n->dW2 = (float*)take(4 * kH2 * kH1);
-  n->dW3T = (float*)take(4 * kH2 * kH3);
-  n->db1 = (float*)take(4 * kH1);
-  n->db2 = (float*)take(4 * kH2);
-  n->db3 = (float*)take(4 * kH3);
-  n->dw4 = (float*)take(4 * kH3);
-  n->db4 = (float*)take(4 * 4);
-  n->loss = (float*)take(4 * 4);
+  n->sums = (float*)take(sizeof(float) * kSums * (size_t)n->ctas);
+  n->images = (unsigned char*)take((size_t)kImage * (n->B / 128));
   n->status = (int*)take(4 * 4);
   return off + 256;
 }
+
+// Forward and backward of one batch, then Adam (STEP) or the gradients.
+template <int ACT, bool STEP>
+int launch_train(const cbmv_mlp* n, const float* X, const float* y, const AdamStep& a, float* grads, float* loss,
+                 cudaStream_t st) {
+  CBMV_CUDA(cudaFuncSetAttribute(mlp_train_kernel<ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmTrain));
+  CBMV_CUDA(cudaFuncSetAttribute(mlp_wgrad_kernel<STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmWgrad));
+  mlp_train_kernel<ACT><<<n->ctas, kTrainThreads, kSmTrain, st>>>(X, y, n->P, n->B, n->images, n->sums, n->status);
+  int rc = check_launch("mlp_train");
+  if (rc) return rc;
+  mlp_wgrad_kernel<STEP><<<kWgradBlocks + kSumBlocks, kWgradThreads, kSmWgrad, st>>>(n->images, n->B / 128, n->sums,
+                                                                                     n->ctas, a, grads, loss, n->status);
+  return check_launch("mlp_wgrad");
+}
+
+template <bool STEP>
+int mlp_batch(const cbmv_mlp* n, const float* X, const float* y, const AdamStep& a, float* grads, float* loss,
+              cudaStream_t st) {
+  return n->act == CBMV_ACT_GELU ? launch_train<CBMV_ACT_GELU, STEP>(n, X, y, a, grads, loss, st)
+                                 : launch_train<CBMV_ACT_RELU, STEP>(n, X, y, a, grads, loss, st);
+}
+
 }  // namespace
+}  // namespace cbmv
 
 using namespace cbmv;
 
@@ -379,8 +713,12 @@ extern "C" int cbmv_mlp_create(int batch, cbmv_mlp** out) {
   CBMV_REQUIRE(out, CBMV_EINVAL, "null pointer argument");
   CBMV_REQUIRE(batch >= 128 && batch % 128 == 0 && batch <= (1 << 22), CBMV_EINVAL,
                "batch must be a multiple of 128 in [128, 4194304]");
+  int dev = 0, sms = 0;
+  CBMV_CUDA(cudaGetDevice(&dev));
+  CBMV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   cbmv_mlp* n = new cbmv_mlp();
   n->B = batch;
+  n->ctas = batch / 128 < sms ? batch / 128 : sms;
   const size_t bytes = carve_mlp(n, nullptr);
   cudaError_t e = cudaMalloc(&n->mem, bytes);
   if (e != cudaSuccess) {
@@ -413,9 +751,8 @@ extern "C" int cbmv_mlp_set_params(cbmv_mlp* n, const float* host) {
   CBMV_CUDA(cudaMemset(n->m, 0, sizeof(float) * kNParams));
   CBMV_CUDA(cudaMemset(n->v, 0, sizeof(float) * kNParams));
   n->step = 0;
-  mlp_pack_kernel<<<64, 256>>>(n->P, n->W1b, n->W1T, n->W2b, n->W2T, n->W3b, n->W3T);
   CBMV_CUDA(cudaDeviceSynchronize());
-  return check_launch("mlp_pack");
+  return CBMV_OK;
 }
 
 extern "C" int cbmv_mlp_get_params(const cbmv_mlp* n, float* host) {
@@ -424,59 +761,18 @@ extern "C" int cbmv_mlp_get_params(const cbmv_mlp* n, float* host) {
   return CBMV_OK;
 }
 
-namespace {
-// forward + backward on one batch; gradients land in n->g (parameter order)
-int mlp_fwd_bwd(cbmv_mlp* n, const float* X, const float* y, cudaStream_t st) {
-  const int B = n->B;
-  const unsigned g = grid_for((int64_t)B * 128, 256);
-  int rc;
-  mlp_prep_kernel<<<g, 256, 0, st>>>(X, B, n->P, n->X0, n->X0T);
-  if ((rc = launch_gemm_bf16(n->X0, n->W1b, n->Z, B, kH1, kK1, n->status, st))) return rc;
-  mlp_bias_act_kernel<<<g, 256, 0, st>>>(n->Z, n->P + kOffB1, B, kH1, n->act, n->S1, n->A1, n->A1T, nullptr);
-  if ((rc = launch_gemm_bf16(n->A1, n->W2b, n->Z, B, kH2, kH1, n->status, st))) return rc;
-  mlp_bias_act_kernel<<<g, 256, 0, st>>>(n->Z, n->P + kOffB2, B, kH2, n->act, n->S2, n->A2, n->A2T, nullptr);
-  if ((rc = launch_gemm_bf16(n->A2, n->W3b, n->Z, B, kH3, kH2, n->status, st))) return rc;
-  mlp_bias_act_kernel<<<g, 256, 0, st>>>(n->Z, n->P + kOffB3, B, kH3, n->act, n->S3, nullptr, nullptr, n->A3f);
-  mlp_head_kernel<<<grid_for((int64_t)B * 32, 256), 256, 0, st>>>(n->A3f, n->S3, y, n->P, B, n->act, n->loss_i,
-                                                                  n->dz, n->dw4_i, n->dS3, n->dS3T, n->dSf);
-  mlp_colsum_kernel<<<1, 64, 0, st>>>(n->dw4_i, B, kH3, n->dw4);
-  mlp_colsum_kernel<<<1, 64, 0, st>>>(n->dz, B, 1, n->db4);
-  mlp_colsum_kernel<<<1, 64, 0, st>>>(n->dSf, B, kH3, n->db3);
-  sum_kernel<<<1, 32, 0, st>>>(n->loss_i, B, n->loss);
-  // layer 3: dW3^T = A2^T dS3, dA2 = dS3 W3
-  if ((rc = launch_gemm_bf16(n->A2T, n->dS3T, n->dW3T, kH2, kH3, B, n->status, st))) return rc;
-  if ((rc = launch_gemm_bf16(n->dS3, n->W3T, n->dA, B, kH2, kH3, n->status, st))) return rc;
-  mlp_dact_kernel<<<g, 256, 0, st>>>(n->dA, n->S2, B, kH2, n->act, n->dS2, n->dS2T, n->dSf);
-  mlp_colsum_kernel<<<1, 128, 0, st>>>(n->dSf, B, kH2, n->db2);
-  // layer 2: dW2 = dS2^T A1, dA1 = dS2 W2
-  if ((rc = launch_gemm_bf16(n->dS2T, n->A1T, n->dW2, kH2, kH1, B, n->status, st))) return rc;
-  if ((rc = launch_gemm_bf16(n->dS2, n->W2T, n->dA, B, kH1, kH2, n->status, st))) return rc;
-  mlp_dact_kernel<<<g, 256, 0, st>>>(n->dA, n->S1, B, kH1, n->act, n->dS1, n->dS1T, n->dSf);
-  mlp_colsum_kernel<<<1, 128, 0, st>>>(n->dSf, B, kH1, n->db1);
-  // layer 1: dW1 = dS1^T X0
-  if ((rc = launch_gemm_bf16(n->dS1T, n->X0T, n->dW1, kH1, kK1, B, n->status, st))) return rc;
-  mlp_gather_grad_kernel<<<64, 256, 0, st>>>(n->dW1, n->db1, n->dW2, n->db2, n->dW3T, n->db3, n->dw4,
-                                             n->db4, n->g);
-  return check_launch("mlp_fwd_bwd");
-}
-}  // namespace
-
 // One Adam step on a batch of B samples: X float32 [B,20] raw CBMV features,
 // y float32 [B] labels (1 = correct match), device memory.  loss (device,
 // may be NULL) receives the batch's mean binary cross-entropy.
 extern "C" int cbmv_mlp_train_step(cbmv_mlp* n, const float* X, const float* y, float lr,
                                    float weight_decay, float* loss, void* stream) {
   CBMV_REQUIRE(n && X && y, CBMV_EINVAL, "null pointer argument");
-  cudaStream_t st = as_stream(stream);
-  int rc = mlp_fwd_bwd(n, X, y, st);
-  if (rc) return rc;
-  n->step++;
   const float b1 = 0.9f, b2 = 0.999f;
-  const float bc1 = 1.0f - powf(b1, (float)n->step), bc2 = 1.0f - powf(b2, (float)n->step);
-  mlp_adam_kernel<<<64, 256, 0, st>>>(n->P, n->m, n->v, n->g, lr, b1, b2, 1e-8f, bc1, bc2, weight_decay);
-  mlp_pack_kernel<<<64, 256, 0, st>>>(n->P, n->W1b, n->W1T, n->W2b, n->W2T, n->W3b, n->W3T);
-  if (loss) CBMV_CUDA(cudaMemcpyAsync(loss, n->loss, sizeof(float), cudaMemcpyDeviceToDevice, st));
-  return check_launch("mlp_train_step");
+  const float step = (float)(n->step + 1);
+  const AdamStep a{n->P, n->m, n->v, lr, b1, b2, 1e-8f, 1.0f - powf(b1, step), 1.0f - powf(b2, step), weight_decay};
+  const int rc = mlp_batch<true>(n, X, y, a, nullptr, loss, as_stream(stream));
+  if (rc == CBMV_OK) n->step++;
+  return rc;
 }
 
 // Gradients of the batch loss without an update (for checking): grads
@@ -485,12 +781,7 @@ extern "C" int cbmv_mlp_train_step(cbmv_mlp* n, const float* X, const float* y, 
 extern "C" int cbmv_mlp_gradients(cbmv_mlp* n, const float* X, const float* y, float* grads, float* loss,
                                   void* stream) {
   CBMV_REQUIRE(n && X && y && grads, CBMV_EINVAL, "null pointer argument");
-  cudaStream_t st = as_stream(stream);
-  int rc = mlp_fwd_bwd(n, X, y, st);
-  if (rc) return rc;
-  CBMV_CUDA(cudaMemcpyAsync(grads, n->g, sizeof(float) * (kNParams - kNormN), cudaMemcpyDeviceToDevice, st));
-  if (loss) CBMV_CUDA(cudaMemcpyAsync(loss, n->loss, sizeof(float), cudaMemcpyDeviceToDevice, st));
-  return CBMV_OK;
+  return mlp_batch<false>(n, X, y, AdamStep{}, grads, loss, as_stream(stream));
 }
 
 extern "C" int cbmv_mlp_set_activation(cbmv_mlp* n, int act) {

@@ -20,12 +20,6 @@ constexpr int kOffW1 = kNormN, kOffB1 = kOffW1 + kH1 * kF, kOffW2 = kOffB1 + kH1
               kOffB2 = kOffW2 + kH2 * kH1, kOffW3 = kOffB2 + kH2, kOffB3 = kOffW3 + kH3 * kH2,
               kOffW4 = kOffB3 + kH3, kOffB4 = kOffW4 + kH3, kNParams = kOffB4 + 1;
 
-// ReLU and its derivative (0 at x = 0)
-__device__ __forceinline__ float relu_t(float x, float* drelu) {
-  if (drelu) *drelu = x > 0.0f ? 1.0f : 0.0f;
-  return x > 0.0f ? x : 0.0f;
-}
-
 // The network's GELU, x * Phi(x) with Phi the standard normal CDF, computed
 // in half-precision (binary16) arithmetic (the fused inference stores its
 // activations as f16 anyway), on the packed half-precision FMA pipe,
@@ -55,31 +49,33 @@ __device__ __forceinline__ __half f16_bits(uint16_t b) { return __ushort_as_half
 constexpr uint16_t kGB0Bits = 0x3ebf, kGB1Bits = 0xbd30, kGB2Bits = 0x3b1c;  // 0.373046875, -0.04296875, 0.00238037109375
 __device__ __forceinline__ __nv_bfloat16 bf16_bits(uint16_t b) { return __ushort_as_bfloat16(b); }
 
-// GELU of x (float32 in, its f16 rounding used) and, for the backward pass,
-// the derivative of the smooth function it approximates at that point:
-// q + x (p + 2 u p'(u)) where 0 < x p + 0.5 < 1, else q (0 or 1), in float32.
-__device__ __forceinline__ float gelu_t(float x, float* dgelu) {
-  const __half xh = __float2half_rn(fminf(fmaxf(x, -65504.0f), 65504.0f));  // saturated, as the fused kernel's cvt
-  const __half u = __hmul(xh, xh);
-  __half p = __hfma(f16_bits(kG2Bits), u, f16_bits(kG1Bits));
-  p = __hfma(p, u, f16_bits(kG0Bits));
-  const __half q = __hfma_sat(xh, p, __float2half_rn(0.5f));
-  const float g = __half2float(__hmul(xh, q));
-  if (dgelu) {
-    const float xf = __half2float(xh), uf = xf * xf;
-    const float g0 = __half2float(f16_bits(kG0Bits)), g1 = __half2float(f16_bits(kG1Bits)),
-                g2 = __half2float(f16_bits(kG2Bits));
-    const float pf = fmaf(fmaf(g2, uf, g1), uf, g0);
-    const float qr = fmaf(xf, pf, 0.5f);
-    const float dq = fmaf(2.0f * uf, fmaf(2.0f * g2, uf, g1), pf);  // d(x p(x^2))/dx
-    *dgelu = qr <= 0.0f ? 0.0f : qr >= 1.0f ? 1.0f : fmaf(xf, dq, qr);
-  }
-  return g;
+// The f16 rounding of two pre-activations, saturated to +-65504 as the
+// fused inference kernel converts them.
+__device__ __forceinline__ __half2 gelu_arg(float a, float b) {
+  return __floats2half2_rn(fminf(fmaxf(a, -65504.0f), 65504.0f), fminf(fmaxf(b, -65504.0f), 65504.0f));
 }
 
-// the network's activation (cbmv_mlp_set_activation) and its derivative
-__device__ __forceinline__ float act_t(int act, float x, float* d) {
-  return act == CBMV_ACT_GELU ? gelu_t(x, d) : relu_t(x, d);
+// GELU of two f16 arguments.
+__device__ __forceinline__ __half2 gelu_f16x2(__half2 x) {
+  const __half2 g0 = __half2half2(f16_bits(kG0Bits)), g1 = __half2half2(f16_bits(kG1Bits)),
+                g2 = __half2half2(f16_bits(kG2Bits));
+  const __half2 u = __hmul2(x, x);
+  __half2 p = __hfma2(g2, u, g1);
+  p = __hfma2(p, u, g0);
+  return __hmul2(x, __hfma2_sat(x, p, __float2half2_rn(0.5f)));
+}
+
+// For the backward pass: the derivative of the smooth function the GELU
+// approximates, q + x (p + 2 u p'(u)) where 0 < x p + 0.5 < 1, else q (0 or
+// 1), in float32 at the f16 argument x.
+__device__ __forceinline__ float gelu_grad(float xf) {
+  const float uf = xf * xf;
+  const float g0 = __half2float(f16_bits(kG0Bits)), g1 = __half2float(f16_bits(kG1Bits)),
+              g2 = __half2float(f16_bits(kG2Bits));
+  const float pf = fmaf(fmaf(g2, uf, g1), uf, g0);
+  const float qr = fmaf(xf, pf, 0.5f);
+  const float dq = fmaf(2.0f * uf, fmaf(2.0f * g2, uf, g1), pf);  // d(x p(x^2))/dx
+  return qr <= 0.0f ? 0.0f : qr >= 1.0f ? 1.0f : fmaf(xf, dq, qr);
 }
 
 __device__ __forceinline__ uint16_t to_bf16(float x) {
@@ -96,11 +92,10 @@ __device__ __forceinline__ uint16_t to_f16(float x) {
 struct cbmv_mlp {
   int B = 0;
   void* mem = nullptr;
-  float *P, *m, *v, *g;                  // params, Adam moments, gathered grads
-  uint16_t *W1b, *W1T, *W2b, *W2T, *W3b, *W3T;
-  uint16_t *X0, *X0T, *A1, *A1T, *A2, *A2T, *dS3, *dS3T, *dS2, *dS2T, *dS1, *dS1T;
-  float *Z, *S1, *S2, *S3, *A3f, *dA, *dSf, *loss_i, *dz, *dw4_i;
-  float *dW1, *dW2, *dW3T, *db1, *db2, *db3, *dw4, *db4, *loss;
+  float *P, *m, *v;      // params, Adam moments
+  int ctas = 0;          // CTAs of the training kernel
+  float* sums = nullptr; // their shares of the bias gradients and the loss
+  unsigned char* images = nullptr;  // the batch's operand tiles for the weight gradients
   int* status;
   int step = 0;
   int act = CBMV_ACT_RELU;    // hidden-layer activation

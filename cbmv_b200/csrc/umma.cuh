@@ -58,6 +58,25 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
          | ((uint32_t)(M >> 4) << 24);   // M / 16
 }
 
+// Instruction descriptor bits for operands read transposed (MN-major).
+constexpr uint32_t kTransposeA = 1u << 15, kTransposeB = 1u << 16;
+
+// The same tile as sw128_desc read the other way round: the tile's R rows
+// are the contraction dimension and its columns the operand's M or N.  An
+// MN-major SW128 operand is 128-byte rows of 64 consecutive M/N elements,
+// eight K rows per 1024-byte group (stride byte offset), further 64-element
+// column blocks one atom (R * 128 bytes) apart (leading byte offset).  Each
+// 16-wide K step advances the start address by 16 rows, 2048 bytes.
+__device__ __forceinline__ uint64_t sw128_desc_mn(uint32_t smem_addr, int R) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr >> 4) & 0x3FFFu);   // start address
+  d |= (uint64_t)(((uint32_t)R * 128u) >> 4) << 16;  // leading byte offset
+  d |= (uint64_t)(1024u >> 4) << 32;               // stride byte offset
+  d |= (uint64_t)1 << 46;                          // descriptor version (sm_100)
+  d |= (uint64_t)2 << 61;                          // SWIZZLE_128B
+  return d;
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -80,6 +99,26 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
   }
   return false;
 }
+
+// Arms `bar` for one phase of `bytes` bytes of bulk loads.
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+// Untiled bulk copies, 16-byte aligned addresses and sizes: global -> shared
+// (completes on `bar`), shared -> global (one bulk group each).
+__device__ __forceinline__ void bulk_load(uint32_t dst_smem, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_smem),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+__device__ __forceinline__ void bulk_store(void* dst, uint32_t src_smem, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src_smem), "r"(bytes)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+// This thread's stores have read shared memory / have completed.
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 __device__ __forceinline__ void fence_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -164,6 +203,15 @@ __device__ __forceinline__ void tmem_ld16_wait(uint32_t* r) {
                :
                : "memory");
 }
+
+// 32 lanes x 8 columns of 32-bit data written to tensor memory (row lane
+// base + i, columns col .. col+7); tmem_st_wait before they are read back
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // 32 lanes x 32 columns of 32-bit data: lane i of the warp receives row
 // (lane base + i), columns col .. col+31; tmem_ld32_wait must follow before
