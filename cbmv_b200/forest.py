@@ -20,9 +20,9 @@ per-tree offsets) and is what both the GPU packer and the tests use:
   value1[n]      class-1 fraction (sklearn keeps both; 1 - value0 is not
                  always bit-equal to it)
 
-pack() turns it into the device layout (csrc/rf.cu): every tree cut into
-two-level blocks of 32 bytes -- one DRAM/L2 sector -- so one load serves two
-levels of a walk:
+pack() turns it into the layout cbmv_forest_create takes (which lays it out
+again for the walk, csrc/rf.cuh): every tree cut into two-level blocks of 32
+bytes:
   words 0-2  float32 thresholds of the block's root (node 0) and of its two
              children (nodes 1, 2); each is t32 = the largest float32 <= the
              float64 threshold (for a float32 x, x <= thr64 exactly when
@@ -31,9 +31,8 @@ levels of a walk:
   words 4-7  the four grandchildren: node 1's left/right, node 2's left/right;
              bit 31 set = leaf index, clear = index of the block rooted there.
 A leaf at node 0 keeps its leaf index in word 4, a leaf at node 1 in word 4,
-a leaf at node 2 in word 6.  Blocks are numbered breadth-first per tree, so
-the top blocks of every tree form a prefix that can be staged in shared
-memory.  Leaf values are float64 (class-0, class-1) fractions.
+a leaf at node 2 in word 6.  Blocks are numbered breadth-first per tree.
+Leaf values are float64 (class-0, class-1) fractions.
 """
 import numpy as np
 
@@ -118,7 +117,7 @@ class FlatForest:
                    int(z["n_features"]), z["value1"] if "value1" in z.files else None)
 
     def pack(self):
-        """Device layout (see the module docstring): blocks uint32 [NB, 8],
+        """The upload layout (see the module docstring): blocks uint32 [NB, 8],
         leaf values float64 [K, 2], per-tree block offsets int32 [T+1], and
         leaf_node int32 [K] (each leaf's sklearn node id within its tree)."""
         if self.n_features >= LEAF_FEATURE:

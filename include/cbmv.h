@@ -177,8 +177,8 @@ int cbmv_features(const double* census, const double* ncc, const double* sob, co
 
 typedef struct cbmv_forest cbmv_forest;
 
-/* Uploads a packed forest (HOST pointers; layout in cbmv_b200/forest.py and
- * csrc/rf.cuh): blocks uint32 [n_blocks,8] -- each 32-byte block holds two
+/* Uploads a packed forest (HOST pointers; layout in cbmv_b200/forest.py):
+ * blocks uint32 [n_blocks,8] -- each 32-byte block holds two
  * tree levels -- leaf_value float64 [n_leaves,2] (class-0 and class-1
  * fractions), tree_offsets int32 [n_trees+1] (first block of each tree).
  * The structure is validated on the host (CBMV_EINVAL on any index out of
