@@ -76,55 +76,6 @@ __global__ void census_desc_kernel(const uint8_t* __restrict__ img, int64_t H, i
   }
 }
 
-template <class T>
-__global__ void census_cost_kernel(const ulonglong2* __restrict__ dl,
-                                   const ulonglong2* __restrict__ dr, int64_t H, int64_t W, int D,
-                                   int w, int layout, T* __restrict__ out) {
-  const VolCoord c = vol_coord(layout, W, D);
-  if (!c.in) return;
-  const int wc = w / 2;
-  const int64_t i = c.y - wc, j = c.x - wc;
-  double v = kRandMax;
-  // matchers.cpp:312-316: rows i < H-w, cols j < W-w, d < min(D, j+1)
-  if (i >= 0 && i < H - w && j >= 0 && j < W - w && c.d <= j) {
-    const ulonglong2 a = dl[c.y * W + c.x];
-    const ulonglong2 b = dr[c.y * W + c.x - c.d];
-    v = (double)(__popcll(a.x ^ b.x) + __popcll(a.y ^ b.y));
-  }
-  out[vol_index(layout, c.y, c.x, c.d, H, W, D)] = cvt_out<T>(v);
-}
-
-// The float32 [H,W,D] census volume of the learned path, without a
-// division per element: a CTA owns 16 columns of one row and 128
-// disparities (lane = d), so the left descriptor is one broadcast load per
-// column and the right one a coalesced run along d.  Same values and
-// sentinels as census_cost_kernel (the popcount sum is exact in float32).
-__global__ void __launch_bounds__(128) census_cost_hwd_f32_kernel(const ulonglong2* __restrict__ dl,
-                                                                  const ulonglong2* __restrict__ dr, int64_t H,
-                                                                  int64_t W, int D, int w, float* __restrict__ out) {
-  const int64_t y = blockIdx.y;
-  const int64_t x0 = (int64_t)blockIdx.x * 16;
-  const int d = blockIdx.z * 128 + threadIdx.x;
-  if (d >= D) return;
-  const int wc = w / 2;
-  const int64_t i = y - wc;
-  const bool row_ok = i >= 0 && i < H - w;
-#pragma unroll 4
-  for (int s = 0; s < 16; s++) {
-    const int64_t x = x0 + s;
-    if (x >= W) break;
-    const int64_t j = x - wc;
-    float v = kRandMaxF;
-    // matchers.cpp:312-316: rows i < H-w, cols j < W-w, d < min(D, j+1)
-    if (row_ok && j >= 0 && j < W - w && d <= j) {
-      const ulonglong2 a = dl[y * W + x];
-      const ulonglong2 b = dr[y * W + x - d];
-      v = (float)(__popcll(a.x ^ b.x) + __popcll(a.y ^ b.y));
-    }
-    out[(y * W + x) * D + d] = v;
-  }
-}
-
 // ------------------------------------------------------------------- NCC
 // Window sum A and 1/sqrt(w^2 B - A^2) (matchers.cpp:115-131); B is exact.
 __global__ void ncc_stats_kernel(const uint8_t* __restrict__ img, int64_t H, int64_t W, int w,
@@ -274,117 +225,220 @@ __global__ void zsad_cost_kernel(const uint8_t* __restrict__ L, const uint8_t* _
   out[vol_index(layout, c.y, c.x, c.d, H, W, D)] = cvt_out<T>(v);
 }
 
-// ------------------------------------------- float32 strip matchers
-// The three window matchers for the learned classifier's float32 volumes
-// ([H,W,D]): a warp owns 32 disparities (lane = d) of one row and walks a
-// strip of SX columns; the window's L and R columns sit in a register ring,
-// so each step loads one new column of each (L uniform across the warp, R
-// at x - d per lane).  Window sums are exact integers (SAD of Sobel
-// responses, sum of L*R, ZSAD as sum |25 (L - R) - (sum L - sum R)| / 25), so
-// the float32 result equals the rounding of the reference's value (its
-// float64 ZSAD chain differs from the exact quotient by ~1e-15 relative).
-// Validity and sentinels as in the reference kernels above.
-enum StripMode { kStripNcc = 0, kStripSadSob = 1, kStripZsad = 2 };
-constexpr int kStripX = 16;
+// ------------------------------------------------------- strip matchers
+// The cost volumes of census (any window) and of the default windows of NCC
+// (3), SAD-on-Sobel (5) and ZSAD (5), float32 or float64, either layout.  A
+// warp owns 32 disparities (lane = d) of a strip of XS columns of one row
+// and walks the strip, so a step adds one window column:
+//   - the window columns the warp meets are staged once in its own shared
+//     memory (XS + w - 1 left columns, 31 more right ones), clamped to the
+//     image there, so a step is one or two shared-memory loads without
+//     address arithmetic or bounds tests;
+//   - NCC packs a column's three bytes in a word (one dp4a per column); SAD
+//     and ZSAD in float32 keep a running window sum over a register ring of
+//     columns; ZSAD in float64 follows the reference's order of operations
+//     on a ring of doubles;
+//   - [D,H,W] outputs are turned around in a shared-memory tile.
+// Every window sum is an exact integer, so a float32 volume is the float32
+// rounding of the reference's value (ZSAD: of the exact quotient; the
+// reference's float64 chain differs from it by ~1e-15 relative).
+// Bound by instruction issue (census: POPC; ZSAD float64: the FP64 pipe, 75
+// additions per value, 0.21 ms of the 0.36).  At 694x554 D=128, us, before
+// in brackets (thread per value, or a strip with its columns loaded from
+// global memory at clamped 64-bit addresses):
+//                  census     NCC        SAD-Sobel  ZSAD
+//   float32 [H,W,D]  63 (93)    94 (199)   92 (282)   120 (369)
+//   float64 [H,W,D]  67 (218)   99 (670)   98 (834)   359 (932)
+//   float64 [D,H,W]             206        144        410
+// against 31 / 61 us for writing the volume.
+enum StripMode { kStripCensus, kStripNcc, kStripSadSob, kStripZsad };
+constexpr int kStripWarps = 4;
 
-template <int MODE, int WIN>
-__global__ void __launch_bounds__(128) matcher_strip_kernel(
-    const void* __restrict__ Lp, const void* __restrict__ Rp, const uint32_t* __restrict__ Al,
-    const uint32_t* __restrict__ Ar, const double* __restrict__ Cl, const double* __restrict__ Cr,
-    const double* __restrict__ ml, const double* __restrict__ mr, int64_t H, int64_t W, int D,
-    float* __restrict__ out) {
-  using Px = typename std::conditional<MODE == kStripSadSob, int32_t, uint8_t>::type;
-  const Px* L = static_cast<const Px*>(Lp);
-  const Px* R = static_cast<const Px*>(Rp);
-  constexpr int r = WIN / 2;
-  const int64_t y = blockIdx.y;
-  const int64_t x0 = (int64_t)blockIdx.x * kStripX;
-  const int d = blockIdx.z * 128 + threadIdx.x;
-  if (d >= D) return;
-  // window rows, clamped into the image (values of clamped rows are never used)
-  int64_t rowoff[WIN];
+struct StripArgs {
+  const void *L, *R;            // census descriptors, uint8 images or int32 Sobel responses
+  const uint32_t *Al, *Ar;      // NCC window sums and 1 / sqrt
+  const double *Cl, *Cr;
+  const double *ml, *mr;        // ZSAD window means (float64 volumes)
+  int64_t H, W;
+  int D, w;
+};
+
+// A column of a 5-pixel-high window of 8-bit pixels as packed 16-bit values
+// scale * pixel + bias (rows 0..4, a sixth half zero) and the pixels' sum.
+__device__ __forceinline__ uint4 zsad_column(const uint8_t* __restrict__ p, int64_t W, unsigned scale, unsigned bias) {
+  const unsigned a = p[0], b = p[W], c = p[2 * W], d = p[3 * W], e = p[4 * W];
+  return make_uint4((scale * a + bias) | (scale * b + bias) << 16, (scale * c + bias) | (scale * d + bias) << 16,
+                    scale * e + bias, a + b + c + d + e);
+}
+
+template <int MODE, class T, int LAYOUT, int XS>
+__global__ void __launch_bounds__(32 * kStripWarps) matcher_strip_kernel(StripArgs a, T* __restrict__ out) {
+  constexpr bool kF64Zsad = MODE == kStripZsad && std::is_same<T, double>::value;
+  constexpr int WIN = MODE == kStripCensus ? 1 : MODE == kStripNcc ? 3 : 5;  // window columns staged
+  constexpr int r0 = WIN / 2, NL = XS + WIN - 1, NR = NL + 31;
+  // shared memory per warp: left columns, right columns, [D,H,W] tile
+  constexpr int kLBytes = kF64Zsad ? XS * 26 * 8 : NL * (MODE == kStripNcc ? 4 : MODE == kStripSadSob ? 32 : 16);
+  constexpr int kRBytes = kF64Zsad ? 5 * NR * 8 : NR * (MODE == kStripNcc ? 4 : MODE == kStripSadSob ? 20 : 16);
+  constexpr int kTile = LAYOUT == CBMV_DHW ? 32 * (XS + 1) * (int)sizeof(T) : 0;
+  constexpr int kBytes = ((kLBytes + 15) / 16 + (kRBytes + 15) / 16 + (kTile + 15) / 16) * 16;
+  __shared__ __align__(16) unsigned char smem[kStripWarps * kBytes];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned char* sl = smem + warp * kBytes;
+  unsigned char* sr = sl + (kLBytes + 15) / 16 * 16;
+  T* tile = reinterpret_cast<T*>(sr + (kRBytes + 15) / 16 * 16);
+  const int64_t H = a.H, W = a.W, y = blockIdx.y;
+  const int D = a.D, ndb = (D + 31) / 32;
+  const int64_t unit = (int64_t)blockIdx.x * kStripWarps + warp;
+  const int64_t x0 = unit / ndb * XS;
+  const int d0 = (int)(unit % ndb) * 32, d = d0 + lane;
+  if (x0 >= W) return;
+  // the reference's valid region (matchers.cpp:168-172, 312-316, 412-423,
+  // 495-505): rows and columns r .. size - w + r - 1, d <= column index - r
+  const int r = a.w / 2;
+  const bool row_ok = y >= r && y < H - a.w + r;
+  const int64_t xend = W - a.w + r;
+  if (row_ok) {
+    const int64_t cl0 = x0 - r0, cr0 = x0 - r0 - d0 - 31, top = (y - r0) * W;
+    auto col = [&](int64_t c) { return c < 0 ? (int64_t)0 : c >= W ? W - 1 : c; };
+    if constexpr (MODE == kStripCensus) {
+      const uint4 *L = static_cast<const uint4*>(a.L) + top, *R = static_cast<const uint4*>(a.R) + top;
+      for (int i = lane; i < NL; i += 32) reinterpret_cast<uint4*>(sl)[i] = __ldg(L + col(cl0 + i));
+      for (int i = lane; i < NR; i += 32) reinterpret_cast<uint4*>(sr)[i] = __ldg(R + col(cr0 + i));
+    } else if constexpr (MODE == kStripNcc) {
+      const uint8_t *L = static_cast<const uint8_t*>(a.L) + top, *R = static_cast<const uint8_t*>(a.R) + top;
+      auto pack = [&](const uint8_t* p) { return (uint32_t)p[0] | (uint32_t)p[W] << 8 | (uint32_t)p[2 * W] << 16; };
+      for (int i = lane; i < NL; i += 32) reinterpret_cast<uint32_t*>(sl)[i] = pack(L + col(cl0 + i));
+      for (int i = lane; i < NR; i += 32) reinterpret_cast<uint32_t*>(sr)[i] = pack(R + col(cr0 + i));
+    } else if constexpr (MODE == kStripSadSob) {
+      const int32_t *L = static_cast<const int32_t*>(a.L) + top, *R = static_cast<const int32_t*>(a.R) + top;
+      for (int i = lane; i < NL; i += 32) {
+        const int32_t* p = L + col(cl0 + i);
+        reinterpret_cast<int4*>(sl)[2 * i] = make_int4(p[0], p[W], p[2 * W], p[3 * W]);
+        reinterpret_cast<int*>(sl)[8 * i + 4] = p[4 * W];
+      }
+      for (int i = lane; i < NR; i += 32) {
+        const int32_t* p = R + col(cr0 + i);
 #pragma unroll
-  for (int wh = 0; wh < WIN; wh++) {
-    int64_t yy = y - r + wh;
-    yy = yy < 0 ? 0 : (yy >= H ? H - 1 : yy);
-    rowoff[wh] = yy * W;
-  }
-  // ring slot contents, computed when the column is loaded: SAD and NCC
-  // keep the column's sum (of |SL - SR|, of L * R), ZSAD keeps 25 (L - R)
-  // per window row
-  int col[WIN];
-  int dif[MODE == kStripZsad ? WIN : 1][WIN];
-  // ZSAD: the column's sum of L minus its sum of R (the window's sum of
-  // these is sum L - sum R, exact: 25 x its mean difference)
-  int cdm[MODE == kStripZsad ? WIN : 1];
-  auto load_col = [&](int slot, int64_t c) {
-    const int64_t cl = c < 0 ? 0 : (c >= W ? W - 1 : c);
-    int64_t cr = c - d;
-    cr = cr < 0 ? 0 : (cr >= W ? W - 1 : cr);
-    int sum = 0;
+        for (int k = 0; k < 5; k++) reinterpret_cast<int*>(sr)[k * NR + i] = p[k * W];
+      }
+    } else if constexpr (!kF64Zsad) {
+      const uint8_t *L = static_cast<const uint8_t*>(a.L) + top, *R = static_cast<const uint8_t*>(a.R) + top;
+      for (int i = lane; i < NL; i += 32) reinterpret_cast<uint4*>(sl)[i] = zsad_column(L + col(cl0 + i), W, 25u, 6375u);
+      for (int i = lane; i < NR; i += 32) reinterpret_cast<uint4*>(sr)[i] = zsad_column(R + col(cr0 + i), W, 25u, 0u);
+    } else {
+      // L - mean of every window pixel, in the reference's order (row by row)
+      const uint8_t *L = static_cast<const uint8_t*>(a.L) + top, *R = static_cast<const uint8_t*>(a.R) + top;
+      for (int i = lane; i < XS * 25; i += 32) {
+        const int s = i / 25, k = i - 25 * s;
+        const int64_t x = x0 + s;
+        if (x >= r && x < xend)
+          reinterpret_cast<double*>(sl)[s * 26 + k] = __dsub_rn((double)L[(k / 5) * W + x - 2 + k % 5], a.ml[y * W + x]);
+      }
+      for (int i = lane; i < NR; i += 32) {
+        const uint8_t* p = R + col(cr0 + i);
 #pragma unroll
-    for (int wh = 0; wh < WIN; wh++) {
-      const int a = (int)__ldg(L + rowoff[wh] + cl), b = (int)__ldg(R + rowoff[wh] + cr);
-      if (MODE == kStripSadSob) sum += abs(a - b);
-      else if (MODE == kStripNcc) sum += a * b;
-      else {
-        dif[MODE == kStripZsad ? slot : 0][wh] = (WIN * WIN) * (a - b);
-        sum += a - b;
+        for (int k = 0; k < 5; k++) reinterpret_cast<double*>(sr)[k * NR + i] = (double)p[k * W];
       }
     }
-    if (MODE == kStripZsad) cdm[MODE == kStripZsad ? slot : 0] = sum;
-    col[slot] = sum;
+  }
+  __syncwarp();
+  // right column of this lane at left column index i: i + 31 - lane
+  const int ro = 31 - lane;
+  T* o = out + (y * W + x0) * D + d;
+  // window columns of the ring: the sum over the column's rows, ZSAD's
+  // packed 25 (L - R) + 6375 per row, ZSAD float64's right pixels
+  int ring[WIN] = {}, sum = 0;
+  uint32_t zr[MODE == kStripZsad && !kF64Zsad ? 15 : 1];
+  double rr[kF64Zsad ? 25 : 1];
+  auto push = [&](int i, int slot) {  // staged column i enters the window
+    if constexpr (MODE == kStripNcc) {
+      const int c = (int)__dp4a(reinterpret_cast<const uint32_t*>(sl)[i], reinterpret_cast<const uint32_t*>(sr)[i + ro], 0u);
+      sum += c - ring[slot];
+      ring[slot] = c;
+    } else if constexpr (MODE == kStripSadSob) {
+      const int4 l = reinterpret_cast<const int4*>(sl)[2 * i];
+      const int l4 = reinterpret_cast<const int*>(sl)[8 * i + 4];
+      const int* q = reinterpret_cast<const int*>(sr) + i + ro;
+      const int c = abs(l.x - q[0]) + abs(l.y - q[NR]) + abs(l.z - q[2 * NR]) + abs(l.w - q[3 * NR]) + abs(l4 - q[4 * NR]);
+      sum += c - ring[slot];
+      ring[slot] = c;
+    } else if constexpr (MODE == kStripZsad && !kF64Zsad) {
+      const uint4 l = reinterpret_cast<const uint4*>(sl)[i], q = reinterpret_cast<const uint4*>(sr)[i + ro];
+      zr[3 * slot] = l.x - q.x;  // 6375 + 25 (L - R) >= 0 in either half: no borrow between them
+      zr[3 * slot + 1] = l.y - q.y;
+      zr[3 * slot + 2] = l.z - q.z;
+      const int c = (int)(l.w - q.w);
+      sum += c - ring[slot];
+      ring[slot] = c;
+    } else if constexpr (kF64Zsad) {
+#pragma unroll
+      for (int k = 0; k < 5; k++) rr[slot * 5 + k] = reinterpret_cast<const double*>(sr)[k * NR + i + ro];
+    }
   };
+  if (row_ok && WIN > 1) {
 #pragma unroll
-  for (int j = 0; j < WIN - 1; j++) load_col(j, x0 - r + j);
-  const bool row_ok = y >= r && y < H - WIN + r;
+    for (int i = 0; i < WIN - 1; i++) push(i, i);
+  }
 #pragma unroll
-  for (int s = 0; s < kStripX; s++) {
+  for (int s = 0; s < XS; s++) {
     const int64_t x = x0 + s;
     if (x >= W) break;
-    load_col((s + WIN - 1) % WIN, x + r);
-    // ring slot (s + k) % WIN holds column x - r + k
-    float v = kRandMaxF;
-    if (row_ok && x >= d + r && x < W - WIN + r) {
-      if (MODE == kStripSadSob) {
-        int acc = 0;
+    T v = (T)kRandMax;
+    if (row_ok) {
+      if constexpr (WIN > 1) push(s + WIN - 1, (s + WIN - 1) % WIN);
+      if (x >= (int64_t)d + r && x < xend) {
+        if constexpr (MODE == kStripCensus) {
+          const uint4 l = reinterpret_cast<const uint4*>(sl)[s], q = reinterpret_cast<const uint4*>(sr)[s + ro];
+          v = (T)(__popc(l.x ^ q.x) + __popc(l.y ^ q.y) + (__popc(l.z ^ q.z) + __popc(l.w ^ q.w)));
+        } else if constexpr (MODE == kStripNcc) {
+          const int64_t pl = y * W + x, pr = pl - d;
+          const double cl = a.Cl[pl], cr = a.Cr[pr];
+          // 9 S - A_L A_R exactly (both below 2^23), then the reference's product (matchers.cpp:179, 181)
+          const double num = (double)(9 * sum - (int)(a.Al[pl] * a.Ar[pr]));
+          v = isfinite(cl) && isfinite(cr) ? (T)(-num * cl * cr) : (T)1.0;
+        } else if constexpr (MODE == kStripSadSob) {
+          v = (T)sum;
+        } else if constexpr (!kF64Zsad) {
+          // sum |X - m| over the window's 25 values X = 25 (L - R), m = sum (L - R) = 25 x their mean difference,
+          // as 2 sum max(X, m) - 50 m (the X sum to 25 m); offset by 6375 so that the packed halves are
+          // unsigned, with the five unused sixth halves counting m' each: 2 S - 60 m'
+          const unsigned m = (unsigned)(sum + 6375), m2 = m * 0x10001u;
+          unsigned S = 0;
 #pragma unroll
-        for (int k = 0; k < WIN; k++) acc += col[(s + k) % WIN];
-        v = (float)acc;
-      } else if (MODE == kStripZsad) {
-        // 25 x (mean L - mean R) over the window, exactly (the window lies
-        // inside both images here, so no column or row was clamped)
-        int m = 0;
-#pragma unroll
-        for (int k = 0; k < WIN; k++) m += cdm[MODE == kStripZsad ? (s + k) % WIN : 0];
-        unsigned acc = 0;
-#pragma unroll
-        for (int k = 0; k < WIN; k++)
-#pragma unroll
-          for (int wh = 0; wh < WIN; wh++) acc = __sad(dif[MODE == kStripZsad ? (s + k) % WIN : 0][wh], m, acc);
-        // acc < 2^24 (WIN^2 terms of at most 2 WIN^2 255) is exact in
-        // float32, and acc / WIN^2 is either an integer or more than 2^-29
-        // (relative) away from every float32 rounding midpoint, so one
-        // correctly rounded float32 division gives the float32 rounding of
-        // the exact quotient -- what rounding a float64 quotient would give
-        static_assert(WIN * WIN * WIN * WIN * 510 < (1 << 24), "ZSAD window sum exact in float32");
-        v = __fdiv_rn((float)acc, (float)(WIN * WIN));
-      } else {
-        const int64_t pl = y * W + x, pr = pl - d;
-        unsigned acc = 0;
-#pragma unroll
-        for (int k = 0; k < WIN; k++) acc += (unsigned)col[(s + k) % WIN];
-        const double cl = Cl[pl], cr = Cr[pr];
-        if (isfinite(cl) && isfinite(cr)) {
-          const unsigned long long aa = (unsigned long long)Al[pl] * (unsigned long long)Ar[pr];
-          const double num = (double)(WIN * WIN) * (double)acc - (double)aa;
-          v = (float)(-num * cl * cr);
+          for (int k = 0; k < 5; k++)  // at most 3 * 12750 per half of a column
+            S = __dp2a_lo(__vmaxu2(zr[3 * k], m2) + __vmaxu2(zr[3 * k + 1], m2) + __vmaxu2(zr[3 * k + 2], m2), 0x0101u, S);
+          // the correctly rounded quotient by 25 (Markstein's division with a correctly rounded reciprocal;
+          // equal to IEEE division for every sum a window can have, 0 .. 318,750)
+          const float acc = (float)(int)(2u * S - 60u * m);
+          constexpr float inv = 1.0f / 25.0f;
+          const float q = __fmul_rn(acc, inv);
+          v = (T)fmaf(fmaf(-q, 25.0f, acc), inv, q);
         } else {
-          v = 1.0f;
+          const double mur = a.mr[y * W + x - d];
+          const double* lm = reinterpret_cast<const double*>(sl) + s * 26;
+          double acc = 0.0;
+#pragma unroll
+          for (int wh = 0; wh < 5; wh++)
+#pragma unroll
+            for (int ww = 0; ww < 5; ww++)  // ((L - muL) - R) + muR, each step rounded as in the reference
+              acc = __dadd_rn(acc, fabs(__dadd_rn(__dsub_rn(lm[wh * 5 + ww], rr[(s + ww) % 5 * 5 + wh]), mur)));
+          v = (T)acc;
         }
       }
     }
-    out[(y * W + x) * D + d] = v;
+    if (LAYOUT == CBMV_DHW) {
+      tile[lane * (XS + 1) + s] = v;
+    } else {
+      if (d < D) *o = v;
+      o += D;
+    }
+  }
+  if (LAYOUT == CBMV_DHW) {
+    __syncwarp();
+    constexpr int kRows = 32 / XS;  // disparities written per step
+    const int64_t x = x0 + lane % XS;
+    for (int k = lane / XS; k < 32 && d0 + k < D; k += kRows)
+      if (x < W) out[((int64_t)(d0 + k) * H + y) * W + x] = tile[k * (XS + 1) + lane % XS];
   }
 }
 
@@ -434,16 +488,31 @@ int launch_census_desc(const uint8_t* img, int64_t H, int64_t W, int w, ulonglon
   return check_launch("census_desc");
 }
 
+// The strip kernels' launch; W / XS * D / 32 warps per row.
+static dim3 strip_grid(const StripArgs& a, int xs) {
+  const int64_t units = ((a.W + xs - 1) / xs) * ((a.D + 31) / 32);
+  return dim3((unsigned)((units + kStripWarps - 1) / kStripWarps), (unsigned)a.H);
+}
+
+template <int MODE, class T, int XS>
+static int launch_strip(const StripArgs& a, int layout, T* out, cudaStream_t st) {
+  const dim3 grid = strip_grid(a, XS);
+  if (layout == CBMV_HWD) matcher_strip_kernel<MODE, T, CBMV_HWD, XS><<<grid, 32 * kStripWarps, 0, st>>>(a, out);
+  else matcher_strip_kernel<MODE, T, CBMV_DHW, XS><<<grid, 32 * kStripWarps, 0, st>>>(a, out);
+  return check_launch("matcher_strip");
+}
+
 template <class T>
 int launch_census_cost(const ulonglong2* dl, const ulonglong2* dr, int64_t H, int64_t W, int D,
                        int w, int layout, T* out, cudaStream_t st) {
-  if (std::is_same<T, float>::value && layout == CBMV_HWD) {
-    const dim3 grid((unsigned)((W + 15) / 16), (unsigned)H, (unsigned)((D + 127) / 128));
-    census_cost_hwd_f32_kernel<<<grid, 128, 0, st>>>(dl, dr, H, W, D, w, reinterpret_cast<float*>(out));
-    return check_launch("census_cost");
-  }
-  census_cost_kernel<T><<<vol_grid(layout, H, W, D), kBlock, 0, st>>>(dl, dr, H, W, D, w, layout, out);
-  return check_launch("census_cost");
+  StripArgs a{};
+  a.L = dl;
+  a.R = dr;
+  a.H = H;
+  a.W = W;
+  a.D = D;
+  a.w = w;
+  return launch_strip<kStripCensus, T, 32>(a, layout, out, st);
 }
 
 int launch_ncc_stats(const uint8_t* img, int64_t H, int64_t W, int w, uint32_t* A, double* C,
@@ -458,6 +527,10 @@ template <class T>
 int launch_ncc_cost(const uint8_t* L, const uint8_t* R, const uint32_t* Al, const uint32_t* Ar,
                     const double* Cl, const double* Cr, int64_t H, int64_t W, int D, int w,
                     int layout, T* out, cudaStream_t st) {
+  if (w == 3) {
+    const StripArgs a{L, R, Al, Ar, Cl, Cr, nullptr, nullptr, H, W, D, w};
+    return launch_strip<kStripNcc, T, 32>(a, layout, out, st);
+  }
   ncc_cost_kernel<T><<<vol_grid(layout, H, W, D), kBlock, 0, st>>>(L, R, Al, Ar, Cl, Cr, H, W, D, w,
                                                                    layout, out);
   return check_launch("ncc_cost");
@@ -471,6 +544,10 @@ int launch_sobel_i32(const uint8_t* img, int64_t H, int64_t W, int32_t* out, cud
 template <class T>
 int launch_sadsob_cost(const int32_t* SL, const int32_t* SR, int64_t H, int64_t W, int D, int w,
                        int layout, T* out, cudaStream_t st) {
+  if (w == 5) {
+    const StripArgs a{SL, SR, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, H, W, D, w};
+    return launch_strip<kStripSadSob, T, 32>(a, layout, out, st);
+  }
   sadsob_cost_kernel<T><<<vol_grid(layout, H, W, D), kBlock, 0, st>>>(SL, SR, H, W, D, w, layout, out);
   return check_launch("sadsob_cost");
 }
@@ -484,43 +561,34 @@ int launch_zsad_means(const uint8_t* img, int64_t H, int64_t W, int w, double* m
 }
 
 template <class T>
-int launch_zsad_cost(const uint8_t* L, const uint8_t* R, const double* ml, const double* mr,
-                     int64_t H, int64_t W, int D, int w, int layout, T* out, cudaStream_t st) {
+static int launch_zsad_general(const uint8_t* L, const uint8_t* R, const double* ml, const double* mr, int64_t H,
+                               int64_t W, int D, int w, int layout, T* out, cudaStream_t st) {
   zsad_cost_kernel<T><<<vol_grid(layout, H, W, D), kBlock, 0, st>>>(L, R, ml, mr, H, W, D, w, layout,
                                                                     out);
   return check_launch("zsad_cost");
 }
 
-template <int MODE, int WIN>
-static int launch_strip(const void* L, const void* R, const uint32_t* Al, const uint32_t* Ar, const double* Cl,
-                        const double* Cr, const double* ml, const double* mr, int64_t H, int64_t W, int D,
-                        float* out, cudaStream_t st) {
-  const dim3 grid((unsigned)((W + kStripX - 1) / kStripX), (unsigned)H, (unsigned)((D + 127) / 128));
-  matcher_strip_kernel<MODE, WIN><<<grid, 128, 0, st>>>(L, R, Al, Ar, Cl, Cr, ml, mr, H, W, D, out);
-  return check_launch("matcher_strip");
+// The float32 volumes of the stand-alone entry point are the float32
+// rounding of the reference's float64 chain; those of the learned path
+// (launch_zsad_cost_f32) of the exact quotient.
+template <class T>
+int launch_zsad_cost(const uint8_t* L, const uint8_t* R, const double* ml, const double* mr,
+                     int64_t H, int64_t W, int D, int w, int layout, T* out, cudaStream_t st) {
+  if (w == 5 && std::is_same<T, double>::value) {
+    const StripArgs a{L, R, nullptr, nullptr, nullptr, nullptr, ml, mr, H, W, D, w};
+    return launch_strip<kStripZsad, double, 16>(a, layout, reinterpret_cast<double*>(out), st);
+  }
+  return launch_zsad_general<T>(L, R, ml, mr, H, W, D, w, layout, out, st);
 }
 
-// float32 [H,W,D] matchers of the learned path: the strip kernels for the
-// default windows, the general kernels otherwise
-int launch_ncc_cost_f32(const uint8_t* L, const uint8_t* R, const uint32_t* Al, const uint32_t* Ar,
-                        const double* Cl, const double* Cr, int64_t H, int64_t W, int D, int w, float* out,
-                        cudaStream_t st) {
-  if (w == 3 && H <= 65535)
-    return launch_strip<kStripNcc, 3>(L, R, Al, Ar, Cl, Cr, nullptr, nullptr, H, W, D, out, st);
-  return launch_ncc_cost<float>(L, R, Al, Ar, Cl, Cr, H, W, D, w, CBMV_HWD, out, st);
-}
-int launch_sadsob_cost_f32(const int32_t* SL, const int32_t* SR, int64_t H, int64_t W, int D, int w, float* out,
-                           cudaStream_t st) {
-  if (w == 5 && H <= 65535)
-    return launch_strip<kStripSadSob, 5>(SL, SR, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, H, W, D,
-                                         out, st);
-  return launch_sadsob_cost<float>(SL, SR, H, W, D, w, CBMV_HWD, out, st);
-}
 int launch_zsad_cost_f32(const uint8_t* L, const uint8_t* R, const double* ml, const double* mr, int64_t H,
                          int64_t W, int D, int w, float* out, cudaStream_t st) {
-  if (w == 5 && H <= 65535)
-    return launch_strip<kStripZsad, 5>(L, R, nullptr, nullptr, nullptr, nullptr, ml, mr, H, W, D, out, st);
-  return launch_zsad_cost<float>(L, R, ml, mr, H, W, D, w, CBMV_HWD, out, st);
+  if (w == 5) {
+    const StripArgs a{L, R, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, H, W, D, w};
+    matcher_strip_kernel<kStripZsad, float, CBMV_HWD, 32><<<strip_grid(a, 32), 32 * kStripWarps, 0, st>>>(a, out);
+    return check_launch("matcher_strip");
+  }
+  return launch_zsad_general<float>(L, R, ml, mr, H, W, D, w, CBMV_HWD, out, st);
 }
 
 template int launch_census_cost<double>(const ulonglong2*, const ulonglong2*, int64_t, int64_t, int,

@@ -438,8 +438,8 @@ static int run_front(cbmv_ctx* c, const cbmv_params* p, const uint8_t* L, const 
   if (f32) {
     float* v[4] = {(float*)w.vol[0], (float*)w.vol[1], (float*)w.vol[2], (float*)w.vol[3]};
     RC(launch_census_cost<float>(w.descL, w.descR, H, W, D, p->censw, CBMV_HWD, v[0], st));
-    RC(launch_ncc_cost_f32(L, R, w.AL, w.AR, w.CL, w.CR, H, W, D, p->nccw, v[1], st));
-    RC(launch_sadsob_cost_f32(w.sobL, w.sobR, H, W, D, p->sobw, v[2], st));
+    RC(launch_ncc_cost<float>(L, R, w.AL, w.AR, w.CL, w.CR, H, W, D, p->nccw, CBMV_HWD, v[1], st));
+    RC(launch_sadsob_cost<float>(w.sobL, w.sobR, H, W, D, p->sobw, CBMV_HWD, v[2], st));
     RC(launch_zsad_cost_f32(L, R, w.muL, w.muR, H, W, D, p->sadw, v[3], st));
     CBMV_CUDA(cudaEventRecord(c->ev[1], st));
     const float* vf[4] = {v[0], v[1], v[2], v[3]};
