@@ -184,63 +184,105 @@ __global__ void d_indices_kernel(const int32_t* __restrict__ gt, int64_t N, int 
 }  // namespace
 
 // ------------------------------------------------------ fused features
-// Per-pixel statistics of one matcher volume for both reference views:
+// Per-pixel statistics of the matcher volumes for both reference views:
 // stats[((m*2 + view)*HW + p)*2 + {0,1}] = {row minimum, likelihood
 // denominator}; view 0 = left reference (row p of the volume), view 1 =
-// right reference (right pixel p: entries C[p + d, d], RAND_MAX when
-// x + d >= W, featextract.cpp:115-152).  One warp per (pixel, view).
-// Row statistics of matcher m: (min, den) in float64 for the exact features
-// and, when statsf is given, (min, 1/den) in float32 for the classifier
-// network (min = 2^31 and 1/den = 0 where the row has only sentinels).
-__global__ void feature_stats_kernel(const double* __restrict__ vol, int m, int64_t H, int64_t W,
-                                     int D, double sigma, double* __restrict__ stats,
-                                     float2* __restrict__ statsf) {
-  const int64_t HW = H * W;
-  const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x / 32);
-  const int lane = threadIdx.x & 31;
-  for (int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; t < 2 * HW; t += nwarps) {
-    const int view = (int)(t / HW);
-    const int64_t p = t - view * HW;
-    const int64_t x = p % W;
-    const double fill = vol[0];  // get_right_cost's fill, featextract.cpp:130
-    double mn = kRandMax;
-    if (view == 0) {
-      const double* r = vol + p * D;
+// right reference (right pixel p: entries C[p + d, d], the fill C[0,0,0]
+// where x + d >= W, featextract.cpp:115-152).
+// Bound by the FP64 pipe: 394 M exponentials of about 27 float64
+// operations each at 694x554 D=128, 0.6 ms.  Left 571 us, right 835 us, all
+// four matchers in a launch; 2351 us with one warp per (pixel, view) that
+// read every row twice, the right view's diagonally, and a full division
+// per term.  The right view through shared-memory tiles: 879 us.
+struct VolsD {
+  const double* v[4];
+};
+
+// view 0: one warp per pixel, its row in registers (KPL per lane; 0: D is
+// beyond 32 KPL of any variant, the row is read twice)
+template <int KPL>
+__global__ void __launch_bounds__(kBlock) stats_left_kernel(VolsD vols, int64_t HW, int D, double* __restrict__ stats) {
+  const int m = blockIdx.y, lane = threadIdx.x & 31;
+  const double* __restrict__ vol = vols.v[m];
+  double* __restrict__ o = stats + (int64_t)(2 * m) * HW * 2;
+  const int64_t nwarps = (int64_t)gridDim.x * (kBlock / 32);
+  for (int64_t p = ((int64_t)blockIdx.x * kBlock + threadIdx.x) >> 5; p < HW; p += nwarps) {
+    const double* r = vol + p * D;
+    double mn = kRandMax, den = 0.0;
+    double v[KPL > 0 ? KPL : 1];
+    if (KPL > 0) {
+#pragma unroll
+      for (int k = 0; k < KPL; k++) {
+        v[k] = lane + 32 * k < D ? __ldg(r + lane + 32 * k) : kRandMax;
+        mn = fmin(mn, v[k]);
+      }
+    } else {
       for (int d = lane; d < D; d += 32) mn = fmin(mn, r[d]);
-    } else {
-      for (int d = lane; d < D; d += 32) mn = fmin(mn, x + d < W ? vol[(p + d) * D + d] : fill);
     }
-    for (int o = 16; o; o >>= 1) mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-    double den = 0.0;
-    if (view == 0) {
-      const double* r = vol + p * D;
-      for (int d = lane; d < D; d += 32) den += lik_term(r[d], mn, sigma);
+    for (int s = 16; s; s >>= 1) mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, s));
+    if (KPL > 0) {
+#pragma unroll
+      for (int k = 0; k < KPL; k++)
+        if (lane + 32 * k < D) den += lik_exp(v[k] - mn, m);
     } else {
-      for (int d = lane; d < D; d += 32)
-        den += lik_term(x + d < W ? vol[(p + d) * D + d] : fill, mn, sigma);
+      for (int d = lane; d < D; d += 32) den += lik_exp(r[d] - mn, m);
     }
     den = warp_sum(den);
-    if (lane == 0) {
-      double* o = stats + ((int64_t)(m * 2 + view) * HW + p) * 2;
-      o[0] = mn;
-      o[1] = den;
-      if (statsf)
-        statsf[(int64_t)(m * 2 + view) * HW + p] =
-            mn == kRandMax ? make_float2(kRandMaxF, 0.0f) : make_float2((float)mn, (float)(1.0 / den));
-    }
+    if (lane == 0) *reinterpret_cast<double2*>(o + 2 * p) = make_double2(mn, den);
   }
 }
 
-__global__ void features_kernel(FeatVols fv, const double* __restrict__ stats, int64_t H, int64_t W,
-                                int D, float* __restrict__ out) {
+// view 1: a warp owns 32 right pixels of one row, lane l the pixel xr = X0 +
+// 31 - l, whose costs are C[xr + d, d].  At step k the lane takes d = k + l
+// (mod D): lanes that have not wrapped around read one row of the volume,
+// x = X0 + 31 + k, at consecutive d, so every step is one or two coalesced
+// runs and all lanes work in all D steps.  The second pass over the 32 x D
+// values finds them in L1 or L2.
+__global__ void __launch_bounds__(kBlock) stats_right_kernel(VolsD vols, int64_t H, int64_t W, int D,
+                                                             double* __restrict__ stats) {
+  const int m = blockIdx.y, lane = threadIdx.x & 31;
+  const double* __restrict__ vol = vols.v[m];
+  const double fill = __ldg(vol);
+  const int64_t nxb = (W + 31) / 32, nwarps = (int64_t)gridDim.x * (kBlock / 32);
+  for (int64_t u = ((int64_t)blockIdx.x * kBlock + threadIdx.x) >> 5; u < H * nxb; u += nwarps) {
+    const int64_t y = u / nxb, xr = u % nxb * 32 + 31 - lane;
+    const double* base = vol + (y * W + xr) * D;
+    const int64_t left = W - xr;  // d < left lies inside the image (no d where the pixel does not)
+    double mn = kRandMax, den = 0.0;
+    int d = lane % D;
+#pragma unroll 8
+    for (int k = 0; k < D; k++) {
+      mn = fmin(mn, d < left ? __ldg(base + (int64_t)d * (D + 1)) : fill);
+      if (++d == D) d = 0;
+    }
+    // D steps on, d is where it began
+#pragma unroll 4
+    for (int k = 0; k < D; k++) {
+      den += lik_exp((d < left ? __ldg(base + (int64_t)d * (D + 1)) : fill) - mn, m);
+      if (++d == D) d = 0;
+    }
+    if (left > 0) *reinterpret_cast<double2*>(stats + ((int64_t)(2 * m + 1) * H * W + y * W + xr) * 2) = make_double2(mn, den);
+  }
+}
+
+// One thread per (pixel, d), its 20 features as five 16-byte stores (VEC)
+// where `out` allows them; I: the type the sample index is divided in.
+template <class I, bool VEC>
+__global__ void __launch_bounds__(kBlock) features_kernel(FeatVols fv, const double* __restrict__ stats, int64_t H,
+                                                          int64_t W, int D, float* __restrict__ out) {
   const int64_t HW = H * W;
   GRID_STRIDE(t, HW * D) {
-    const int64_t p = t / D;
-    const int d = (int)(t - p * D);
+    const I p = (I)t / (I)D;
     float f[20];
-    features_at(fv.v, stats, HW, W, D, p, p % W, d, f);
+    features_at(fv.v, stats, HW, W, D, (int64_t)p, (int64_t)(p % (I)W), (int)((I)t - p * (I)D), f);
+    if (VEC) {
+      float4* o = reinterpret_cast<float4*>(out + t * 20);
 #pragma unroll
-    for (int k = 0; k < 20; k++) out[t * 20 + k] = f[k];
+      for (int k = 0; k < 5; k++) o[k] = make_float4(f[4 * k], f[4 * k + 1], f[4 * k + 2], f[4 * k + 3]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 20; k++) out[t * 20 + k] = f[k];
+    }
   }
 }
 
@@ -524,12 +566,14 @@ int launch_feature_stats_f32(const float* const* vols, int64_t H, int64_t W, int
   return check_launch("feature_stats_f32");
 }
 
-int launch_feature_stats(const double* const* vols, int64_t H, int64_t W, int D, double* stats,
-                         cudaStream_t st, float2* statsf) {
-  const int64_t warps = 2 * H * W;
-  for (int m = 0; m < 4; m++)
-    feature_stats_kernel<<<grid_for(warps * 32, kBlock), kBlock, 0, st>>>(vols[m], m, H, W, D,
-                                                                          hSigma[m], stats, statsf);
+int launch_feature_stats(const double* const* vols, int64_t H, int64_t W, int D, double* stats, cudaStream_t st) {
+  const VolsD v = {{vols[0], vols[1], vols[2], vols[3]}};
+  const int64_t HW = H * W;
+  const dim3 grid(grid_for(HW * 32, kBlock), 4);
+  if (D <= 128) stats_left_kernel<4><<<grid, kBlock, 0, st>>>(v, HW, D, stats);
+  else if (D <= 256) stats_left_kernel<8><<<grid, kBlock, 0, st>>>(v, HW, D, stats);
+  else stats_left_kernel<0><<<grid, kBlock, 0, st>>>(v, HW, D, stats);
+  stats_right_kernel<<<dim3(grid_for(H * ((W + 31) / 32) * 32, kBlock), 4), kBlock, 0, st>>>(v, H, W, D, stats);
   return check_launch("feature_stats");
 }
 
@@ -656,10 +700,15 @@ extern "C" int cbmv_features(const double* census, const double* ncc, const doub
   double* stats = nullptr;
   CBMV_CUDA(cudaMallocAsync(&stats, sizeof(double) * 16 * H * W, st));
   const double* vols[4] = {census, ncc, sob, sad};
-  int rc = launch_feature_stats(vols, H, W, D, stats, st, nullptr);
+  int rc = launch_feature_stats(vols, H, W, D, stats, st);
   if (!rc) {
     FeatVols fv = {{census, ncc, sob, sad}};
-    features_kernel<<<grid_for(H * W * D, kBlock), kBlock, 0, st>>>(fv, stats, H, W, D, out);
+    const unsigned grid = grid_for(H * W * D, kBlock);
+    const bool vec = ((uintptr_t)out & 15) == 0, small = H * W * D < ((int64_t)1 << 32);
+    if (small && vec) features_kernel<uint32_t, true><<<grid, kBlock, 0, st>>>(fv, stats, H, W, D, out);
+    else if (small) features_kernel<uint32_t, false><<<grid, kBlock, 0, st>>>(fv, stats, H, W, D, out);
+    else if (vec) features_kernel<int64_t, true><<<grid, kBlock, 0, st>>>(fv, stats, H, W, D, out);
+    else features_kernel<int64_t, false><<<grid, kBlock, 0, st>>>(fv, stats, H, W, D, out);
     rc = check_launch("features");
   }
   CBMV_CUDA(cudaFreeAsync(stats, st));

@@ -10,19 +10,30 @@ namespace cbmv {
 // ratio epsilon (test.py:548-551) and likelihood sigma (test.py:71-73).
 static __constant__ double kEps[4] = {0.01, 1.01, 0.01, 0.01};
 static __constant__ double kSigma[4] = {2.0 * 8 * 8, 0.02, 2.0 * 100 * 100, 2.0 * 100 * 100};
-static const double hSigma[4] = {2.0 * 8 * 8, 0.02, 2.0 * 100 * 100, 2.0 * 100 * 100};
+static __constant__ double kInvSigma64[4] = {1.0 / (2.0 * 8 * 8), 1.0 / 0.02, 1.0 / (2.0 * 100 * 100),
+                                             1.0 / (2.0 * 100 * 100)};
+
+// exp(-(t * t) / sigma of matcher m) (featextract.cpp:433-434, 440).  The
+// quotient is the IEEE one by Markstein's division: with y = 1/sigma
+// correctly rounded, q = a y is within one unit of a/sigma (|y sigma - 1| <=
+// 0.44 * 2^-53 for the three constants), and one correction by the exact
+// remainder rounds correctly.  Beyond 746 the exponential is 0 in float64;
+// the branch also keeps infinities out of the correction.
+__device__ __forceinline__ double lik_exp(double t, int m) {
+  const double a = t * t, q = a * kInvSigma64[m];
+  if (q > 746.0) return 0.0;
+  return exp(-fma(fma(-q, kSigma[m], a), kInvSigma64[m], q));
+}
 
 // ratio / likelihood of cost c against the statistics (min, den) of its row
 // (featextract.cpp:333, :440).
-__device__ __forceinline__ void confidences(double c, double mn, double den, double e, double sigma,
-                                            float* ratio, float* lik) {
+__device__ __forceinline__ void confidences(double c, double mn, double den, int m, float* ratio, float* lik) {
   if (mn == kRandMax) {
     *ratio = 0.0f;
     *lik = 0.0f;
   } else {
-    *ratio = (float)((mn + e) / (c + e));
-    const double t = c - mn;
-    *lik = (float)(exp(-((t * t) / sigma)) / den);
+    *ratio = (float)((mn + kEps[m]) / (c + kEps[m]));
+    *lik = (float)(lik_exp(c - mn, m) / den);
   }
 }
 
@@ -39,10 +50,10 @@ __device__ __forceinline__ void features_at(const double* const* vols, const dou
     const double c = vols[m][p * D + d];
     f[m] = (float)c;
     const double* sl = stats + ((int64_t)(m * 2 + 0) * HW + p) * 2;
-    confidences(c, sl[0], sl[1], kEps[m], kSigma[m], &f[4 + m], &f[8 + m]);
+    confidences(c, sl[0], sl[1], m, &f[4 + m], &f[8 + m]);
     if (x >= d) {
       const double* sr = stats + ((int64_t)(m * 2 + 1) * HW + (p - d)) * 2;
-      confidences(c, sr[0], sr[1], kEps[m], kSigma[m], &f[12 + m], &f[16 + m]);
+      confidences(c, sr[0], sr[1], m, &f[12 + m], &f[16 + m]);
     } else {
       f[12 + m] = 0.0f;
       f[16 + m] = 0.0f;
@@ -62,12 +73,12 @@ __device__ __forceinline__ void features_store(const double* const* vols, const 
     float r, l;
     f[m * stride] = (float)c;
     const double* sl = stats + ((int64_t)(m * 2 + 0) * HW + p) * 2;
-    confidences(c, sl[0], sl[1], kEps[m], kSigma[m], &r, &l);
+    confidences(c, sl[0], sl[1], m, &r, &l);
     f[(4 + m) * stride] = r;
     f[(8 + m) * stride] = l;
     if (x >= d) {
       const double* sr = stats + ((int64_t)(m * 2 + 1) * HW + (p - d)) * 2;
-      confidences(c, sr[0], sr[1], kEps[m], kSigma[m], &r, &l);
+      confidences(c, sr[0], sr[1], m, &r, &l);
     } else {
       r = 0.0f;
       l = 0.0f;
@@ -77,37 +88,8 @@ __device__ __forceinline__ void features_store(const double* const* vols, const 
   }
 }
 
-// The features of matchers m0 and m0+1 only: f[2g + i] is feature group g
-// (0 cost, 1 ratio, 2 likelihood, 3 right ratio, 4 right likelihood) of
-// matcher m0 + i, i.e. reference column 4g + m0 + i.
-__device__ __forceinline__ void features_pair(const double* const* vols, const double* stats,
-                                              int64_t HW, int D, int64_t p, int64_t x, int d, int m0,
-                                              float* f) {
-#pragma unroll
-  for (int i = 0; i < 2; i++) {
-    const int m = m0 + i;
-    const double c = vols[m][p * D + d];
-    float r, l;
-    f[i] = (float)c;
-    const double* sl = stats + ((int64_t)(m * 2 + 0) * HW + p) * 2;
-    confidences(c, sl[0], sl[1], kEps[m], kSigma[m], &r, &l);
-    f[2 + i] = r;
-    f[4 + i] = l;
-    if (x >= d) {
-      const double* sr = stats + ((int64_t)(m * 2 + 1) * HW + (p - d)) * 2;
-      confidences(c, sr[0], sr[1], kEps[m], kSigma[m], &r, &l);
-    } else {
-      r = 0.0f;
-      l = 0.0f;
-    }
-    f[6 + i] = r;
-    f[8 + i] = l;
-  }
-}
-
 struct FeatVols {
   const double* v[4];
 };
-
 
 }  // namespace cbmv

@@ -34,8 +34,7 @@ int launch_zsad_cost(const uint8_t* L, const uint8_t* R, const double* ml, const
 // the learned path's float32 [H,W,D] ZSAD (rounded from the exact quotient)
 int launch_zsad_cost_f32(const uint8_t* L, const uint8_t* R, const double* ml, const double* mr, int64_t H,
                          int64_t W, int D, int w, float* out, cudaStream_t st);
-int launch_feature_stats(const double* const* vols, int64_t H, int64_t W, int D, double* stats,
-                         cudaStream_t st, float2* statsf = nullptr);
+int launch_feature_stats(const double* const* vols, int64_t H, int64_t W, int D, double* stats, cudaStream_t st);
 // (min, 1/den) in float32 of float32 volumes, both views, the four matchers
 int launch_feature_stats_f32(const float* const* vols, int64_t H, int64_t W, int D, float2* statsf,
                              cudaStream_t st);
