@@ -386,32 +386,37 @@ __global__ void sgm_combine_kernel(SgmOut o, int64_t n, const float* base, float
   }
 }
 
-// cbca (post.cu:399-450), any layout.
+// cbca (post.cu:399-450) of one (y, x, d), any layout: the float sum over the
+// support in the reference's order (rows ascending, then columns ascending,
+// from 0) divided by its pixels; the input where the match is outside.
+__device__ __forceinline__ float cbca_one(const float* __restrict__ lc, const float* __restrict__ rc,
+                                          const float* __restrict__ in, int64_t H, int64_t W, int64_t D, int layout,
+                                          int direction, int64_t y, int64_t x, int64_t d) {
+  const int64_t xm = x + d * direction;
+  if (xm < 0 || xm >= W) return in[vol_index(layout, y, x, d, H, W, D)];
+  const int yy_s = (int)fmaxf(lc[(2 * H + y) * W + x], rc[(2 * H + y) * W + xm]);
+  const int yy_t = (int)fminf(lc[(3 * H + y) * W + x], rc[(3 * H + y) * W + xm]);
+  const float dd = (float)(d * direction);
+  float sum = 0.0f;
+  int cnt = 0;
+  for (int yy = yy_s + 1; yy < yy_t; yy++) {
+    const int xx_s = (int)fmaxf(lc[(0 * H + yy) * W + x], rc[(0 * H + yy) * W + xm] - dd);
+    const int xx_t = (int)fminf(lc[(1 * H + yy) * W + x], rc[(1 * H + yy) * W + xm] - dd);
+    for (int xx = xx_s + 1; xx < xx_t; xx++) {
+      sum += in[vol_index(layout, yy, xx, d, H, W, D)];
+      cnt++;
+    }
+  }
+  return sum / (float)cnt;
+}
+
 __global__ void cbca_kernel(const float* __restrict__ lc, const float* __restrict__ rc,
                             const float* __restrict__ in, int64_t H, int64_t W, int64_t D,
                             int layout, int direction, float* __restrict__ out) {
   GRID_STRIDE(id, H * W * D) {
     int64_t y, x, d;
     decode(layout, id, H, W, D, &y, &x, &d);
-    const int64_t xm = x + d * direction;
-    if (xm < 0 || xm >= W) {
-      out[id] = in[id];
-      continue;
-    }
-    const int yy_s = (int)fmaxf(lc[(2 * H + y) * W + x], rc[(2 * H + y) * W + xm]);
-    const int yy_t = (int)fminf(lc[(3 * H + y) * W + x], rc[(3 * H + y) * W + xm]);
-    const float dd = (float)(d * direction);
-    float sum = 0.0f;
-    int cnt = 0;
-    for (int yy = yy_s + 1; yy < yy_t; yy++) {
-      const int xx_s = (int)fmaxf(lc[(0 * H + yy) * W + x], rc[(0 * H + yy) * W + xm] - dd);
-      const int xx_t = (int)fminf(lc[(1 * H + yy) * W + x], rc[(1 * H + yy) * W + xm] - dd);
-      for (int xx = xx_s + 1; xx < xx_t; xx++) {
-        sum += in[vol_index(layout, yy, xx, d, H, W, D)];
-        cnt++;
-      }
-    }
-    out[id] = sum / (float)cnt;
+    out[id] = cbca_one(lc, rc, in, H, W, D, layout, direction, y, x, d);
   }
 }
 
@@ -669,6 +674,134 @@ __device__ __forceinline__ uint32_t pack_rel_arms(const float* __restrict__ c, i
 template <int B>
 __device__ __forceinline__ int rel_arm(uint32_t w) {
   return (int)((int32_t)(w << (24 - 8 * B)) >> 24);
+}
+
+// cbca on [D,H,W] volumes (the drop-in's layout) in the reference's order:
+// a CTA owns 32 columns x 16 rows of eight disparities, one per warp (lane =
+// column).  A support row's interval depends on its own row only, so a warp
+// reads and masks each row of its tile once (eleven taps, those outside the
+// interval as 0: adding 0 changes no sum) and adds the eleven values to the
+// running sum of every one of four output rows whose support has the row --
+// the rows ascend, so each sum runs in the reference's order.  A support
+// that reaches beyond five pixels (cross arms of L1 > 6) is summed by
+// cbca_one.  Bound by instruction issue (the masks of a row are formed for
+// every four outputs, 14 rows; eight outputs at once need 79 registers and
+// were slower, 613 us).  694x320 D=128: 533 us a pass, 1380 us with a
+// thread per output walking its support (cbca_kernel).
+constexpr int CD_X = 32, CD_Y = 16, CD_D = 8, CD_G = 4, CD_HALO = 5;
+
+// The arms of one pixel packed as pack_rel_arms does, without conversions
+// (an arm below 2^22 is read off its sum with 1.5 * 2^23); *odd: one of them
+// is no whole number, or too large for that.
+__device__ __forceinline__ uint32_t pack_whole_arms(const float* __restrict__ c, int64_t HW, int64_t o, int x, int y,
+                                                    bool* odd) {
+  constexpr float kMagic = 12582912.0f;
+  uint32_t w = 0;
+#pragma unroll
+  for (int a = 0; a < 4; a++) {
+    const float v = __ldg(c + a * HW + o), t = __fadd_rn(v, kMagic);
+    *odd |= !(__fsub_rn(t, kMagic) == v && fabsf(v) < 4194304.0f);
+    w |= (uint32_t)(clamp_i8(__float_as_int(t) - __float_as_int(kMagic) - (a < 2 ? x : y)) & 0xFF) << (8 * a);
+  }
+  return w;
+}
+
+// taps lo..hi (bit k + 5) of an interval, those within five pixels
+__device__ __forceinline__ uint32_t tap_mask(int lo, int hi) {
+  const int a = min(max(lo + CD_HALO, 0), 31), b = min(max(hi + CD_HALO + 1, 0), 31);
+  return ((1u << b) - 1u) & ~((1u << a) - 1u);
+}
+
+__global__ void __launch_bounds__(32 * CD_D) cbca_dhw_kernel(const float* __restrict__ lc, const float* __restrict__ rc,
+                                                               const float* __restrict__ in, int H, int W, int D,
+                                                               int direction, float* __restrict__ out) {
+  constexpr int SR = CD_Y + 2 * CD_HALO, SX = CD_X + 2 * CD_HALO, NXM = CD_X + CD_D - 1, NT = 2 * CD_HALO + 1;
+  __shared__ uint32_t sAL[SR][CD_X];  // packed relative arms, left view at (yy, x)
+  __shared__ uint32_t sAR[SR][NXM];   // right view at (yy, x + d * direction)
+  __shared__ float tiles[CD_D][SR][SX];
+  const int ntx = (W + CD_X - 1) / CD_X, nty = (H + CD_Y - 1) / CD_Y;
+  const int64_t t = blockIdx.x;
+  const int X0 = (int)(t % ntx) * CD_X, Y0 = (int)(t / ntx % nty) * CD_Y, D0 = (int)(t / ((int64_t)ntx * nty)) * CD_D;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t HW = (int64_t)H * W;
+  const int xm_lo = direction > 0 ? X0 + D0 : X0 - (D0 + CD_D - 1);
+  bool odd = false;  // an arm that is no whole number: the sums are left to cbca_one
+  for (int r = warp; r < SR; r += CD_D) {
+    const int yy = Y0 - CD_HALO + r;
+    const bool rok = yy >= 0 && yy < H;  // outside the image: an empty interval
+    const int64_t o = (int64_t)yy * W;
+    sAL[r][lane] = rok && X0 + lane < W ? pack_whole_arms(lc, HW, o + X0 + lane, X0 + lane, yy, &odd) : 0u;
+    for (int j = lane; j < NXM; j += 32) {
+      const int xm = xm_lo + j;
+      sAR[r][j] = rok && xm >= 0 && xm < W ? pack_whole_arms(rc, HW, o + xm, xm, yy, &odd) : 0u;
+    }
+  }
+  odd = __syncthreads_or(odd);
+  const int x = X0 + lane;
+  float(*tile)[SX] = tiles[warp];
+  const int xa = X0 - CD_HALO + lane, xb = xa + 32;
+  const bool oka = xa >= 0 && xa < W, okb = lane < SX - 32 && xb < W;
+  const int d = D0 + warp;
+  if (d >= D) return;
+  const float* src = in + (int64_t)d * HW + (int64_t)(Y0 - CD_HALO) * W + xa;
+#pragma unroll
+  for (int r = 0; r < SR; r++) {
+    const bool rok = Y0 - CD_HALO + r >= 0 && Y0 - CD_HALO + r < H;
+    tile[r][lane] = rok && oka ? __ldg(src) : 0.0f;
+    if (lane < SX - 32) tile[r][lane + 32] = rok && okb ? __ldg(src + 32) : 0.0f;
+    src += W;
+  }
+  __syncwarp();
+  if (x >= W) return;
+  const int xm = x + d * direction;
+  const bool match = xm >= 0 && xm < W;
+  const int jr = match ? xm - xm_lo : 0;
+  float* dst = out + (int64_t)d * HW + x;
+#pragma unroll 1
+  for (int g = 0; g < CD_Y && Y0 + g < H; g += CD_G) {
+    // the rows of every output's support as taps; its sum; its pixels, and from bit 16 up the
+    // rows (or the support itself) that reach beyond the taps
+    uint32_t vm[CD_G];
+    float sum[CD_G];
+    int cnt[CD_G];
+#pragma unroll
+    for (int j = 0; j < CD_G; j++) {
+      const uint32_t wl = sAL[g + j + CD_HALO][lane], wr = sAR[g + j + CD_HALO][jr];
+      const int lo = max(rel_arm<2>(wl), rel_arm<2>(wr)) + 1, hi = min(rel_arm<3>(wl), rel_arm<3>(wr)) - 1;
+      vm[j] = tap_mask(lo, hi);
+      cnt[j] = odd || (hi >= lo && (lo < -CD_HALO || hi > CD_HALO)) ? 1 << 16 : 0;
+      sum[j] = 0.0f;
+    }
+#pragma unroll
+    for (int r = 0; r < CD_G + 2 * CD_HALO; r++) {
+      const uint32_t wl = sAL[g + r][lane], wr = sAR[g + r][jr];
+      const int lo = max(rel_arm<0>(wl), rel_arm<0>(wr)) + 1, hi = min(rel_arm<1>(wl), rel_arm<1>(wr)) - 1;
+      const uint32_t hm = tap_mask(lo, hi);
+      int len = hi - lo + 1;
+      len = len <= 0 ? 0 : lo < -CD_HALO || hi > CD_HALO ? 1 << 16 : len;
+      float v[NT];
+#pragma unroll
+      for (int k = 0; k < NT; k++) {
+        v[k] = tile[g + r][lane + k];
+        if (!(hm & (1u << k))) v[k] = 0.0f;
+      }
+#pragma unroll
+      for (int j = r > 2 * CD_HALO ? r - 2 * CD_HALO : 0; j < CD_G && j <= r; j++)
+        if (vm[j] & (1u << (r - j))) {
+#pragma unroll
+          for (int k = 0; k < NT; k++) sum[j] += v[k];
+          cnt[j] += len;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < CD_G; j++) {
+      const int y = Y0 + g + j;
+      if (y >= H) break;
+      float v = match ? sum[j] / (float)cnt[j] : tile[g + j + CD_HALO][lane + CD_HALO];
+      if (match && cnt[j] >= 1 << 16) v = cbca_one(lc, rc, in, H, W, D, CBMV_DHW, direction, y, x, d);
+      dst[(int64_t)y * W] = v;
+    }
+  }
 }
 
 template <int CS_TY>
@@ -1262,6 +1395,11 @@ int launch_cbca(const float* lc, const float* rc, const float* in, int64_t H, in
     cbca_hwd_tiled_kernel<<<grid, 256, smem, st>>>(lc, rc, in, (int)H, (int)W, D, direction, halo,
                                                    out);
     return check_launch("cbca_tiled");
+  }
+  const int64_t dhw_tiles = ((W + CD_X - 1) / CD_X) * ((H + CD_Y - 1) / CD_Y) * ((D + CD_D - 1) / CD_D);
+  if (layout == CBMV_DHW && H < (1 << 30) && W < (1 << 30) && dhw_tiles < ((int64_t)1 << 31)) {
+    cbca_dhw_kernel<<<(unsigned)dhw_tiles, 32 * CD_D, 0, st>>>(lc, rc, in, (int)H, (int)W, D, direction, out);
+    return check_launch("cbca_dhw");
   }
   cbca_kernel<<<grid_for(H * W * D, kBlock), kBlock, 0, st>>>(lc, rc, in, H, W, D, layout, direction,
                                                              out);
