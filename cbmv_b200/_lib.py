@@ -81,6 +81,8 @@ SIGNATURES = {
     "cbmv_mlp_get_precision": [_vp, _vp],
     "cbmv_cross": [_vp, _i64, _i64, _int, _flt, _vp, _vp],
     "cbmv_sgm": [_vp, _vp, _vp, _i64, _i64, _int, _flt, _flt, _flt, _flt, _flt, _flt, _int, _vp, _vp],
+    "cbmv_sgm_scratch_bytes": [_i64, _i64, _int],
+    "cbmv_sgm_scratch": [_vp, _vp, _vp, _i64, _i64, _int, _flt, _flt, _flt, _flt, _flt, _flt, _int, _vp, _vp, _vp],
     "cbmv_cbca": [_vp, _vp, _vp, _i64, _i64, _int, _int, _int, _vp, _vp],
     "cbmv_cbca_separable": [_vp, _vp, _vp, _i64, _i64, _int, _int, _int, _vp, _vp],
     "cbmv_wta": [_vp, _i64, _i64, _int, _int, _vp, _vp],
@@ -112,7 +114,8 @@ SIGNATURES = {
     "cbmv_batch_timings": [_vp, _vp, _vp, _vp],
 }
 _RESTYPE = {"cbmv_last_error": ctypes.c_char_p, "cbmv_version": ctypes.c_char_p,
-            "cbmv_params_default": None, "cbmv_census_static_max_pixels": ctypes.c_int64}
+            "cbmv_params_default": None, "cbmv_census_static_max_pixels": ctypes.c_int64,
+            "cbmv_sgm_scratch_bytes": ctypes.c_int64}
 
 _lib = None
 

@@ -1528,24 +1528,54 @@ extern "C" int cbmv_cross(const float* img, int64_t H, int64_t W, int L1, float 
   return launch_cross(img, H, W, L1, tau1, out, as_stream(stream));
 }
 
-extern "C" int cbmv_sgm(const float* imL, const float* imR, const float* in, int64_t H, int64_t W,
-                        int D, float pi1, float pi2, float tau_so, float alpha1, float q1, float q2,
-                        int direction, float* out, void* stream) {
+static int check_sgm(const float* imL, const float* imR, const float* in, int64_t H, int64_t W, int D, int direction,
+                     const float* out) {
   REQ_PTR(imL && imR && in && out);
   REQ_HW(H, W);
   CBMV_REQUIRE(D > 0 && D <= 1024, CBMV_ERANGE, "D=%d not in 1..1024", D);
   CBMV_REQUIRE(in != out, CBMV_EINVAL, "sgm: in and out must differ");
   CBMV_REQUIRE(direction == 1 || direction == -1, CBMV_EINVAL, "direction must be +-1");
-  cudaStream_t st = as_stream(stream);
-  const int64_t HW = H * W, V = HW * D;
-  float* scratch = nullptr;
-  CBMV_CUDA(cudaMallocAsync(&scratch, sizeof(float) * (4 * HW + 4 * V), st));
-  SgmGrad g{scratch, scratch + HW, scratch + 2 * HW, scratch + 3 * HW};
-  SgmOut o{{scratch + 4 * HW, scratch + 4 * HW + V, scratch + 4 * HW + 2 * V, scratch + 4 * HW + 3 * V}};
-  SgmParams sp{pi1, pi2, tau_so, alpha1, q1, q2, direction};
+  return CBMV_OK;
+}
+
+// scratch: the direction volumes, then the image differences
+static int run_sgm(const float* imL, const float* imR, const float* in, int64_t H, int64_t W, int D,
+                   const SgmParams& sp, float* out, float* scratch, cudaStream_t st) {
+  const int64_t HW = H * W, V = HW * D, S = (V + 3) / 4 * 4;  // every volume 16-byte aligned
+  SgmOut o{{scratch, scratch + S, scratch + 2 * S, scratch + 3 * S}};
+  float* gr = scratch + 4 * S;
+  SgmGrad g{gr, gr + HW, gr + 2 * HW, gr + 3 * HW};
   int rc = launch_sgm_grad(imL, imR, H, W, &g, st);
   if (!rc) rc = launch_sgm4(g, in, H, W, D, sp, o, st);
   if (!rc) rc = launch_sgm_combine(o, V, out, 1.0f, out, st);
+  return rc;
+}
+
+extern "C" int64_t cbmv_sgm_scratch_bytes(int64_t H, int64_t W, int D) {
+  if (H <= 0 || W <= 0 || H > (1 << 30) || W > (1 << 30) || D <= 0 || D > 1024) return -1;
+  return (int64_t)sizeof(float) * (4 * ((H * W * D + 3) / 4 * 4) + 4 * H * W);
+}
+
+extern "C" int cbmv_sgm_scratch(const float* imL, const float* imR, const float* in, int64_t H, int64_t W, int D,
+                                float pi1, float pi2, float tau_so, float alpha1, float q1, float q2, int direction,
+                                float* out, void* scratch, void* stream) {
+  const int rc = check_sgm(imL, imR, in, H, W, D, direction, out);
+  if (rc) return rc;
+  REQ_PTR(scratch);
+  CBMV_REQUIRE(((uintptr_t)scratch & 15) == 0, CBMV_EINVAL, "sgm: scratch must be 16-byte aligned");
+  return run_sgm(imL, imR, in, H, W, D, SgmParams{pi1, pi2, tau_so, alpha1, q1, q2, direction}, out,
+                 static_cast<float*>(scratch), as_stream(stream));
+}
+
+extern "C" int cbmv_sgm(const float* imL, const float* imR, const float* in, int64_t H, int64_t W,
+                        int D, float pi1, float pi2, float tau_so, float alpha1, float q1, float q2,
+                        int direction, float* out, void* stream) {
+  int rc = check_sgm(imL, imR, in, H, W, D, direction, out);
+  if (rc) return rc;
+  cudaStream_t st = as_stream(stream);
+  float* scratch = nullptr;
+  CBMV_CUDA(cudaMallocAsync(&scratch, (size_t)cbmv_sgm_scratch_bytes(H, W, D), st));
+  rc = run_sgm(imL, imR, in, H, W, D, SgmParams{pi1, pi2, tau_so, alpha1, q1, q2, direction}, out, scratch, st);
   CBMV_CUDA(cudaFreeAsync(scratch, st));
   return rc;
 }

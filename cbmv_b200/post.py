@@ -75,11 +75,14 @@ def cross(img, out, L1, tau1):
 def sgm(left, right, in_cost, out_cost, tmp, pi1, pi2, tau_so, alpha1, sgm_q1, sgm_q2, direction):
     """post.cu:263-333: out_cost += the four scan directions' path costs of
     in_cost ([H,W,D]).  `tmp` is the reference's per-line scratch; the path
-    values live in registers here, so it is unused."""
+    values live in registers here, so it is unused.  The scratch comes from
+    torch's caching allocator, on the stream the call runs on."""
     H, W, D = in_cost.ins
-    _lib.call("cbmv_sgm", left.ptr, right.ptr, in_cost.ptr, H, W, D, float(pi1), float(pi2),
+    need = _lib.lib().cbmv_sgm_scratch_bytes(H, W, D)
+    scratch = torch.empty(max(need, 16), dtype=torch.uint8, device="cuda")
+    _lib.call("cbmv_sgm_scratch", left.ptr, right.ptr, in_cost.ptr, H, W, D, float(pi1), float(pi2),
               float(tau_so), float(alpha1), float(sgm_q1), float(sgm_q2), int(direction),
-              out_cost.ptr, _s())
+              out_cost.ptr, scratch.data_ptr(), _s())
 
 
 def cbca(leftc, rightc, vol, vol_out, direction):

@@ -271,6 +271,16 @@ int cbmv_cross(const float* img, int64_t H, int64_t W, int L1, float tau1, float
 int cbmv_sgm(const float* imL, const float* imR, const float* in, int64_t H, int64_t W, int D,
              float pi1, float pi2, float tau_so, float alpha1, float q1, float q2, int direction,
              float* out, void* stream);
+/* cbmv_sgm with its scratch -- the four directions' path costs and the image
+ * differences, cbmv_sgm_scratch_bytes(H, W, D) bytes, 16-byte aligned -- in
+ * the caller's device memory, for callers whose allocator keeps blocks
+ * between calls: cbmv_sgm takes it from the stream-ordered pool, which
+ * returns 16 B per (p,d) to the driver at every synchronisation.  -1 for
+ * sizes cbmv_sgm rejects. */
+int64_t cbmv_sgm_scratch_bytes(int64_t H, int64_t W, int D);
+int cbmv_sgm_scratch(const float* imL, const float* imR, const float* in, int64_t H, int64_t W,
+                     int D, float pi1, float pi2, float tau_so, float alpha1, float q1, float q2,
+                     int direction, float* out, void* scratch, void* stream);
 /* cbca (post.cu:399-450) on a volume of layout `layout`; in != out. */
 int cbmv_cbca(const float* crossL, const float* crossR, const float* in, int64_t H, int64_t W,
               int D, int layout, int direction, float* out, void* stream);
