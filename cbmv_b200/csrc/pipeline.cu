@@ -114,7 +114,7 @@ struct Work {
   float *volA, *volB;
   float* volC;  // the right view's cost of the _interp post (else null)
   float *imL, *imR, *crossL, *crossR, *dtmp, *dtmp2, *dright, *outlier;
-  float* grad;  // SGM neighbour differences: left h/v, right h/v
+  void* codes;  // SGM image classes
   uint32_t* masks;  // CBCA support words, 4 B per (p,d), live beside the SGM volumes
   bool prepped = false;  // the post's image terms were launched on the side stream (prep_ev)
   double* mom;
@@ -152,7 +152,7 @@ Work carve(void* base, int64_t H, int64_t W, int D, size_t* bytes, bool f32, boo
   w.dtmp2 = c.take<float>(HW);
   w.dright = c.take<float>(HW);
   w.outlier = c.take<float>(HW);
-  w.grad = c.take<float>(4 * HW);
+  w.codes = c.take<char>(sgm_codes_bytes(H, W));
   // the support words: their own volume on the float32 path (the SGM's four
   // direction volumes take all four matcher volumes), the third float64
   // matcher volume otherwise (the SGM uses only the first two)
@@ -312,14 +312,14 @@ static int cost_chain(cbmv_ctx* c, const cbmv_params* p, Work& w, int64_t H, int
     float* t = cur; cur = oth; oth = t;
   }
   SgmParams sp{p->pi1, p->pi2, p->tau_so, p->alpha1, p->sgm_q1, p->sgm_q2, direction};
-  SgmGrad g{w.grad, w.grad + HW, w.grad + 2 * HW, w.grad + 3 * HW};
+  const SgmCodes g = sgm_codes_at(w.codes, H, W);
   // the four direction volumes reuse the cost volumes, dead by now
   const int64_t V = HW * D;
   SgmOut so = w.f32 ? SgmOut{{(float*)w.vol[0], (float*)w.vol[1], (float*)w.vol[2], (float*)w.vol[3]}}
                     : SgmOut{{(float*)w.vol[0], (float*)w.vol[0] + V, (float*)w.vol[1], (float*)w.vol[1] + V}};
   for (int i = 0; i < p->sgm_i; i++) {
     // out = ((L0 + L1 + L2) + L3) / 4   (test.py:379-383)
-    RC(launch_sgm4(g, cur, H, W, D, sp, so, st, p->sgm_prefetch));
+    RC(launch_sgm4(g, cur, H, W, D, sp, so, st));
     RC(launch_sgm_combine(so, V, nullptr, 0.25f, oth, st));
     float* t = cur; cur = oth; oth = t;
   }
@@ -340,7 +340,7 @@ static int cost_chain(cbmv_ctx* c, const cbmv_params* p, Work& w, int64_t H, int
 // occlusions and mismatches (left-right check) and fills them
 // (interpolate_mismatch, then interpolate_occlusion) before the median.
 // The post's image terms (do_post's normalisation, test.py:485-504; the
-// cross arms; the SGM's neighbour differences): they depend on the images
+// cross arms; the SGM's classes): they depend on the images
 // only, so the fused paths launch them on the side stream at the start of
 // the call, beside the matchers.
 static int post_prep(const cbmv_params* p, const uint8_t* L, const uint8_t* R, int64_t H, int64_t W, Work& w,
@@ -350,8 +350,7 @@ static int post_prep(const cbmv_params* p, const uint8_t* L, const uint8_t* R, i
   RC(launch_normalise(R, HW, w.mom + 2, w.imR, s));
   RC(launch_cross(w.imL, H, W, p->L1, p->tau1, w.crossL, s));
   RC(launch_cross(w.imR, H, W, p->L1, p->tau1, w.crossR, s));
-  SgmGrad g{w.grad, w.grad + HW, w.grad + 2 * HW, w.grad + 3 * HW};
-  if (p->sgm_i > 0) RC(launch_sgm_grad(w.imL, w.imR, H, W, &g, s));
+  if (p->sgm_i > 0) RC(launch_sgm_codes(w.imL, w.imR, H, W, p->tau_so, sgm_codes_at(w.codes, H, W), s));
   return CBMV_OK;
 }
 

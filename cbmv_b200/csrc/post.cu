@@ -7,11 +7,11 @@
 // Gaussian).  Where the reference accumulates in float64 (the SGM path
 // values and their sum over the four directions) the sums here are float32.
 //
-// SGM runs one scan direction per launch with one warp per scan line and the
-// scan inside the kernel (the reference launches one kernel per scan step,
-// 2(W+H) launches per call, post.cu:273-330); each lane holds D/32 path
-// values in registers, the minimum over d is a warp-shuffle reduction, and
-// the next step's costs are loaded one step ahead.
+// SGM runs all four scan directions in one launch with one warp per scan line
+// and the scan inside the kernel (the reference launches one kernel per scan
+// step, 2(W+H) launches per call, post.cu:273-330); the lanes hold the path
+// values in registers, the minimum over d is a warp reduction, and the next
+// steps' costs are loaded ahead.
 #include "common.cuh"
 #include "post.cuh"
 
@@ -59,35 +59,103 @@ __global__ void cross_kernel(const float* __restrict__ x0, int64_t H, int64_t W,
   }
 }
 
-// Absolute differences of neighbouring pixels of a normalised image:
-// gh[y][x] = |I[y][x] - I[y][x-1]|, gv[y][x] = |I[y][x] - I[y-1][x]| (0 on
-// the first column / row).  SGM's image terms D1 and D2 (post.cu:230-237)
-// are exactly these values (|a - b| == |b - a| in IEEE arithmetic).
-__global__ void grad_kernel(const float* __restrict__ img, int64_t H, int64_t W,
-                            float* __restrict__ gh, float* __restrict__ gv) {
-  GRID_STRIDE(p, H * W) {
-    const int64_t y = p / W, x = p - y * W;
-    const float c = img[p];
-    gh[p] = x > 0 ? fabsf(c - img[p - 1]) : 0.0f;
-    gv[p] = y > 0 ? fabsf(c - img[p - W]) : 0.0f;
+// SGM's image terms (post.cu:230-248).  A step's penalties depend only on
+// whether the left difference D1 and the right difference D2 of the scan
+// direction's neighbouring pixels lie below or above tau_so, so the scan
+// reads two bits per pixel, {D < tau, D > tau}, packed along the scan: 32
+// pixels of a row for the horizontal directions, 32 rows of a column for the
+// vertical ones (|a - b| == |b - a| in IEEE arithmetic: one difference per
+// pair of neighbours serves both directions along it).  Where a right
+// difference leaves the image D2 = 10.  A warp takes a 32 x 32 tile.
+__global__ void __launch_bounds__(128) sgm_codes_kernel(const float* __restrict__ imL, const float* __restrict__ imR,
+                                                      int H, int W, float tau, SgmCodes g) {
+  const int lane = threadIdx.x & 31, gw = (W + 31) / 32, gh = (H + 31) / 32;
+  const int64_t n = (int64_t)gridDim.x * 4;
+  for (int64_t u = ((int64_t)blockIdx.x * 128 + threadIdx.x) >> 5; u < (int64_t)2 * gw * gh; u += n) {
+    const bool right = u >= (int64_t)gw * gh;
+    const int64_t t = u - (right ? (int64_t)gw * gh : 0);
+    const int tw = (int)(t % gw), th = (int)(t / gw), x = 32 * tw + lane;
+    const float* im = right ? imR : imL;
+    const float none = right ? 10.0f : 0.0f;
+    const bool xok = x < W;
+    uint2 rows = make_uint2(0u, 0u), cols = make_uint2(0u, 0u);  // row 32 th + lane; column x
+    float up = xok && th > 0 ? __ldg(im + ((int64_t)32 * th - 1) * W + x) : 0.0f;
+    for (int r = 0; r < 32; r++) {
+      const int y = 32 * th + r;
+      if (y >= H) break;
+      const float v = xok ? __ldg(im + (int64_t)y * W + x) : 0.0f;
+      float before = __shfl_up_sync(0xffffffffu, v, 1);
+      if (lane == 0 && x > 0) before = __ldg(im + (int64_t)y * W + x - 1);
+      const float dh = xok && x > 0 ? fabsf(v - before) : none, dv = xok && y > 0 ? fabsf(v - up) : none;
+      up = v;
+      const uint32_t lo = __ballot_sync(0xffffffffu, dh < tau), hi = __ballot_sync(0xffffffffu, dh > tau);
+      if (lane == r) rows = make_uint2(lo, hi);
+      cols.x |= (uint32_t)(dv < tau) << r;
+      cols.y |= (uint32_t)(dv > tau) << r;
+    }
+    if (32 * th + lane < H) (right ? g.right_h : g.left_h)[((int64_t)32 * th + lane) * gw + tw] = rows;
+    if (xok) (right ? g.right_v : g.left_v)[(int64_t)th * W + x] = cols;
   }
 }
 
-// sgm2 (post.cu:178-261) for all four scan directions in one launch (one
-// scan routine, the direction a run-time argument: a single copy of the
-// code keeps the instruction cache warm across the four directions): one
-// warp per scan line (the 2H horizontal and 2W vertical lines run
-// concurrently, each direction writing its path costs to its own volume),
-// lane = d (mod 32), KPL disparities per lane.  The scan runs inside the
-// kernel; the step's costs, D1 and the per-d D2 do not depend on the
-// recursion and are loaded PF steps ahead from a register ring.
-template <int KPL, int PF, bool FULL>
-__device__ __noinline__ void sgm_scan(const SgmGrad& g, const float* __restrict__ in, int H, int W, int D,
-                                      const SgmParams& sp, int line, float* __restrict__ out, const int DIR) {
+// sgm2 (post.cu:178-261): one scan direction of one line.  A warp scans a
+// line, lane l holding the KPL consecutive disparities KPL l .. KPL l + KPL-1
+// of the path costs: the d-1 / d+1 neighbours are in the lane's own registers
+// except at its two ends (two shuffles), the minimum over d is one
+// `redux.sync.min.f32`.  Disparities beyond D hold +inf, which no minimum
+// takes.  The four directions (2H + 2W lines) run in one launch through this
+// one routine, the direction a run-time argument, each writing its own
+// volume.
+// A step's costs and classes do not depend on the recursion.  The warp copies
+// the cost rows of the next PF steps into a shared-memory ring with
+// asynchronous copies: loads into a register ring did not stay in flight
+// (the warp's few scoreboards make the wait for the oldest one for the newest
+// too).  Rows are copied and stored as VEC consecutive floats per lane, whole
+// sectors per instruction, so with KPL != VEC a step's path costs pass
+// through shared memory on their way out (two passes over every sector made
+// 2.9 ms of 1482x994 D=256 where each lane copied its own 8).  The classes of 32 steps are
+// loaded at once and folded into one word per disparity, whose bit says
+// whether the pair agrees: with class loads in every step, even ones ahead,
+// the scan waited for them (380 to 450 us per launch at 694x554 D=128
+// against 240 without any).
+// Per launch, us (before: loads in registers, float differences, lanes
+// strided by 32 where D % 4 != 0): 694x554 D=128 242 (382), at 5.9 TB/s of
+// its 1.42 GB; 451x319 D=70 98 (262); 901x600 D=192 554 (990); 1482x994
+// D=256 1990 (2673).  A ring of eight steps, blocks of 4 to 16 lines, and a
+// cap on registers for more resident lines changed nothing; two steps lose
+// 60 us at D=128.
+template <int KPL>
+constexpr int sgm_depth() { return KPL <= 12 ? 4 : 2; }
+
+template <int BYTES>
+__device__ __forceinline__ void copy_async(uint32_t dst, const void* src, bool on) {
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(on ? 16 : 0) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(BYTES), "r"(on ? BYTES : 0) : "memory");
+}
+
+template <int KPL, bool FULL, int VEC>
+__global__ void __launch_bounds__(64) sgm_kernel(SgmCodes g, const float* __restrict__ in, int H, int W, int D,
+                                               SgmParams sp, SgmOut o) {
+  constexpr int PF = sgm_depth<KPL>(), NV = (KPL + VEC - 1) / VEC, WORDS = 32 * NV * VEC;
+  constexpr bool kStaged = KPL != VEC;  // rows pass through shared memory between lanes
+  extern __shared__ __align__(16) float sgm_ring[];
   const int lane = threadIdx.x & 31;
-  const int nsteps = DIR <= 1 ? W : H;
-  const int dx = DIR == 0 ? 1 : DIR == 1 ? -1 : 0;
+  int line = (int)(((int64_t)blockIdx.x * 64 + threadIdx.x) >> 5), dir;
+  if (line < 2 * H) {
+    dir = line >= H;
+    line -= dir * H;
+  } else {
+    line -= 2 * H;
+    if (line >= 2 * W) return;
+    dir = 2 + (line >= W);
+    line -= (dir - 2) * W;
+  }
+  float* __restrict__ out = dir == 0 ? o.dir[0] : dir == 1 ? o.dir[1] : dir == 2 ? o.dir[2] : o.dir[3];
   const float inf = __int_as_float(0x7f800000);
+  const bool horizontal = dir <= 1;
+  const int nsteps = horizontal ? W : H;
   // penalties of post.cu:239-248; the alpha1 split of :252/:255 applies to
   // the d-1 term in direction 2 and to the d+1 term in direction 3
   const float p1[3] = {sp.pi1, sp.pi1 / (sp.q1 * sp.q2), sp.pi1 / sp.q1};
@@ -95,294 +163,183 @@ __device__ __noinline__ void sgm_scan(const SgmGrad& g, const float* __restrict_
   float p1lo[3], p1hi[3];
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    p1lo[c] = DIR == 2 ? p1[c] / sp.alpha1 : p1[c];
-    p1hi[c] = DIR == 3 ? p1[c] / sp.alpha1 : p1[c];
+    p1lo[c] = dir == 2 ? p1[c] / sp.alpha1 : p1[c];
+    p1hi[c] = dir == 3 ? p1[c] / sp.alpha1 : p1[c];
   }
-  const float* gl = DIR <= 1 ? g.lh : g.lv;
-  const float* gr = DIR <= 1 ? g.rh : g.rv;
-  // the difference to the previous pixel of the scan sits at the later of
-  // the two pixels in the neighbour-difference images
-  const int gshift = DIR == 1 ? 1 : DIR == 3 ? W : 0;
-  // step s visits pixel p0 + s * pstep, column x0 + s * dx
-  const int64_t p0 = DIR == 0 ? (int64_t)line * W
-                   : DIR == 1 ? (int64_t)line * W + W - 1
-                   : DIR == 2 ? (int64_t)line
+  // step t visits pixel p0 + t * pstep; the difference to the step before
+  // sits at the later (right or lower) of the two pixels
+  const int64_t p0 = dir == 0 ? (int64_t)line * W
+                   : dir == 1 ? (int64_t)line * W + W - 1
+                   : dir == 2 ? (int64_t)line
                               : (int64_t)(H - 1) * W + line;
-  const int64_t pstep = DIR == 0 ? 1 : DIR == 1 ? -1 : DIR == 2 ? (int64_t)W : -(int64_t)W;
-  const int x0 = DIR == 0 ? 0 : DIR == 1 ? W - 1 : line;
-  // post.cu:232-237: D2 = 10 when the matching pixel xx = x + d*direction
-  // or its predecessor xx - dx leaves the image, i.e. unless
-  // max(0, dx) <= xx < min(W, W + dx)
-  const int s = sp.direction;
-  const int xlo = max(0, dx);
-  const unsigned xspan = (unsigned)(min(W, W + dx) - xlo);
-
-  struct Step {
-    float cost[KPL], d2[KPL];
-    float d1;
-  };
-  auto load = [&](int step, Step& st) {
-    const int64_t ind2 = p0 + step * pstep;
-    const int xl = x0 + step * dx + lane * s - xlo;  // xx - xlo of this lane's d = lane
-    const float* src = in + ind2 * D + lane;
-    const float* grp = gr + ind2 + gshift + lane * s;
-    st.d1 = step > 0 ? gl[ind2 + gshift] : 0.0f;
+  const int64_t pstep = dir == 0 ? 1 : dir == 1 ? -1 : dir == 2 ? (int64_t)W : -(int64_t)W;
+  const int s = sp.direction, d0 = KPL * lane;
+  const float* lsrc = in + p0 * D + lane * VEC;  // this lane's vectors: floats (v * 32 + lane) * VEC of a row
+  const int64_t vstride = pstep * D;
+  // the class position of step t (the later, right or lower, pixel of the
+  // pair): t forwards, nsteps - t backwards; agree[k] bit c & 31: at position
+  // c the classes of disparity d0 + k agree (both below tau or both above),
+  // low: the left one is below
+  const int forward = dir == 0 || dir == 2 ? 1 : -1;
+  int c = forward > 0 ? 1 : nsteps - 1;
+  uint32_t agree[KPL], low = 0;
+  const int gw = (W + 31) / 32;
+  const uint2 outside = make_uint2(10.0f < sp.tau_so ? 0xFFFFFFFFu : 0u, 10.0f > sp.tau_so ? 0xFFFFFFFFu : 0u);
+  auto load_classes = [&]() {
+    const int group = c >> 5;
+    const uint2 l = __ldg(horizontal ? g.left_h + (int64_t)line * gw + group : g.left_v + (int64_t)group * W + line);
+    const uint2* __restrict__ row = horizontal ? g.right_h + (int64_t)line * gw : g.right_v + (int64_t)group * W;
 #pragma unroll
     for (int k = 0; k < KPL; k++) {
-      const bool dk = FULL || lane + 32 * k < D;
-      st.cost[k] = dk ? src[32 * k] : inf;
-      const bool inside = (unsigned)(xl + 32 * k * s) < xspan;
-      st.d2[k] = (step > 0 && dk && inside) ? grp[32 * k * s] : 10.0f;
-    }
-  };
-  float prev[KPL];
-  Step ring[PF];
-#pragma unroll
-  for (int i = 0; i < PF; i++)
-    if (i < nsteps) load(i, ring[i]);
-  for (int s0 = 0; s0 < nsteps; s0 += PF) {
-#pragma unroll
-    for (int i = 0; i < PF; i++) {
-      const int step = s0 + i;
-      if (step >= nsteps) break;
-      const Step cur = ring[i];
-      if (step + PF < nsteps) load(step + PF, ring[i]);
-      float L[KPL];
-      if (step == 0) {
-#pragma unroll
-        for (int k = 0; k < KPL; k++) L[k] = cur.cost[k];
+      uint2 q = outside;
+      if (horizontal) {
+        const int p = 32 * group + (d0 + k) * s, w = p >> 5;  // right pixel of the group's first position
+        const uint2 a = (unsigned)w < (unsigned)gw ? __ldg(row + w) : outside;
+        const uint2 b = (unsigned)(w + 1) < (unsigned)gw ? __ldg(row + w + 1) : outside;
+        q = make_uint2(__funnelshift_r(a.x, b.x, p), __funnelshift_r(a.y, b.y, p));
       } else {
-        float mn = prev[0];
-#pragma unroll
-        for (int k = 1; k < KPL; k++) mn = fminf(mn, prev[k]);
-#pragma unroll
-        for (int o = 16; o; o >>= 1) mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-        const bool d1lo = cur.d1 < sp.tau_so, d1hi = cur.d1 > sp.tau_so;
-        // class 0 (both gradients below tau) or 1 (both above) when the step's
-        // D1 allows it and D2 agrees, else class 2
-        const float a2 = d1lo ? p2[0] : p2[1], a1lo = d1lo ? p1lo[0] : p1lo[1],
-                    a1hi = d1lo ? p1hi[0] : p1hi[1];
-#pragma unroll
-        for (int k = 0; k < KPL; k++) {
-          const int d = lane + 32 * k;
-          // neighbours d-1 and d+1 of the previous step: lane 31 hands lane 0
-          // its value of the previous disparity block, lane 0 hands lane 31
-          // its value of the next one
-          const float up = lane == 31 ? prev[k > 0 ? k - 1 : 0] : prev[k];
-          const float dn = lane == 0 ? prev[k + 1 < KPL ? k + 1 : k] : prev[k];
-          const float lo = __shfl_sync(0xffffffffu, up, (lane + 31) & 31);
-          const float hi = __shfl_sync(0xffffffffu, dn, (lane + 1) & 31);
-          const float D2 = cur.d2[k];
-          const bool ca = d1lo ? D2 < sp.tau_so : (d1hi && D2 > sp.tau_so);
-          float cost = fminf(prev[k], mn + (ca ? a2 : p2[2]));
-          if (d - 1 >= 0) cost = fminf(cost, lo + (ca ? a1lo : p1lo[2]));
-          if (d + 1 < D) cost = fminf(cost, hi + (ca ? a1hi : p1hi[2]));
-          L[k] = (FULL || d < D) ? cur.cost[k] + cost - mn : inf;
-        }
+        const int p = line + (d0 + k) * s;
+        if ((unsigned)p < (unsigned)W) q = __ldg(row + p);
       }
-      float* dst = out + (p0 + step * pstep) * D + lane;
-#pragma unroll
-      for (int k = 0; k < KPL; k++) {
-        if (FULL || lane + 32 * k < D) dst[32 * k] = L[k];
-        prev[k] = L[k];
-      }
+      agree[k] = (l.x & q.x) | (l.y & q.y);
     }
-  }
-}
-
-// The same scan with each lane holding KPL CONSECUTIVE disparities, d =
-// KPL * lane + k (KPL a multiple of 4, D a multiple of 4): a step's path
-// costs are KPL/4 float4 loads and stores per lane, the d-1 / d+1
-// neighbours are in the lane's own registers except at its two ends (two
-// shuffles per step instead of two per register), and the minimum over d
-// is one `redux.sync.min.f32`.  The matching direction S (+-1) and FULL
-// (D == 32 * KPL) are compile-time, the step's addresses advance by
-// constant strides, and step 0 (whose path cost is its cost) loads no
-// image terms.  Per element the arithmetic and its order are those of
-// sgm_scan, so the results are the same bit for bit.
-template <int KPL, int PF, bool FULL, int S>
-__device__ __noinline__ void sgm_scan_c(const SgmGrad& g, const float* __restrict__ in, int H, int W, int D,
-                                        const SgmParams& sp, int line, float* __restrict__ out, const int DIR) {
-  static_assert(KPL % 4 == 0, "float4 path costs");
-  constexpr int NV = KPL / 4;
-  const int lane = threadIdx.x & 31;
-  const int nsteps = DIR <= 1 ? W : H;
-  const int dx = DIR == 0 ? 1 : DIR == 1 ? -1 : 0;
-  const float inf = __int_as_float(0x7f800000);
-  const float p1[3] = {sp.pi1, sp.pi1 / (sp.q1 * sp.q2), sp.pi1 / sp.q1};
-  const float p2[3] = {sp.pi2, sp.pi2 / (sp.q1 * sp.q2), sp.pi2 / sp.q1};
-  float p1lo[3], p1hi[3];
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    p1lo[c] = DIR == 2 ? p1[c] / sp.alpha1 : p1[c];
-    p1hi[c] = DIR == 3 ? p1[c] / sp.alpha1 : p1[c];
-  }
-  const float* gl = DIR <= 1 ? g.lh : g.lv;
-  const float* gr = DIR <= 1 ? g.rh : g.rv;
-  const int gshift = DIR == 1 ? 1 : DIR == 3 ? W : 0;
-  const int64_t p0 = DIR == 0 ? (int64_t)line * W
-                   : DIR == 1 ? (int64_t)line * W + W - 1
-                   : DIR == 2 ? (int64_t)line
-                              : (int64_t)(H - 1) * W + line;
-  const int64_t pstep = DIR == 0 ? 1 : DIR == 1 ? -1 : DIR == 2 ? (int64_t)W : -(int64_t)W;
-  const int x0 = DIR == 0 ? 0 : DIR == 1 ? W - 1 : line;
-  const int xlo = max(0, dx);
-  const unsigned xspan = (unsigned)(min(W, W + dx) - xlo);
-  const int d0 = KPL * lane;  // this lane's first disparity
-  const bool lane_on = FULL || d0 < D;  // D % 4 == 0: a float4 is all in or all out
-
-  struct Step {
-    float cost[KPL], d2[KPL];
-    float d1;
+    low = l.x;
   };
-  // the next step to load: its pixel's path-cost row, its image terms
-  // (D1 at gl[.], D2 at gr[. + d*S]) and the matching column of its first
-  // disparity relative to the span where D2 exists
-  const float* lsrc = in + p0 * D + d0;
-  const float* lgl = gl + p0 + gshift;
-  const float* lgr = gr + p0 + gshift + d0 * S;
-  int lxl = x0 + d0 * S - xlo;
-  const int64_t vstride = pstep * D;
-  auto load_costs = [&](Step& st) {
-    const float4* src = reinterpret_cast<const float4*>(lsrc);
+  auto vec_on = [&](int v) { return FULL ? (KPL % VEC == 0 || (v * 32 + lane) * VEC < D) : (v * 32 + lane) * VEC < D; };
+  float* ring = sgm_ring + (threadIdx.x >> 5) * (PF + kStaged) * WORDS;
+  float* stage = ring + PF * WORDS;
+  const uint32_t ring_at = (uint32_t)__cvta_generic_to_shared(ring);
+  auto load = [&](int slot) {  // the next step's costs
+    const uint32_t at = ring_at + slot * (WORDS * 4);
 #pragma unroll
-    for (int v = 0; v < NV; v++) {
-      const bool on = lane_on && (FULL || d0 + 4 * v < D);
-      const float4 c = on ? src[v] : make_float4(inf, inf, inf, inf);
-      st.cost[4 * v] = c.x;
-      st.cost[4 * v + 1] = c.y;
-      st.cost[4 * v + 2] = c.z;
-      st.cost[4 * v + 3] = c.w;
-    }
+    for (int v = 0; v < NV; v++)  // with VEC > 1, D % VEC == 0: all in or all out
+      copy_async<4 * VEC>(at + (v * 32 + lane) * VEC * 4, lsrc + v * 32 * VEC, vec_on(v));
     lsrc += vstride;
   };
-  // a step >= 1: costs, D1 and the per-d D2 (10 where the matching pixel
-  // or its predecessor leaves the image, post.cu:232-237)
-  auto load = [&](Step& st) {
-    load_costs(st);
-    st.d1 = *lgl;
+  float* ldst = out + p0 * D + lane * VEC;
+  // KPL floats between registers and their place in a row in shared memory
+  auto get = [&](const float* at, float* f) {
+    if constexpr (KPL % 4 == 0) {
 #pragma unroll
-    for (int k = 0; k < KPL; k++) {
-      const bool inside = (FULL || d0 + k < D) && (unsigned)(lxl + k * S) < xspan;
-      st.d2[k] = inside ? lgr[k * S] : 10.0f;
+      for (int k = 0; k < KPL; k += 4) *reinterpret_cast<float4*>(f + k) = *reinterpret_cast<const float4*>(at + d0 + k);
+    } else if constexpr (KPL % 2 == 0) {
+#pragma unroll
+      for (int k = 0; k < KPL; k += 2) *reinterpret_cast<float2*>(f + k) = *reinterpret_cast<const float2*>(at + d0 + k);
+    } else {
+#pragma unroll
+      for (int k = 0; k < KPL; k++) f[k] = at[d0 + k];
     }
-    lgl += pstep;
-    lgr += pstep;
-    lxl += dx;
   };
-  float prev[KPL];
-  Step ring[PF];
-  {
-    // step 0: the path cost is the cost
-    Step st0;
-    load_costs(st0);
-    lgl += pstep;
-    lgr += pstep;
-    lxl += dx;
+  auto put = [&](float* at, const float* f) {
+    if constexpr (KPL % 4 == 0) {
 #pragma unroll
-    for (int k = 0; k < KPL; k++) prev[k] = st0.cost[k];
-    float4* dst = reinterpret_cast<float4*>(out + p0 * D + d0);
+      for (int k = 0; k < KPL; k += 4) *reinterpret_cast<float4*>(at + d0 + k) = *reinterpret_cast<const float4*>(f + k);
+    } else if constexpr (KPL % 2 == 0) {
 #pragma unroll
-    for (int v = 0; v < NV; v++)
-      if (lane_on && (FULL || d0 + 4 * v < D))
-        dst[v] = make_float4(prev[4 * v], prev[4 * v + 1], prev[4 * v + 2], prev[4 * v + 3]);
-  }
+      for (int k = 0; k < KPL; k += 2) *reinterpret_cast<float2*>(at + d0 + k) = *reinterpret_cast<const float2*>(f + k);
+    } else {
 #pragma unroll
-  for (int i = 0; i < PF; i++)
-    if (1 + i < nsteps) load(ring[i]);
-  float* ldst = out + (p0 + pstep) * D + d0;
-  for (int s0 = 1; s0 < nsteps; s0 += PF) {
-#pragma unroll
-    for (int i = 0; i < PF; i++) {
-      const int step = s0 + i;
-      if (step >= nsteps) break;
-      const Step cur = ring[i];
-      if (step + PF < nsteps) load(ring[i]);
-      float m = fminf(fminf(prev[0], prev[1]), fminf(prev[2], prev[3]));
-#pragma unroll
-      for (int k = 4; k < KPL; k++) m = fminf(m, prev[k]);
-      float mn;
-      asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(mn) : "f"(m));
-      // the neighbours across the lane's ends: d0 - 1 from the previous
-      // lane's last register, d0 + KPL from the next lane's first
-      const float lo0 = __shfl_up_sync(0xffffffffu, prev[KPL - 1], 1);
-      const float hiL = __shfl_down_sync(0xffffffffu, prev[0], 1);
-      const bool d1lo = cur.d1 < sp.tau_so, d1hi = cur.d1 > sp.tau_so;
-      const float a2 = d1lo ? p2[0] : p2[1], a1lo = d1lo ? p1lo[0] : p1lo[1], a1hi = d1lo ? p1hi[0] : p1hi[1];
-      float L[KPL];
-#pragma unroll
-      for (int k = 0; k < KPL; k++) {
-        const int d = d0 + k;
-        const float lo = k > 0 ? prev[k - 1] : lo0;
-        const float hi = k + 1 < KPL ? prev[k + 1] : hiL;
-        const float D2 = cur.d2[k];
-        const bool ca = d1lo ? D2 < sp.tau_so : (d1hi && D2 > sp.tau_so);
-        float cost = fminf(prev[k], mn + (ca ? a2 : p2[2]));
-        if (k > 0 || d - 1 >= 0) cost = fminf(cost, lo + (ca ? a1lo : p1lo[2]));
-        if (FULL ? (k + 1 < KPL || lane < 31) : d + 1 < D) cost = fminf(cost, hi + (ca ? a1hi : p1hi[2]));
-        L[k] = (FULL || d < D) ? cur.cost[k] + cost - mn : inf;
-      }
-      float4* dst = reinterpret_cast<float4*>(ldst);
+      for (int k = 0; k < KPL; k++) at[d0 + k] = f[k];
+    }
+  };
+  auto store = [&](const float* L) {
+    __align__(16) float f[NV * VEC];
+    if constexpr (kStaged) {
+      put(stage, L);
+      __syncwarp();
 #pragma unroll
       for (int v = 0; v < NV; v++)
-        if (lane_on && (FULL || d0 + 4 * v < D)) dst[v] = make_float4(L[4 * v], L[4 * v + 1], L[4 * v + 2], L[4 * v + 3]);
-      ldst += vstride;
 #pragma unroll
-      for (int k = 0; k < KPL; k++) prev[k] = L[k];
+        for (int k = 0; k < VEC; k++) f[v * VEC + k] = stage[(v * 32 + lane) * VEC + k];
+    } else {
+#pragma unroll
+      for (int k = 0; k < KPL; k++) f[k] = L[k];
     }
+#pragma unroll
+    for (int v = 0; v < NV; v++)
+      if (vec_on(v)) {
+        float* to = ldst + v * 32 * VEC;
+        if constexpr (VEC == 4) *reinterpret_cast<float4*>(to) = make_float4(f[4 * v], f[4 * v + 1], f[4 * v + 2], f[4 * v + 3]);
+        else if constexpr (VEC == 2) *reinterpret_cast<float2*>(to) = make_float2(f[2 * v], f[2 * v + 1]);
+        else *to = f[v];
+      }
+    ldst += vstride;
+  };
+  float prev[KPL];
+#pragma unroll
+  for (int k = 0; k < KPL; k++)  // step 0: the path cost is the cost
+    prev[k] = FULL || d0 + k < D ? __ldg(in + p0 * D + d0 + k) : inf;
+  store(prev);
+  lsrc += vstride;
+  if (nsteps > 1) load_classes();
+#pragma unroll
+  for (int i = 0; i < PF; i++) {  // step 1 + i in slot i, one group per step
+    if (1 + i < nsteps) load(i);
+    asm volatile("cp.async.commit_group;" ::: "memory");
   }
-}
-
-template <int KPL, int PF, bool FULL, int S>
-__global__ void __launch_bounds__(128) sgm4c_kernel(SgmGrad g, const float* __restrict__ in, int H, int W,
-                                                    int D, SgmParams sp, SgmOut o) {
-  const int warp = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  int dir = -1, line = 0;
-  if (warp < H) {
-    dir = 0;
-    line = warp;
-  } else if (warp < 2 * H) {
-    dir = 1;
-    line = warp - H;
-  } else if (warp < 2 * H + W) {
-    dir = 2;
-    line = warp - 2 * H;
-  } else if (warp < 2 * H + 2 * W) {
-    dir = 3;
-    line = warp - 2 * H - W;
+  int slot = 0;
+  for (int t = 1; t < nsteps; t++) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(PF - 1) : "memory");
+    if (kStaged) __syncwarp();  // the row's copies of every lane; the staged row of the step before is out
+    __align__(16) float cost[KPL];
+    get(ring + slot * WORDS, cost);
+    const uint32_t bit = 1u << (c & 31);
+    float m = prev[0];
+#pragma unroll
+    for (int k = 1; k < KPL; k++) m = fminf(m, prev[k]);
+    float mn;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(mn) : "f"(m));
+    // the neighbours across the lane's ends: d0 - 1 from the previous
+    // lane's last register, d0 + KPL from the next lane's first
+    float below = __shfl_up_sync(0xffffffffu, prev[KPL - 1], 1), above = __shfl_down_sync(0xffffffffu, prev[0], 1);
+    if (lane == 0) below = inf;
+    if (lane == 31) above = inf;
+    // penalty class 0 (both below tau) or 1 (both above) where the classes agree, else 2
+    const bool below_tau = low & bit;
+    const float a2 = mn + (below_tau ? p2[0] : p2[1]), c2 = mn + p2[2];
+    const float alo = below_tau ? p1lo[0] : p1lo[1], ahi = below_tau ? p1hi[0] : p1hi[1];
+    __align__(16) float L[KPL];
+#pragma unroll
+    for (int k = 0; k < KPL; k++) {
+      const bool same = agree[k] & bit;
+      const float lo = (k > 0 ? prev[k > 0 ? k - 1 : 0] : below) + (same ? alo : p1lo[2]);
+      const float hi = (k + 1 < KPL ? prev[k + 1 < KPL ? k + 1 : 0] : above) + (same ? ahi : p1hi[2]);
+      const float best = fminf(fminf(fminf(prev[k], same ? a2 : c2), lo), hi);
+      L[k] = FULL || d0 + k < D ? cost[k] + best - mn : inf;
+    }
+    store(L);
+#pragma unroll
+    for (int k = 0; k < KPL; k++) prev[k] = L[k];
+    // every lane has read the slot (its values are in registers): refill it with step t + PF
+    if (t + PF < nsteps) load(slot);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    slot = slot + 1 == PF ? 0 : slot + 1;
+    c += forward;
+    if ((c & 31) == (forward > 0 ? 0 : 31) && t + 1 < nsteps) load_classes();
   }
-  if (dir >= 0) sgm_scan_c<KPL, PF, FULL, S>(g, in, H, W, D, sp, line, o.dir[dir], dir);
-}
-
-template <int KPL, int PF, bool FULL>
-__global__ void __launch_bounds__(128) sgm4_kernel(SgmGrad g, const float* __restrict__ in, int H,
-                                                   int W, int D, SgmParams sp, SgmOut o) {
-  const int warp = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  int dir = -1, line = 0;
-  if (warp < H) {
-    dir = 0;
-    line = warp;
-  } else if (warp < 2 * H) {
-    dir = 1;
-    line = warp - H;
-  } else if (warp < 2 * H + W) {
-    dir = 2;
-    line = warp - 2 * H;
-  } else if (warp < 2 * H + 2 * W) {
-    dir = 3;
-    line = warp - 2 * H - W;
-  }
-  if (dir >= 0) sgm_scan<KPL, PF, FULL>(g, in, H, W, D, sp, line, o.dir[dir], dir);
 }
 
 // out = base + (((L0 + L1) + L2) + L3) * scale over n elements (base may be
 // out itself, or null for 0): the four directions summed as post.cu
-// sgm_w adds them (directions in order 0..3).
-__global__ void sgm_combine_kernel(SgmOut o, int64_t n, const float* base, float scale,
-                                   float* out) {
+// sgm_w adds them (directions in order 0..3).  V: float4 (n / 4 of them) or float.
+__device__ __forceinline__ float sgm_sum(float a, float b, float c, float d) { return ((a + b) + c) + d; }
+__device__ __forceinline__ float4 sgm_sum(float4 a, float4 b, float4 c, float4 d) {
+  return make_float4(sgm_sum(a.x, b.x, c.x, d.x), sgm_sum(a.y, b.y, c.y, d.y), sgm_sum(a.z, b.z, c.z, d.z),
+                     sgm_sum(a.w, b.w, c.w, d.w));
+}
+__device__ __forceinline__ float scaled(float s, float k) { return s * k; }
+__device__ __forceinline__ float4 scaled(float4 s, float k) { return make_float4(s.x * k, s.y * k, s.z * k, s.w * k); }
+__device__ __forceinline__ float added(float b, float s, float k) { return b + s * k; }
+__device__ __forceinline__ float4 added(float4 b, float4 s, float k) {
+  return make_float4(b.x + s.x * k, b.y + s.y * k, b.z + s.z * k, b.w + s.w * k);
+}
+template <class V>
+__global__ void __launch_bounds__(256) sgm_combine_kernel(const V* __restrict__ l0, const V* __restrict__ l1,
+                                                        const V* __restrict__ l2, const V* __restrict__ l3, int64_t n,
+                                                        const V* base, float scale, V* out) {
   GRID_STRIDE(i, n) {
-    const float s = ((o.dir[0][i] + o.dir[1][i]) + o.dir[2][i]) + o.dir[3][i];
-    out[i] = base ? base[i] + s * scale : s * scale;
+    const V s = sgm_sum(l0[i], l1[i], l2[i], l3[i]);
+    out[i] = base ? added(base[i], s, scale) : scaled(s, scale);
   }
 }
 
@@ -1305,81 +1262,53 @@ int launch_cross(const float* img, int64_t H, int64_t W, int L1, float tau1, flo
   return check_launch("cross");
 }
 
-int launch_sgm_grad(const float* imL, const float* imR, int64_t H, int64_t W, SgmGrad* g,
-                    cudaStream_t st) {
-  grad_kernel<<<grid_for(H * W, 256), 256, 0, st>>>(imL, H, W, g->lh, g->lv);
-  grad_kernel<<<grid_for(H * W, 256), 256, 0, st>>>(imR, H, W, g->rh, g->rv);
-  return check_launch("sgm_grad");
+int launch_sgm_codes(const float* imL, const float* imR, int64_t H, int64_t W, float tau, const SgmCodes& g,
+                     cudaStream_t st) {
+  sgm_codes_kernel<<<grid_for(2 * ((H + 31) / 32) * ((W + 31) / 32) * 32, 128), 128, 0, st>>>(imL, imR, (int)H, (int)W,
+                                                                                              tau, g);
+  return check_launch("sgm_codes");
 }
 
-// prefetch: steps loaded ahead (1, 2 or 4; 0 = the default: shallow
-// prefetch keeps the scan at ~80 registers, measured faster than deeper
-// rings, whose registers cost more occupancy than they hide latency).
-// The results do not depend on it.
-template <int KPL>
-static void sgm4_launch(const SgmGrad& g, const float* in, int H, int W, int D, const SgmParams& sp,
-                        const SgmOut& o, cudaStream_t st, int prefetch) {
-  const int lines = 2 * H + 2 * W;
-  const int blocks = (lines * 32 + 127) / 128;
-  constexpr int PF0 = KPL <= 2 ? 4 : KPL <= 8 ? 2 : 1;
-  const int pf = prefetch > 0 && KPL <= 8 ? prefetch : PF0;
-  if (D == 32 * KPL) {  // every lane's disparities exist: no bounds tests on d
-    if (pf >= 4) sgm4_kernel<KPL, KPL <= 8 ? 4 : 1, true><<<blocks, 128, 0, st>>>(g, in, H, W, D, sp, o);
-    else if (pf >= 2) sgm4_kernel<KPL, KPL <= 8 ? 2 : 1, true><<<blocks, 128, 0, st>>>(g, in, H, W, D, sp, o);
-    else sgm4_kernel<KPL, 1, true><<<blocks, 128, 0, st>>>(g, in, H, W, D, sp, o);
-  } else {
-    if (pf >= 4) sgm4_kernel<KPL, KPL <= 8 ? 4 : 1, false><<<blocks, 128, 0, st>>>(g, in, H, W, D, sp, o);
-    else if (pf >= 2) sgm4_kernel<KPL, KPL <= 8 ? 2 : 1, false><<<blocks, 128, 0, st>>>(g, in, H, W, D, sp, o);
-    else sgm4_kernel<KPL, 1, false><<<blocks, 128, 0, st>>>(g, in, H, W, D, sp, o);
-  }
-}
-
-// The consecutive-disparity scan (sgm_scan_c) for D a multiple of 4 in
-// (64, 512] with 16-byte aligned volumes; 2 steps loaded ahead (default,
-// measured faster at 694x554 D=128: post 2.74 against 2.88 ms) or 1.
-template <int KPL>
-static void sgm4c_launch(const SgmGrad& g, const float* in, int H, int W, int D, const SgmParams& sp,
-                         const SgmOut& o, cudaStream_t st, int prefetch) {
-  const int lines = 2 * H + 2 * W;
-  const int blocks = (lines * 32 + 127) / 128;
-  const bool full = D == 32 * KPL;
-#define SGM4C(PF_, FULL_, S_) sgm4c_kernel<KPL, PF_, FULL_, S_><<<blocks, 128, 0, st>>>(g, in, H, W, D, sp, o)
-  if (sp.direction > 0) {
-    if (prefetch == 1) { if (full) SGM4C(1, true, 1); else SGM4C(1, false, 1); }
-    else { if (full) SGM4C(2, true, 1); else SGM4C(2, false, 1); }
-  } else {
-    if (prefetch == 1) { if (full) SGM4C(1, true, -1); else SGM4C(1, false, -1); }
-    else { if (full) SGM4C(2, true, -1); else SGM4C(2, false, -1); }
-  }
-#undef SGM4C
-}
-
-static bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
-
-int launch_sgm4(const SgmGrad& g, const float* in, int64_t H, int64_t W, int D, const SgmParams& sp,
-                const SgmOut& o, cudaStream_t st, int prefetch) {
-  const int kpl = (D + 31) / 32;
-  const int h = (int)H, w = (int)W;
-  const bool vec = D % 4 == 0 && D > 64 && D <= 512 && aligned16(in) && aligned16(o.dir[0]) &&
-                   aligned16(o.dir[1]) && aligned16(o.dir[2]) && aligned16(o.dir[3]);
-  if (vec) {
-    if (D <= 128) sgm4c_launch<4>(g, in, h, w, D, sp, o, st, prefetch);
-    else if (D <= 256) sgm4c_launch<8>(g, in, h, w, D, sp, o, st, prefetch);
-    else sgm4c_launch<16>(g, in, h, w, D, sp, o, st, prefetch);
-    return check_launch("sgm4");
-  }
-  if (kpl <= 1) sgm4_launch<1>(g, in, h, w, D, sp, o, st, prefetch);
-  else if (kpl <= 2) sgm4_launch<2>(g, in, h, w, D, sp, o, st, prefetch);
-  else if (kpl <= 4) sgm4_launch<4>(g, in, h, w, D, sp, o, st, prefetch);
-  else if (kpl <= 8) sgm4_launch<8>(g, in, h, w, D, sp, o, st, prefetch);
-  else if (kpl <= 16) sgm4_launch<16>(g, in, h, w, D, sp, o, st, prefetch);
-  else sgm4_launch<32>(g, in, h, w, D, sp, o, st, prefetch);
+template <int KPL, bool FULL, int VEC>
+static int sgm_launch(const SgmCodes& g, const float* in, int H, int W, int D, const SgmParams& sp, const SgmOut& o,
+                      cudaStream_t st) {
+  constexpr int words = 32 * ((KPL + VEC - 1) / VEC) * VEC, smem = 2 * (sgm_depth<KPL>() + (KPL != VEC)) * words * 4;
+  static_assert(smem <= 48 * 1024, "no opt-in to more shared memory");
+  sgm_kernel<KPL, FULL, VEC><<<(2 * H + 2 * W + 1) / 2, 64, smem, st>>>(g, in, H, W, D, sp, o);
   return check_launch("sgm4");
+}
+
+int launch_sgm4(const SgmCodes& g, const float* in, int64_t H, int64_t W, int D, const SgmParams& sp,
+                const SgmOut& o, cudaStream_t st) {
+  const int h = (int)H, w = (int)W;
+  const uintptr_t at = (uintptr_t)in | (uintptr_t)o.dir[0] | (uintptr_t)o.dir[1] | (uintptr_t)o.dir[2] | (uintptr_t)o.dir[3];
+  const int vec = D % 4 == 0 && at % 16 == 0 ? 4 : D % 2 == 0 && at % 8 == 0 ? 2 : 1;
+  // the fewest disparities per lane that cover D in 32 lanes, rows in the
+  // widest vectors that D and the volumes' alignment allow
+#define SGM(KPL)                                                                                        \
+  if (D <= 32 * KPL) {                                                                                  \
+    if (vec == 4 && D == 32 * KPL) return sgm_launch<KPL, true, 4>(g, in, h, w, D, sp, o, st);          \
+    if (vec == 4) return sgm_launch<KPL, false, 4>(g, in, h, w, D, sp, o, st);                          \
+    if (vec == 2) return sgm_launch<KPL, false, 2>(g, in, h, w, D, sp, o, st);                          \
+    return sgm_launch<KPL, false, 1>(g, in, h, w, D, sp, o, st);                                        \
+  }
+  SGM(1) SGM(2) SGM(3) SGM(4) SGM(5) SGM(6) SGM(7) SGM(8) SGM(10) SGM(12) SGM(16) SGM(24) SGM(32)
+#undef SGM
+  return set_error(CBMV_ERANGE, "D=%d beyond 1024", D);
 }
 
 int launch_sgm_combine(const SgmOut& o, int64_t n, const float* base, float scale, float* out,
                        cudaStream_t st) {
-  sgm_combine_kernel<<<grid_for(n, 256), 256, 0, st>>>(o, n, base, scale, out);
+  const uintptr_t at = (uintptr_t)o.dir[0] | (uintptr_t)o.dir[1] | (uintptr_t)o.dir[2] | (uintptr_t)o.dir[3] |
+                       (uintptr_t)base | (uintptr_t)out;
+  if (n % 4 == 0 && at % 16 == 0) {
+    auto f4 = [](const float* p) { return reinterpret_cast<const float4*>(p); };
+    sgm_combine_kernel<<<grid_for(n / 4, 256), 256, 0, st>>>(f4(o.dir[0]), f4(o.dir[1]), f4(o.dir[2]), f4(o.dir[3]), n / 4,
+                                                             f4(base), scale, reinterpret_cast<float4*>(out));
+  } else {
+    sgm_combine_kernel<float><<<grid_for(n, 256), 256, 0, st>>>(o.dir[0], o.dir[1], o.dir[2], o.dir[3], n, base, scale,
+                                                                out);
+  }
   return check_launch("sgm_combine");
 }
 
@@ -1538,14 +1467,13 @@ static int check_sgm(const float* imL, const float* imR, const float* in, int64_
   return CBMV_OK;
 }
 
-// scratch: the direction volumes, then the image differences
+// scratch: the direction volumes, then the image classes
 static int run_sgm(const float* imL, const float* imR, const float* in, int64_t H, int64_t W, int D,
                    const SgmParams& sp, float* out, float* scratch, cudaStream_t st) {
-  const int64_t HW = H * W, V = HW * D, S = (V + 3) / 4 * 4;  // every volume 16-byte aligned
+  const int64_t V = H * W * D, S = (V + 3) / 4 * 4;  // every volume 16-byte aligned
   SgmOut o{{scratch, scratch + S, scratch + 2 * S, scratch + 3 * S}};
-  float* gr = scratch + 4 * S;
-  SgmGrad g{gr, gr + HW, gr + 2 * HW, gr + 3 * HW};
-  int rc = launch_sgm_grad(imL, imR, H, W, &g, st);
+  const SgmCodes g = sgm_codes_at(scratch + 4 * S, H, W);
+  int rc = launch_sgm_codes(imL, imR, H, W, sp.tau_so, g, st);
   if (!rc) rc = launch_sgm4(g, in, H, W, D, sp, o, st);
   if (!rc) rc = launch_sgm_combine(o, V, out, 1.0f, out, st);
   return rc;
@@ -1553,7 +1481,7 @@ static int run_sgm(const float* imL, const float* imR, const float* in, int64_t 
 
 extern "C" int64_t cbmv_sgm_scratch_bytes(int64_t H, int64_t W, int D) {
   if (H <= 0 || W <= 0 || H > (1 << 30) || W > (1 << 30) || D <= 0 || D > 1024) return -1;
-  return (int64_t)sizeof(float) * (4 * ((H * W * D + 3) / 4 * 4) + 4 * H * W);
+  return (int64_t)sizeof(float) * 4 * ((H * W * D + 3) / 4 * 4) + sgm_codes_bytes(H, W);
 }
 
 extern "C" int cbmv_sgm_scratch(const float* imL, const float* imR, const float* in, int64_t H, int64_t W, int D,

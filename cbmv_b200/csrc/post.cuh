@@ -13,18 +13,28 @@ struct SgmParams {
 
 int launch_cross(const float* img, int64_t H, int64_t W, int L1, float tau1, float* out,
                  cudaStream_t st);
-// Neighbour differences of both normalised images (see post.cu grad_kernel).
-struct SgmGrad {
-  float *lh, *lv, *rh, *rv;
+// Classes of both normalised images' neighbour differences (see post.cu
+// sgm_codes_kernel), 32 positions per word pair: rows [H][ceil(W / 32)] and
+// columns [ceil(H / 32)][W] of each image, in 8-byte aligned memory.
+struct SgmCodes {
+  uint2 *left_h, *left_v, *right_h, *right_v;
 };
-int launch_sgm_grad(const float* imL, const float* imR, int64_t H, int64_t W, SgmGrad* g,
-                    cudaStream_t st);
+inline int64_t sgm_codes_bytes(int64_t H, int64_t W) {
+  return 2 * (H * ((W + 31) / 32) + (H + 31) / 32 * W) * (int64_t)sizeof(uint2);
+}
+inline SgmCodes sgm_codes_at(void* at, int64_t H, int64_t W) {
+  uint2* c = static_cast<uint2*>(at);
+  const int64_t nh = H * ((W + 31) / 32), nv = (H + 31) / 32 * W;
+  return SgmCodes{c, c + nh, c + nh + nv, c + 2 * nh + nv};
+}
+int launch_sgm_codes(const float* imL, const float* imR, int64_t H, int64_t W, float tau, const SgmCodes& g,
+                     cudaStream_t st);
 // Path costs of the four scan directions, one volume each.
 struct SgmOut {
   float* dir[4];
 };
-int launch_sgm4(const SgmGrad& g, const float* in, int64_t H, int64_t W, int D, const SgmParams& sp,
-                const SgmOut& o, cudaStream_t st, int prefetch = 0);
+int launch_sgm4(const SgmCodes& g, const float* in, int64_t H, int64_t W, int D, const SgmParams& sp,
+                const SgmOut& o, cudaStream_t st);
 // out = base + (((L0 + L1) + L2) + L3) * scale; base may be null or out.
 int launch_sgm_combine(const SgmOut& o, int64_t n, const float* base, float scale, float* out,
                        cudaStream_t st);
