@@ -309,7 +309,7 @@ int launch_features_gather(const double* const* vols, const double* stats, int64
 // ---------------------------------------------- float32 row statistics
 // The classifier network's row statistics (min, 1/den) in float32 from
 // float32 volumes (the learned path never needs the float64 features):
-// statsf[(m*2 + view)*HW + p], min = 2^31 and 1/den = 0 where the row holds
+// statsf[(m*2 + view)*HW + p], min = -e and 1/den = 0 where the row holds
 // only sentinels.  All four matchers in one launch (blockIdx.y = matcher).
 struct VolsF {
   const float* v[4];
@@ -317,8 +317,9 @@ struct VolsF {
 static __constant__ float kInvSigmaF32[4] = {(float)(1.0 / (2.0 * 8 * 8)), (float)(1.0 / 0.02),
                                              (float)(1.0 / (2.0 * 100 * 100)), (float)(1.0 / (2.0 * 100 * 100))};
 
-__device__ __forceinline__ float2 stats_pair(float mn, float den) {
-  return mn == kRandMaxF ? make_float2(kRandMaxF, 0.0f) : make_float2(mn, 1.0f / den);
+// of matcher m; a row of sentinels has min = -e, so that its ratio (min + e) / (c + e) is 0, and 1/den = 0
+__device__ __forceinline__ float2 stats_pair(int m, float mn, float den) {
+  return mn == kRandMaxF ? make_float2(-kEpsF[m], 0.0f) : make_float2(mn, 1.0f / den);
 }
 
 // view 0: one warp per pixel, the pixel's D costs are contiguous
@@ -359,7 +360,7 @@ __global__ void stats_f32_left_kernel(VolsF vols, int64_t HW, int D, float2* __r
       }
     }
     for (int o = 16; o; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
-    if (lane == 0) statsf[(int64_t)(m * 2) * HW + p] = stats_pair(mn, den);
+    if (lane == 0) statsf[(int64_t)(m * 2) * HW + p] = stats_pair(m, mn, den);
   }
 }
 
@@ -408,7 +409,7 @@ __global__ void __launch_bounds__(RS_PIX) stats_f32_right_kernel(VolsF vols, int
       }
     }
   }
-  if (xr < W) statsf[(int64_t)(m * 2 + 1) * H * W + y * W + xr] = stats_pair(mn, den);
+  if (xr < W) statsf[(int64_t)(m * 2 + 1) * H * W + y * W + xr] = stats_pair(m, mn, den);
 }
 
 // view 0 for D a multiple of 4 up to 128: a pixel's row is one float4 per
@@ -445,8 +446,8 @@ __global__ void __launch_bounds__(256) stats_f32_left_q_kernel(VolsF vols, int64
       da += __shfl_xor_sync(0xffffffffu, da, o);
       db += __shfl_xor_sync(0xffffffffu, db, o);
     }
-    if (lane == 0) out[p] = stats_pair(ma, da);
-    if (lane == 1 && two) out[p2] = stats_pair(mb, db);
+    if (lane == 0) out[p] = stats_pair(m, ma, da);
+    if (lane == 1 && two) out[p2] = stats_pair(m, mb, db);
   }
 }
 
@@ -484,7 +485,7 @@ __global__ void __launch_bounds__(256) stats_f32_left_g8_kernel(VolsF vols, int6
     }
 #pragma unroll
     for (int o = 4; o; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
-    if (li == 0 && on) out[p] = stats_pair(mn, den);
+    if (li == 0 && on) out[p] = stats_pair(m, mn, den);
   }
 }
 
@@ -536,7 +537,7 @@ __global__ void __launch_bounds__(RS_PIX) stats_f32_right_q_kernel(VolsF vols, i
       }
     }
   }
-  if (xr < Wi) statsf[(int64_t)(m * 2 + 1) * H * W + y * W + xr] = stats_pair(mn, den);
+  if (xr < Wi) statsf[(int64_t)(m * 2 + 1) * H * W + y * W + xr] = stats_pair(m, mn, den);
 }
 
 int launch_feature_stats_f32(const float* const* vols, int64_t H, int64_t W, int D, float2* statsf,

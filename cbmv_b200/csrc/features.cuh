@@ -10,6 +10,8 @@ namespace cbmv {
 // ratio epsilon (test.py:548-551) and likelihood sigma (test.py:71-73).
 static __constant__ double kEps[4] = {0.01, 1.01, 0.01, 0.01};
 static __constant__ double kSigma[4] = {2.0 * 8 * 8, 0.02, 2.0 * 100 * 100, 2.0 * 100 * 100};
+// the learned path's in float32
+static __constant__ float kEpsF[4] = {0.01f, 1.01f, 0.01f, 0.01f};
 static __constant__ double kInvSigma64[4] = {1.0 / (2.0 * 8 * 8), 1.0 / 0.02, 1.0 / (2.0 * 100 * 100),
                                              1.0 / (2.0 * 100 * 100)};
 
