@@ -234,20 +234,19 @@ def forest_visits_per_unit(pipe, gf, flat, l, r, n=65536):
 
 
 def launches_per_pair(prm, classifier="mlp"):
-    """Kernel launches of one cbmv_run_mlp / cbmv_run_rf call (pipeline.cu)
-    for parameters prm.  Front end: census descriptors, NCC sums and Sobel of
-    both images (6) plus the ZSAD window means (2) except on the learned path
-    with window 5, whose strip kernel forms them itself; 4 cost volumes; the
-    row statistics (learned path 2, forest path one per volume, 4); 1
-    features + classifier.  Post: image normalisation (4), cross arms (2),
-    the SGM neighbour differences (2, with any SGM iteration); per cost
-    chain one CBCA support build (when the passes read precomputed
-    supports, L1 <= 6 and not exact_cbca) and one launch per CBCA pass, 2
-    per SGM iteration; WTA + subpixel; with interpolate the right view's
+    """Steps of one cbmv_run_mlp / cbmv_run_rf call for parameters prm, one
+    per image and stage, as the launch lists under profiles/ count them.
+    Front end: census descriptors, NCC sums and Sobel of both images (6) plus
+    the ZSAD window means (2) except on the learned path with window 5; 4
+    cost volumes; the row statistics (learned path 2, forest path one per
+    volume, 4); 1 features + classifier.  Post: image normalisation (4),
+    cross arms (2), the SGM neighbour differences (2, with any SGM
+    iteration); per cost chain one CBCA support build (when the passes read
+    precomputed supports, L1 <= 6 and not exact_cbca) and one per CBCA pass,
+    2 per SGM iteration; WTA + subpixel; with interpolate the right view's
     cost (1), its chain and its WTA (1), and the left-right check and fills
-    (3); median per iteration; mean2d.  33 (learned) and 37 (forest) with
-    the defaults, as the ncu launch lists of the headline step count them
-    per pass."""
+    (3); median per iteration; mean2d.  33 (learned) and 37 (forest) with the
+    defaults.  Several of these steps share one launch: pair_launches."""
     f32 = classifier == "mlp"
     front = 6 + (0 if (f32 and prm.sadw == 5) else 2) + 4 + (2 if f32 else 4) + 1
     masked = not prm.exact_cbca and prm.L1 - 1 <= 5
@@ -257,6 +256,19 @@ def launches_per_pair(prm, classifier="mlp"):
     if prm.interpolate:
         post += 1 + chain + 1 + 3
     return front + post
+
+
+def pair_launches(prm, classifier="mlp"):
+    """Kernel launches of one cbmv_run_mlp / cbmv_run_rf call: the steps of
+    launches_per_pair, less those that share a launch.  One launch forms the
+    terms of both images (the NCC sums with window 3 and the ZSAD means with
+    window 5 among them), one their moments, one the normalised images with
+    their arms, one the SGM's classes; the row statistics are two launches on
+    either path.  23 with the defaults, as counted in a profile of the call."""
+    f32 = classifier == "mlp"
+    shared = 5 - (2 if prm.nccw != 3 else 0) + (0 if f32 or prm.sadw != 5 else 2)
+    shared += (0 if f32 else 2) + 4 + (1 if prm.sgm_i else 0)
+    return launches_per_pair(prm, classifier) - shared
 
 
 def run_cbmv(a, ws, rank, local):
@@ -356,7 +368,7 @@ def run_cbmv(a, ws, rank, local):
         head = a.classifier
     h = res[head]
 
-    launches = launches_per_pair(pipe.params, head)
+    launches = pair_launches(pipe.params, head)
 
     hbm, hbm_kind = peaks()
     tc, tc_kind = tensor_peak()
@@ -673,10 +685,10 @@ def run_batch(a, ws, rank, local):
                                "(means over the timed steps)"},
         "sequential_ms": seq_ms, "sequential_value": units / (seq_ms / 1e3),
         "identical_to_sequential": bool(same), "bad2_nonocc_mean": float(np.mean(bad)),
-        "gpu_launches": a.steps * len(all_shapes) * launches_per_pair(_lib.default_params(), "mlp"),
+        "gpu_launches": a.steps * len(all_shapes) * pair_launches(_lib.default_params(), "mlp"),
         "gpu_launches_note": "this package's kernels inside the graphs over the timed steps: %d per pair "
                              "x %d pairs per step, one graph launch per step per GPU"
-                             % (launches_per_pair(_lib.default_params(), "mlp"), len(all_shapes)),
+                             % (pair_launches(_lib.default_params(), "mlp"), len(all_shapes)),
         "clocks": clk.summary(),
     }
 

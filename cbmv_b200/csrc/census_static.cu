@@ -75,8 +75,7 @@ extern "C" int cbmv_census_static(const uint8_t* L, const uint8_t* R, int64_t H,
   cudaStream_t st = as_stream(stream);
   // Every descriptor the cost kernel reads is written by this call first
   // (both lie in the valid window region), so nothing needs clearing.
-  if ((rc = launch_census_desc(L, H, W, wsize, dl, st))) return rc;
-  if ((rc = launch_census_desc(R, H, W, wsize, dr, st))) return rc;
+  if ((rc = launch_census_descs(L, R, H, W, wsize, dl, dr, st))) return rc;
   return dtype == CBMV_F64 ? launch_census_cost(dl, dr, H, W, D, wsize, layout, (double*)out, st)
                            : launch_census_cost(dl, dr, H, W, D, wsize, layout, (float*)out, st);
 }

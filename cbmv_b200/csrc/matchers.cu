@@ -16,6 +16,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "pipeline.cuh"
 
 namespace cbmv {
 namespace {
@@ -223,6 +224,70 @@ __global__ void zsad_cost_kernel(const uint8_t* __restrict__ L, const uint8_t* _
     v = s;
   }
   out[vol_index(layout, c.y, c.x, c.d, H, W, D)] = cvt_out<T>(v);
+}
+
+// ------------------------------------------------------ image terms
+// The per-pixel terms of the default windows -- census descriptors (11),
+// NCC sums (3), Sobel responses, ZSAD means (5) -- of one or two images
+// (blockIdx.y) in one launch, from one shared-memory tile of the image; each
+// array may be null.  The values and the regions written are those of the
+// kernels above.  Bound by its 121 byte reads of shared memory per pixel, the
+// tile's halo read from L2; both 694x554 images together 25 us (119 us in six
+// launches that read every window from global memory), 96x64 5.2 us (29).
+constexpr int kTermX = 32, kTermY = 16, kTermHalo = 5;
+
+__global__ void __launch_bounds__(256) match_terms_kernel(MatchTerms t, int64_t H, int64_t W) {
+  constexpr int SX = kTermX + 2 * kTermHalo, SY = kTermY + 2 * kTermHalo, P = 48;
+  __shared__ uint8_t px[SY][P];
+  const int im = blockIdx.y;
+  const uint8_t* __restrict__ img = t.img[im];
+  const int64_t ntx = (W + kTermX - 1) / kTermX;
+  const int64_t X0 = blockIdx.x % ntx * kTermX, Y0 = blockIdx.x / ntx * kTermY;
+  for (int q = threadIdx.x; q < SY * P; q += 256) {
+    const int r = q / P, c = q % P;
+    const int64_t y = Y0 - kTermHalo + r, x = X0 - kTermHalo + c;
+    if (c < SX) px[r][c] = y >= 0 && y < H && x >= 0 && x < W ? __ldg(img + y * W + x) : 0;
+  }
+  __syncthreads();
+  const int lx = threadIdx.x & 31;
+  const int64_t x = X0 + lx;
+  // pixel (i + r, j + r) of a w-wide window, r = w / 2, exists for i < H - w, j < W - w
+  auto inside = [&](int64_t y, int w) { return y >= w / 2 && y < H - w + w / 2 && x >= w / 2 && x < W - w + w / 2; };
+  for (int ly = threadIdx.x >> 5; ly < kTermY; ly += 8) {
+    const int64_t y = Y0 + ly, p = y * W + x;
+    if (y >= H || x >= W) continue;
+    const uint8_t* c0 = &px[ly + kTermHalo][lx + kTermHalo];
+    if (t.desc[im] && inside(y, 11)) {
+      const int c = *c0;
+      uint32_t b[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+      for (int k = 0; k < 121; k++)
+        if (c < (int)c0[(k / 11 - 5) * P + k % 11 - 5]) b[k >> 5] |= 1u << (k & 31);
+      t.desc[im][p] = make_ulonglong2(b[0] | (unsigned long long)b[1] << 32, b[2] | (unsigned long long)b[3] << 32);
+    }
+    if (t.A[im] && inside(y, 3)) {
+      unsigned a = 0, sq = 0;
+#pragma unroll
+      for (int k = 0; k < 9; k++) {
+        const unsigned v = c0[(k / 3 - 1) * P + k % 3 - 1];
+        a += v;
+        sq += v * v;
+      }
+      t.A[im][p] = a;
+      t.C[im][p] = 1.0 / sqrt((double)(9u * sq) - (double)a * (double)a);
+    }
+    if (t.mean[im] && inside(y, 5)) {
+      int sum = 0;
+#pragma unroll
+      for (int k = 0; k < 25; k++) sum += c0[(k / 5 - 2) * P + k % 5 - 2];
+      t.mean[im][p] = (double)sum / 25.0;
+    }
+    if (t.sob[im]) {
+      // matchers.cpp:539-548: written at (i+1, j+1) for i < H-3, j < W-3
+      const bool in = y >= 1 && y - 1 < H - 3 && x >= 1 && x - 1 < W - 3;
+      t.sob[im][p] = in ? -(int)c0[-P - 1] + (int)c0[-P + 1] - 2 * (int)c0[-1] + 2 * (int)c0[1] - (int)c0[P - 1] + (int)c0[P + 1] : 0;
+    }
+  }
 }
 
 // ------------------------------------------------------- strip matchers
@@ -480,11 +545,24 @@ __global__ void fill_kernel(T* out, int64_t n, T v) {
     out[p] = v;
 }
 
-int launch_census_desc(const uint8_t* img, int64_t H, int64_t W, int w, ulonglong2* desc,
-                       cudaStream_t st) {
+int launch_match_terms(const MatchTerms& t, int64_t H, int64_t W, cudaStream_t st) {
+  const int64_t tiles = ((W + kTermX - 1) / kTermX) * ((H + kTermY - 1) / kTermY);
+  CBMV_REQUIRE(tiles < ((int64_t)1 << 31), CBMV_ERANGE, "image too large for the term grid");
+  match_terms_kernel<<<dim3((unsigned)tiles, t.img[1] ? 2 : 1), 256, 0, st>>>(t, H, W);
+  return check_launch("match_terms");
+}
+
+int launch_census_descs(const uint8_t* L, const uint8_t* R, int64_t H, int64_t W, int w, ulonglong2* dl,
+                        ulonglong2* dr, cudaStream_t st) {
+  if (w == 11) {
+    MatchTerms t{{L, R}};
+    t.desc[0] = dl, t.desc[1] = dr;
+    return launch_match_terms(t, H, W, st);
+  }
   if (H <= w || W <= w) return CBMV_OK;
   const int64_t n = (H - w) * (W - w);
-  census_desc_kernel<<<grid_for(n, kBlock), kBlock, 0, st>>>(img, H, W, w, desc);
+  census_desc_kernel<<<grid_for(n, kBlock), kBlock, 0, st>>>(L, H, W, w, dl);
+  census_desc_kernel<<<grid_for(n, kBlock), kBlock, 0, st>>>(R, H, W, w, dr);
   return check_launch("census_desc");
 }
 
@@ -534,11 +612,6 @@ int launch_ncc_cost(const uint8_t* L, const uint8_t* R, const uint32_t* Al, cons
   ncc_cost_kernel<T><<<vol_grid(layout, H, W, D), kBlock, 0, st>>>(L, R, Al, Ar, Cl, Cr, H, W, D, w,
                                                                    layout, out);
   return check_launch("ncc_cost");
-}
-
-int launch_sobel_i32(const uint8_t* img, int64_t H, int64_t W, int32_t* out, cudaStream_t st) {
-  sobel_kernel<int32_t><<<grid_for(H * W, kBlock), kBlock, 0, st>>>(img, H, W, out);
-  return check_launch("sobel");
 }
 
 template <class T>
@@ -623,8 +696,7 @@ extern "C" int cbmv_census(const uint8_t* L, const uint8_t* R, int64_t H, int64_
   CBMV_CUDA(cudaMallocAsync(&s.p, (size_t)H * W * sizeof(ulonglong2) * 2, st));
   ulonglong2* dl = (ulonglong2*)s.p;
   ulonglong2* dr = dl + H * W;
-  if ((rc = launch_census_desc(L, H, W, wsize, dl, st))) return rc;
-  if ((rc = launch_census_desc(R, H, W, wsize, dr, st))) return rc;
+  if ((rc = launch_census_descs(L, R, H, W, wsize, dl, dr, st))) return rc;
   rc = dtype == CBMV_F64 ? launch_census_cost(dl, dr, H, W, D, wsize, layout, (double*)out, st)
                          : launch_census_cost(dl, dr, H, W, D, wsize, layout, (float*)out, st);
   CBMV_CUDA(cudaFreeAsync(s.p, st));
@@ -644,8 +716,14 @@ extern "C" int cbmv_ncc(const uint8_t* L, const uint8_t* R, int64_t H, int64_t W
   double* Cr = Cl + n;
   uint32_t* Al = (uint32_t*)(Cr + n);
   uint32_t* Ar = Al + n;
-  if ((rc = launch_ncc_stats(L, H, W, wsize, Al, Cl, st))) return rc;
-  if ((rc = launch_ncc_stats(R, H, W, wsize, Ar, Cr, st))) return rc;
+  if (wsize == 3) {
+    MatchTerms t{{L, R}};
+    t.A[0] = Al, t.A[1] = Ar, t.C[0] = Cl, t.C[1] = Cr;
+    rc = launch_match_terms(t, H, W, st);
+  } else if (!(rc = launch_ncc_stats(L, H, W, wsize, Al, Cl, st))) {
+    rc = launch_ncc_stats(R, H, W, wsize, Ar, Cr, st);
+  }
+  if (rc) return rc;
   rc = dtype == CBMV_F64
            ? launch_ncc_cost(L, R, Al, Ar, Cl, Cr, H, W, D, wsize, layout, (double*)out, st)
            : launch_ncc_cost(L, R, Al, Ar, Cl, Cr, H, W, D, wsize, layout, (float*)out, st);
@@ -703,8 +781,14 @@ extern "C" int cbmv_zsad(const uint8_t* L, const uint8_t* R, int64_t H, int64_t 
   CBMV_CUDA(cudaMallocAsync(&s.p, n * 2 * sizeof(double), st));
   double* ml = (double*)s.p;
   double* mr = ml + n;
-  if ((rc = launch_zsad_means(L, H, W, wsize, ml, st))) return rc;
-  if ((rc = launch_zsad_means(R, H, W, wsize, mr, st))) return rc;
+  if (wsize == 5) {
+    MatchTerms t{{L, R}};
+    t.mean[0] = ml, t.mean[1] = mr;
+    rc = launch_match_terms(t, H, W, st);
+  } else if (!(rc = launch_zsad_means(L, H, W, wsize, ml, st))) {
+    rc = launch_zsad_means(R, H, W, wsize, mr, st);
+  }
+  if (rc) return rc;
   rc = dtype == CBMV_F64
            ? launch_zsad_cost(L, R, ml, mr, H, W, D, wsize, layout, (double*)out, st)
            : launch_zsad_cost(L, R, ml, mr, H, W, D, wsize, layout, (float*)out, st);

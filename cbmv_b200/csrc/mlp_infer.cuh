@@ -189,41 +189,66 @@ __device__ __forceinline__ void conf_f32(float c, float inv_ce, float2 st, float
 }
 
 // Stage the inference weights from the float32 parameter vector, and the
-// constant tile of the bias MMAs.
+// constant tile of the bias MMAs, 16 bytes (eight columns of a row) at a
+// time: every weight row starts on a 16-byte boundary of the vector.  The
+// whole kernel at 96x64 D=16 (one tile per group) 29.1 -> 24.6 us against two
+// bytes at a time.
+template <bool F16>
+__device__ __forceinline__ uint32_t pair(float lo, float hi) {
+  return Op16<F16>::bits(lo) | (uint32_t)Op16<F16>::bits(hi) << 16;
+}
+template <bool F16>
+__device__ __forceinline__ uint4 pack8(const float* __restrict__ p) {
+  const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+  return make_uint4(pair<F16>(a.x, a.y), pair<F16>(a.z, a.w), pair<F16>(b.x, b.y), pair<F16>(b.z, b.w));
+}
+template <bool F16>
+__device__ __forceinline__ uint32_t pack_split(float x) {  // high, low part
+  float hi, lo;
+  Op16<F16>::split(x, &hi, &lo);
+  return pair<F16>(hi, lo);
+}
+
 template <bool F16>
 __device__ __forceinline__ void stage_inference_weights(const float* __restrict__ P, unsigned char* sW1, unsigned char* sW2,
                                         unsigned char* sW3, unsigned char* sW4, unsigned char* sOne) {
-  for (int q = threadIdx.x; q < 128 * 64; q += blockDim.x) {
-    const int r = q >> 6, k = q & 63;
-    float v = 0.0f, hi, lo;
-    if (k < kF) {
-      v = P[kOffW1 + r * kF + k];
-    } else if (k == kF || k == kF + 1) {
-      Op16<F16>::split(P[kOffB1 + r], &hi, &lo);
-      v = k == kF ? hi : lo;
-    } else if (k == kColB2 || k == kColB2 + 1) {
-      Op16<F16>::split(P[kOffB2 + r], &hi, &lo);
-      v = k == kColB2 ? hi : lo;
-    } else if (r < kH3 && (k == kColB3 || k == kColB3 + 1)) {
-      Op16<F16>::split(P[kOffB3 + r], &hi, &lo);
-      v = k == kColB3 ? hi : lo;
+  static_assert(kOffW1 % 4 == 0 && kF % 4 == 0 && kOffW2 % 4 == 0 && kOffW3 % 4 == 0 && kOffW4 % 4 == 0 && kF == 20, "aligned rows");
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  for (int q = threadIdx.x; q < 128 * 8; q += blockDim.x) {
+    const int r = q >> 3, k = (q & 7) * 8;
+    uint4 v = zero;
+    if (k < 16) {
+      v = pack8<F16>(P + kOffW1 + r * kF + k);
+    } else if (k == 16) {  // the last four features, then b1
+      const float4 a = __ldg(reinterpret_cast<const float4*>(P + kOffW1 + r * kF + k));
+      v = make_uint4(pair<F16>(a.x, a.y), pair<F16>(a.z, a.w), pack_split<F16>(P[kOffB1 + r]), 0u);
+    } else if (k == kColB2) {
+      v.x = pack_split<F16>(P[kOffB2 + r]);
+    } else if (k == kColB3 && r < kH3) {
+      v.x = pack_split<F16>(P[kOffB3 + r]);
     }
-    *reinterpret_cast<uint16_t*>(sW1 + umma::sw128_offset(128, r, k)) = Op16<F16>::bits(v);
-    *reinterpret_cast<uint16_t*>(sOne + umma::sw128_offset(128, r, k)) = Op16<F16>::bits(k < 2 ? 1.0f : 0.0f);
+    *reinterpret_cast<uint4*>(sW1 + umma::sw128_offset(128, r, k)) = v;
+    *reinterpret_cast<uint4*>(sOne + umma::sw128_offset(128, r, k)) = k == 0 ? make_uint4(Op16<F16>::kOneOne, 0u, 0u, 0u) : zero;
   }
-  for (int q = threadIdx.x; q < 128 * 128; q += blockDim.x) {
-    const int r = q >> 7, k = q & 127;
-    *reinterpret_cast<uint16_t*>(sW2 + umma::sw128_offset(128, r, k)) = Op16<F16>::bits(P[kOffW2 + q]);
+  for (int q = threadIdx.x; q < 128 * 16; q += blockDim.x) {
+    const int r = q >> 4, k = (q & 15) * 8;
+    *reinterpret_cast<uint4*>(sW2 + umma::sw128_offset(128, r, k)) = pack8<F16>(P + kOffW2 + r * kH1 + k);
   }
-  for (int q = threadIdx.x; q < 64 * 128; q += blockDim.x) {
-    const int r = q >> 7, k = q & 127;
-    *reinterpret_cast<uint16_t*>(sW3 + umma::sw128_offset(64, r, k)) = Op16<F16>::bits(P[kOffW3 + q]);
+  for (int q = threadIdx.x; q < 64 * 16; q += blockDim.x) {
+    const int r = q >> 4, k = (q & 15) * 8;
+    *reinterpret_cast<uint4*>(sW3 + umma::sw128_offset(64, r, k)) = pack8<F16>(P + kOffW3 + r * kH2 + k);
   }
-  for (int q = threadIdx.x; q < 16 * 64; q += blockDim.x) {
-    const int r = q >> 6, k = q & 63;
-    float hi, lo;
-    Op16<F16>::split(P[kOffW4 + k], &hi, &lo);
-    *reinterpret_cast<uint16_t*>(sW4 + umma::sw128_offset(16, r, k)) = Op16<F16>::bits(r == 0 ? hi : r == 1 ? lo : 0.0f);
+  for (int q = threadIdx.x; q < 16 * 8; q += blockDim.x) {
+    const int r = q >> 3, k = (q & 7) * 8;
+    float w[8];  // row 0: high parts, row 1: low parts
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      float hi, lo;
+      Op16<F16>::split(P[kOffW4 + k + i], &hi, &lo);
+      w[i] = r == 0 ? hi : r == 1 ? lo : 0.0f;
+    }
+    *reinterpret_cast<uint4*>(sW4 + umma::sw128_offset(16, r, k)) =
+        make_uint4(pair<F16>(w[0], w[1]), pair<F16>(w[2], w[3]), pair<F16>(w[4], w[5]), pair<F16>(w[6], w[7]));
   }
 }
 

@@ -301,11 +301,10 @@ static int cost_chain(cbmv_ctx* c, const cbmv_params* p, Work& w, int64_t H, int
     RC(launch_cbca_mask_build(crossA, crossB, H, W, D, direction, masks, st));
   }
   auto cbca = [&](const float* in, float* out) {
-    const int rows = p->cbca_rows == 16 ? 16 : 32;
     if (p->exact_cbca)
       return launch_cbca(crossA, crossB, in, H, W, D, CBMV_HWD, direction, out, st, p->L1 - 1);
-    if (masked) return launch_cbca_masked(masks, in, H, W, D, out, st, rows);
-    return launch_cbca_sep(crossA, crossB, in, H, W, D, direction, out, st, p->L1 - 1, rows);
+    if (masked) return launch_cbca_masked(masks, in, H, W, D, out, st, p->cbca_rows);
+    return launch_cbca_sep(crossA, crossB, in, H, W, D, direction, out, st, p->L1 - 1, p->cbca_rows == 16 ? 16 : 32);
   };
   for (int i = 0; i < p->cbca_i1; i++) {
     RC(cbca(cur, oth));
@@ -345,11 +344,7 @@ static int cost_chain(cbmv_ctx* c, const cbmv_params* p, Work& w, int64_t H, int
 // the call, beside the matchers.
 static int post_prep(const cbmv_params* p, const uint8_t* L, const uint8_t* R, int64_t H, int64_t W, Work& w,
                      cudaStream_t s) {
-  const int64_t HW = H * W;
-  RC(launch_normalise(L, HW, w.mom, w.imL, s));
-  RC(launch_normalise(R, HW, w.mom + 2, w.imR, s));
-  RC(launch_cross(w.imL, H, W, p->L1, p->tau1, w.crossL, s));
-  RC(launch_cross(w.imR, H, W, p->L1, p->tau1, w.crossR, s));
+  RC(launch_normalise_cross(L, R, H, W, w.mom, p->L1, p->tau1, w.imL, w.imR, w.crossL, w.crossR, s));
   if (p->sgm_i > 0) RC(launch_sgm_codes(w.imL, w.imR, H, W, p->tau_so, sgm_codes_at(w.codes, H, W), s));
   return CBMV_OK;
 }
@@ -422,18 +417,23 @@ static int run_front(cbmv_ctx* c, const cbmv_params* p, const uint8_t* L, const 
     CBMV_CUDA(cudaEventRecord(c->prep_ev, c->side));
     w.prepped = true;
   }
-  RC(launch_census_desc(L, H, W, p->censw, w.descL, st));
-  RC(launch_census_desc(R, H, W, p->censw, w.descR, st));
-  RC(launch_ncc_stats(L, H, W, p->nccw, w.AL, w.CL, st));
-  RC(launch_ncc_stats(R, H, W, p->nccw, w.AR, w.CR, st));
-  // the learned path's ZSAD strip kernel (window 5) forms the window means
-  // itself, from the column sums it holds anyway
-  if (!(f32 && p->sadw == 5)) {
+  // the terms of both images in one launch (census window 11, checked above);
+  // other NCC and ZSAD windows have their own.  The learned path's ZSAD strip
+  // kernel (window 5) forms the window means itself, from the column sums it
+  // holds anyway
+  MatchTerms t{{L, R}, {w.descL, w.descR}};
+  t.sob[0] = w.sobL, t.sob[1] = w.sobR;
+  if (p->nccw == 3) t.A[0] = w.AL, t.A[1] = w.AR, t.C[0] = w.CL, t.C[1] = w.CR;
+  if (p->sadw == 5 && !f32) t.mean[0] = w.muL, t.mean[1] = w.muR;
+  RC(launch_match_terms(t, H, W, st));
+  if (p->nccw != 3) {
+    RC(launch_ncc_stats(L, H, W, p->nccw, w.AL, w.CL, st));
+    RC(launch_ncc_stats(R, H, W, p->nccw, w.AR, w.CR, st));
+  }
+  if (p->sadw != 5) {
     RC(launch_zsad_means(L, H, W, p->sadw, w.muL, st));
     RC(launch_zsad_means(R, H, W, p->sadw, w.muR, st));
   }
-  RC(launch_sobel_i32(L, H, W, w.sobL, st));
-  RC(launch_sobel_i32(R, H, W, w.sobR, st));
   if (f32) {
     float* v[4] = {(float*)w.vol[0], (float*)w.vol[1], (float*)w.vol[2], (float*)w.vol[3]};
     RC(launch_census_cost<float>(w.descL, w.descR, H, W, D, p->censw, CBMV_HWD, v[0], st));

@@ -11,8 +11,19 @@ namespace cbmv {
 // (CBMV_ERANGE beyond), W > 0, window odd and <= wmax, dtype and layout.
 int check_common(const void* a, const void* b, const void* out, int64_t H, int64_t W, int D, int w,
                  int dtype, int layout, int wmax);
-int launch_census_desc(const uint8_t* img, int64_t H, int64_t W, int w, ulonglong2* desc,
-                       cudaStream_t st);
+// Per-pixel matcher terms of one or two images (img[1] null: one) at the
+// default windows; null arrays are not formed.
+struct MatchTerms {
+  const uint8_t* img[2];
+  ulonglong2* desc[2];  // census, 11 x 11
+  uint32_t* A[2];       // NCC, 3 x 3: window sum and 1 / sqrt(9 B - A^2)
+  double* C[2];
+  double* mean[2];      // ZSAD, 5 x 5
+  int32_t* sob[2];      // Sobel responses
+};
+int launch_match_terms(const MatchTerms& t, int64_t H, int64_t W, cudaStream_t st);
+int launch_census_descs(const uint8_t* L, const uint8_t* R, int64_t H, int64_t W, int w, ulonglong2* dl,
+                        ulonglong2* dr, cudaStream_t st);
 template <class T>
 int launch_census_cost(const ulonglong2* dl, const ulonglong2* dr, int64_t H, int64_t W, int D,
                        int w, int layout, T* out, cudaStream_t st);
@@ -22,7 +33,6 @@ template <class T>
 int launch_ncc_cost(const uint8_t* L, const uint8_t* R, const uint32_t* Al, const uint32_t* Ar,
                     const double* Cl, const double* Cr, int64_t H, int64_t W, int D, int w,
                     int layout, T* out, cudaStream_t st);
-int launch_sobel_i32(const uint8_t* img, int64_t H, int64_t W, int32_t* out, cudaStream_t st);
 template <class T>
 int launch_sadsob_cost(const int32_t* SL, const int32_t* SR, int64_t H, int64_t W, int D, int w,
                        int layout, T* out, cudaStream_t st);

@@ -1222,36 +1222,85 @@ __global__ void f32_to_f64_kernel(const float* __restrict__ in, int64_t n, doubl
   GRID_STRIDE(i, n) out[i] = (double)in[i];
 }
 
-// Sums of an image and of its squares in float64 (one block).
-// Sum and sum of squares of the image as exact 64-bit integers (so the
-// result does not depend on the order of the additions), accumulated by
-// every block into mom[0..1] with integer atomics; mom is zeroed first.
-__global__ void moments_kernel(const uint8_t* __restrict__ img, int64_t n,
-                               unsigned long long* __restrict__ mom) {
+// Sum and sum of squares of two images (blockIdx.y) as exact 64-bit
+// integers, so the result does not depend on the order of the additions:
+// summed per block, then two integer atomics on the zeroed mom[2 * image].
+// Bytes are read four at a time from the first aligned one on.  694x554: 6.7 us
+// for both images (49 us with two atomics per warp and one byte per load).
+__global__ void __launch_bounds__(256) moments_kernel(const uint8_t* __restrict__ L, const uint8_t* __restrict__ R,
+                                                    int64_t n, unsigned long long* __restrict__ mom) {
+  const uint8_t* __restrict__ img = blockIdx.y ? R : L;
+  const int64_t head = min(n, (int64_t)(-(intptr_t)img & 3)), words = (n - head) / 4;
   unsigned long long a = 0, b = 0;
-  GRID_STRIDE(i, n) {
-    const unsigned v = img[i];
-    a += v;
-    b += v * v;
+  GRID_STRIDE(i, words) {
+    const uint32_t v = __ldg(reinterpret_cast<const uint32_t*>(img + head) + i);
+    a += __dp4a(v, 0x01010101u, 0u);
+    b += __dp4a(v, v, 0u);
   }
+  if (blockIdx.x == 0) {
+    const int64_t tail = head + 4 * words;
+    for (int64_t i = threadIdx.x; i < head + (n - tail); i += 256) {
+      const unsigned v = img[i < head ? i : tail + i - head];
+      a += v;
+      b += v * v;
+    }
+  }
+  __shared__ unsigned long long s[2][8];
   for (int o = 16; o; o >>= 1) {
     a += __shfl_xor_sync(0xffffffffu, a, o);
     b += __shfl_xor_sync(0xffffffffu, b, o);
   }
   if ((threadIdx.x & 31) == 0) {
-    atomicAdd(mom, a);
-    atomicAdd(mom + 1, b);
+    s[0][threadIdx.x >> 5] = a;
+    s[1][threadIdx.x >> 5] = b;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    unsigned long long t = 0;
+    for (int k = 0; k < 8; k++) t += s[threadIdx.x][k];
+    atomicAdd(mom + 2 * blockIdx.y + threadIdx.x, t);
   }
 }
 
-// (I - mean) / std in float32 with float32 mean and population std, as
-// test.py:489-492 does with numpy on the float32 image.
-__global__ void normalise_kernel(const uint8_t* __restrict__ img, int64_t n,
-                                 const unsigned long long* __restrict__ mom, float* __restrict__ out) {
-  const double mean = (double)mom[0] / (double)n;
-  const double var = fmax((double)mom[1] / (double)n - mean * mean, 0.0);
-  const float m = (float)mean, s = (float)sqrt(var);
-  GRID_STRIDE(i, n) out[i] = ((float)img[i] - m) / s;
+// Two images (blockIdx.y): (I - mean) / std in float32 with float32 mean and
+// population std, as test.py:489-492 does with numpy on the float32 image,
+// and the cross arms of the result (cross_kernel's).  An 8-bit image has 256
+// normalised values: each block divides them once, and a pixel's neighbours
+// are looked up instead of read from the image the same launch writes.  Bound
+// by the arms' chain of dependent reads; both images of 694x554 24 us (77 us
+// as four launches), 96x64 5.9 us (19).
+__global__ void __launch_bounds__(256) normalise_cross_kernel(const uint8_t* __restrict__ L, const uint8_t* __restrict__ R,
+                                                            int64_t H, int64_t W,
+                                                            const unsigned long long* __restrict__ mom, int L1, float tau1,
+                                                            float* __restrict__ imL, float* __restrict__ imR,
+                                                            float* __restrict__ crossL, float* __restrict__ crossR) {
+  __shared__ float value[256];
+  const int64_t n = H * W;
+  const uint8_t* __restrict__ img = blockIdx.y ? R : L;
+  float* __restrict__ out = blockIdx.y ? imR : imL;
+  float* __restrict__ arms = blockIdx.y ? crossR : crossL;
+  const double mean = (double)mom[2 * blockIdx.y] / (double)n;
+  const double var = fmax((double)mom[2 * blockIdx.y + 1] / (double)n - mean * mean, 0.0);
+  value[threadIdx.x] = ((float)threadIdx.x - (float)mean) / (float)sqrt(var);
+  __syncthreads();
+  GRID_STRIDE(p, n) {
+    const int64_t y = p / W, x = p - y * W;
+    const float c = value[img[p]];
+    out[p] = c;
+#pragma unroll
+    for (int dir = 0; dir < 4; dir++) {
+      // steps to the image's edge, and the pixel offset of one
+      const int64_t room = dir == 0 ? x : dir == 1 ? W - 1 - x : dir == 2 ? y : H - 1 - y;
+      const int64_t step = dir == 0 ? -1 : dir == 1 ? 1 : dir == 2 ? -W : W;
+      int64_t k = 1;
+      for (; k <= room; k++) {
+        if (k == 1) continue;
+        if (fabsf(c - value[__ldg(img + p + k * step)]) >= tau1) break;  // rule 1
+        if (k >= L1) break;                                              // rule 2
+      }
+      arms[dir * n + p] = (float)((dir <= 1 ? x : y) + ((dir & 1) ? k : -k));
+    }
+  }
 }
 
 }  // namespace
@@ -1353,25 +1402,38 @@ int launch_cbca_sep(const float* lc, const float* rc, const float* in, int64_t H
   }
 }
 
+// Tiles of the separable CBCA's kernels with `rows` rows each.  A tile's
+// halo costs 10 rows, so 32 rows are the least work (a pass at 694x554 D=128:
+// 238 us); below kCbcaFull tiles (two per SM) they leave SMs idle and each
+// tile is a longer chain: 96x64 D=16, 24 tiles of 32 rows 19.6 us, 96 of 8
+// rows 6.8 (the support build 26.0 and 20.1 us).
+static unsigned cbca_tiles(int64_t H, int64_t W, int D, int rows) {
+  return (unsigned)(((W + CS_TX - 1) / CS_TX) * ((H + rows - 1) / rows) * ((D + CS_TD - 1) / CS_TD));
+}
+constexpr unsigned kCbcaFull = 296;
+
 int launch_cbca_mask_build(const float* lc, const float* rc, int64_t H, int64_t W, int D, int direction,
                            uint32_t* mask, cudaStream_t st) {
   CBMV_REQUIRE(H < (1 << 30) && W < (1 << 30) &&
                    (int64_t)((W + CS_TX - 1) / CS_TX) * ((H + 15) / 16) * ((D + CS_TD - 1) / CS_TD) <
                        ((int64_t)1 << 31),
                CBMV_ERANGE, "cbca: volume too large");
-  constexpr int TY = 32;
-  const int64_t tiles = (int64_t)((W + CS_TX - 1) / CS_TX) * ((H + TY - 1) / TY) * ((D + CS_TD - 1) / CS_TD);
-  cbca_mask_build_kernel<TY><<<(unsigned)tiles, 256, 0, st>>>(lc, rc, (int)H, (int)W, D, direction, mask);
+  const unsigned tiles32 = cbca_tiles(H, W, D, 32), tiles8 = cbca_tiles(H, W, D, 8);
+  if (tiles32 >= kCbcaFull) cbca_mask_build_kernel<32><<<tiles32, 256, 0, st>>>(lc, rc, (int)H, (int)W, D, direction, mask);
+  else cbca_mask_build_kernel<8><<<tiles8, 256, 0, st>>>(lc, rc, (int)H, (int)W, D, direction, mask);
   return check_launch("cbca_mask_build");
 }
 
-// tile rows 16 or 32 (the results do not depend on them)
+// tile rows 16 or 32, 0: by the volume (the results do not depend on them)
 int launch_cbca_masked(const uint32_t* mask, const float* in, int64_t H, int64_t W, int D, float* out,
                        cudaStream_t st, int rows) {
   CBMV_REQUIRE(H < (1 << 30) && W < (1 << 30) &&
                    (int64_t)((W + CS_TX - 1) / CS_TX) * ((H + 15) / 16) * ((D + CS_TD - 1) / CS_TD) <
                        ((int64_t)1 << 31),
                CBMV_ERANGE, "cbca: volume too large");
+  if (rows == 0)
+    rows = cbca_tiles(H, W, D, 32) >= kCbcaFull ? 32 : cbca_tiles(H, W, D, 16) >= kCbcaFull ? 16 : 8;
+  if (rows == 8) return launch_cbca_masked_t<8>(mask, in, H, W, D, out, st);
   if (rows == 16) return launch_cbca_masked_t<16>(mask, in, H, W, D, out, st);
   return launch_cbca_masked_t<32>(mask, in, H, W, D, out, st);
 }
@@ -1398,12 +1460,14 @@ int launch_mean2d(const float* in, int64_t H, int64_t W, const float* kernel, in
   return check_launch("mean2d");
 }
 
-int launch_normalise(const uint8_t* img, int64_t n, double* mom, float* out, cudaStream_t st) {
+int launch_normalise_cross(const uint8_t* L, const uint8_t* R, int64_t H, int64_t W, double* mom, int L1, float tau1,
+                           float* imL, float* imR, float* crossL, float* crossR, cudaStream_t st) {
   unsigned long long* m = reinterpret_cast<unsigned long long*>(mom);
-  CBMV_CUDA(cudaMemsetAsync(m, 0, 2 * sizeof(unsigned long long), st));
-  moments_kernel<<<grid_for(n, 256), 256, 0, st>>>(img, n, m);
-  normalise_kernel<<<grid_for(n, 256), 256, 0, st>>>(img, n, m, out);
-  return check_launch("normalise");
+  const int64_t n = H * W;
+  CBMV_CUDA(cudaMemsetAsync(m, 0, 4 * sizeof(unsigned long long), st));
+  moments_kernel<<<dim3(grid_for(n / 16 + 1, 256), 2), 256, 0, st>>>(L, R, n, m);
+  normalise_cross_kernel<<<dim3(grid_for(n, 256), 2), 256, 0, st>>>(L, R, H, W, m, L1, tau1, imL, imR, crossL, crossR);
+  return check_launch("normalise_cross");
 }
 
 // get_right_cost (featextract.cpp:115-152) of a float32 [H,W,D] volume:

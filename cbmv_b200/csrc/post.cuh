@@ -52,14 +52,16 @@ int launch_cbca_sep(const float* lc, const float* rc, const float* in, int64_t H
 int launch_cbca_mask_build(const float* lc, const float* rc, int64_t H, int64_t W, int D, int direction,
                            uint32_t* mask, cudaStream_t st);
 int launch_cbca_masked(const uint32_t* mask, const float* in, int64_t H, int64_t W, int D, float* out,
-                       cudaStream_t st, int rows = 32);
+                       cudaStream_t st, int rows = 0);
 constexpr int kCbcaMaskMaxHalo = 5;
 int launch_wta_subpixel(const float* cost, int64_t H, int64_t W, int D, float* disp_int,
                         float* disp, cudaStream_t st);
 int launch_median(const float* in, int64_t H, int64_t W, int k, float* out, cudaStream_t st);
 int launch_mean2d(const float* in, int64_t H, int64_t W, const float* kernel, int ks, float alpha2,
                   float* out, cudaStream_t st);
-int launch_normalise(const uint8_t* img, int64_t n, double* mom, float* out, cudaStream_t st);
+// do_post's normalisation (test.py:485-504) of both images and their cross arms; mom: 4 doubles of scratch
+int launch_normalise_cross(const uint8_t* L, const uint8_t* R, int64_t H, int64_t W, double* mom, int L1, float tau1,
+                           float* imL, float* imR, float* crossL, float* crossR, cudaStream_t st);
 // get_right_cost of a float32 [H,W,D] volume (the _interp post's right view)
 int launch_right_cost_f32(const float* in, int64_t H, int64_t W, int D, float* out, cudaStream_t st);
 int launch_outlier(const float* d0, const float* d1, int64_t H, int64_t W, int disp_max, float* out,

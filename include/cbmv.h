@@ -347,8 +347,8 @@ typedef struct cbmv_params {
    * (cbmv_batch). */
   int mlp_ctas;
   /* Launch shapes that do not change the results (picked by the batch
-   * autotuner): rows per CBCA tile, 16 or 32 (0 = 32); SGM steps loaded
-   * ahead, 0, 1, 2 or 4: no longer a choice (the scan's ring in shared
+   * autotuner): rows per CBCA tile, 16 or 32 (0 = by the volume's size); SGM
+   * steps loaded ahead, 0, 1, 2 or 4: no longer a choice (the scan's ring in shared
    * memory has a depth fixed by the disparity count), still checked. */
   int cbca_rows, sgm_prefetch;
   /* Post-processing chain, Testing.eval_prob's `interpolate` (main.py:70,
