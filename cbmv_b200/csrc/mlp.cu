@@ -10,6 +10,8 @@
 // timeout the kernel records an error in `status` and returns.
 #include <cuda_bf16.h>
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "mlp_net.cuh"
 #include "umma.cuh"
@@ -153,22 +155,28 @@ extern "C" int cbmv_gemm_bf16(const uint16_t* A, const uint16_t* B, float* C, in
 // bias gradients are column sums of the float32 deltas, reduced over a
 // warp's 32 rows by a 31-step exchange per 32 columns.
 //
+// Four threads take a row, 16 warps: with two threads and 8 warps a tile's
+// chain of epilogues took 24.5 us, now 19.
+//
 // mlp_wgrad_kernel forms the weight gradients, contractions over the batch,
 // from the operand tiles the first kernel stored as they were (bulk copies
-// both ways, swizzle included): eight CTAs own a 64 x 64 block of dW1, dW2
-// or dW3^T each and stream the tiles through a ring of stages.  A block is
-// one accumulator chain in sample order: partial sums in the first kernel
-// would be quicker (33 us in all at 8192) but move the gradients by the
-// rounding of a single chain, 6e-5 relative at 32768.  It is bound by what
-// one SM takes in, 32 KB per tile at 0.44 us.
-// Measured, forward and backward of one batch: 34 us at 128 samples, 59 us
-// at 8192 (7.99 ms before), 156 us at 32768.
+// both ways, swizzle included): a CTA owns a 64 x 64 block of dW1, dW2 or
+// dW3^T and streams the tiles through a ring of stages, bound by what one SM
+// takes in, 32 KB per tile at 0.44 us.  From 8 to 64 tiles a cluster of four
+// CTAs splits a block's tiles and adds the four sums through distributed
+// shared memory (at 8192 samples 29 -> 13.5 us); fewer tiles are too short a
+// chain, and above 64 a block stays one accumulator chain in sample order:
+// the tensor core truncates, so split sums, though nearer to float64, move
+// away from the single chain's (1.0e-5 relative at 8192, 6e-5 at 32768).  Its
+// CTAs are set up while the first kernel runs (programmatic launch).
+// Measured, forward and backward of one batch: 25 us at 128 samples, 33 us
+// at 8192 (7.99 ms as 24 launches), 147 us at 32768.
 // All sums have a fixed order, so a batch gives the same gradients every time.
 // ====================================================================
 namespace cbmv {
 namespace {
 
-constexpr int kTrainThreads = 256;  // two threads per tile row, each half of the columns
+constexpr int kTrainThreads = 512;  // four threads per tile row, each a quarter of the columns
 // a CTA's share of the sums over the samples: db1, db2, db3, dw4, db4, loss
 constexpr int kSums = kH1 + kH2 + 2 * kH3 + 2;
 
@@ -177,7 +185,8 @@ constexpr int kSums = kH1 + kH2 + 2 * kH3 + 2;
 constexpr uint32_t kAtom = 128 * 128;  // one SW128 atom of 128 rows x 64 columns
 constexpr uint32_t kTX0 = 0, kTA1 = kTX0 + kAtom, kTA2 = kTA1 + 2 * kAtom, kTD3 = kTA2 + 2 * kAtom,
                    kTW1 = kTD3 + kAtom, kTW2 = kTW1 + kAtom, kTW3 = kTW2 + 2 * kAtom, kTEnd = kTW3 + kAtom;
-constexpr size_t kSmTrain = 1024 + kTEnd;
+constexpr uint32_t kTScr = kTEnd;  // [32][128] floats of the output layer's dot products
+constexpr size_t kSmTrain = 1024 + kTScr + 32 * 128 * 4;
 // the stored image of a tile: X0, A1, A2, dS3, dS2, dS1
 constexpr uint32_t kID2 = kTD3 + kAtom, kID1 = kID2 + 2 * kAtom, kImage = kID1 + 2 * kAtom;
 // tensor-memory columns
@@ -218,11 +227,16 @@ __device__ __forceinline__ float2 train_grad(uint32_t s) {
   return ACT == CBMV_ACT_GELU ? make_float2(gelu_grad(x.x), gelu_grad(x.y)) : x;
 }
 
-// Sums over the warp's lanes of 32 values each: lane l receives the sum of
-// v[l].  Every step exchanges one half of the remaining values (31 shuffles).
-__device__ __forceinline__ float warp_colsum(float (&v)[32], int lane) {
+// Sums over the warp's lanes of N values each (32 or 16): lane l receives the
+// sum of v[l % N].  Every step exchanges one half of the remaining values (31
+// shuffles); 16 values are first added across the half-warps.
+template <int N>
+__device__ __forceinline__ float warp_colsum(float (&v)[N], int lane) {
+  if (N == 16)
 #pragma unroll
-  for (int o = 16; o; o >>= 1) {
+    for (int i = 0; i < N; i++) v[i] += __shfl_xor_sync(0xffffffffu, v[i], 16);
+#pragma unroll
+  for (int o = N / 2; o; o >>= 1) {
     const bool up = lane & o;
 #pragma unroll
     for (int i = 0; i < o; i++) {
@@ -240,12 +254,14 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   __shared__ float s_nrm[kNormN], s_b1[kH1], s_b2[kH2], s_b3[kH3], s_w4[kH3];
-  __shared__ float s_b4;
+  __shared__ float s_b4, s_z[128];
   __shared__ float s_red[4][kSums];
   __shared__ uint64_t bar;
   __shared__ uint32_t tmem_base;
-  const int tid = threadIdx.x, lane = tid & 31, quad = (tid >> 5) & 3, half = tid >> 7, row = tid & 127;
+  const int tid = threadIdx.x, lane = tid & 31, quad = (tid >> 5) & 3, part = tid >> 7, row = tid & 127;
 
+  // the weight gradients' CTAs may take free SMs and set up; they wait for this grid's end
+  asm volatile("griddepcontrol.launch_dependents;");
   if (tid < 32) umma::tmem_alloc(&tmem_base, kTrainCols);
   if (tid == 0) umma::mbar_init(&bar, 1);
   // weights, K-major; columns of X0 and W1 beyond the 20 features are zero
@@ -268,8 +284,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     const int r = q >> 4, k = (q & 15) * 8;
     stage8(base + kTW3 + umma::sw128_offset(64, r, k), P + kOffW3 + r * kH2 + k);
   }
-  for (int j = 4 * half; j < 4 * half + 4; j++)
-    if (j >= 4) *reinterpret_cast<uint4*>(base + kTX0 + umma::sw128_offset(128, row, 8 * j)) = zero;
+  *reinterpret_cast<uint4*>(base + kTX0 + umma::sw128_offset(128, row, 8 * (4 + part))) = zero;
   if (tid < kNormN) s_nrm[tid] = P[tid];
   if (tid < kH1) s_b1[tid] = P[kOffB1 + tid];
   if (tid < kH2) s_b2[tid] = P[kOffB2 + tid];
@@ -307,15 +322,15 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     umma::tc_fence_after();
     return r != 0;
   };
-  // column sums of this CTA's tiles (warp `quad` of either half): db1 and
-  // db2 columns 64*half + 32*i + lane, db3 and dw4 column 32*half + lane
-  float db1[2] = {0, 0}, db2[2] = {0, 0}, db3 = 0.0f, dw4 = 0.0f, db4 = 0.0f, loss = 0.0f;
+  // column sums of this CTA's tiles (warp `quad` of each quarter): db1 and
+  // db2 column 32*part + lane, db3 and dw4 column 16*part + lane % 16
+  float db1 = 0.0f, db2 = 0.0f, db3 = 0.0f, dw4 = 0.0f, db4 = 0.0f, loss = 0.0f;
 
   // hidden layer: accumulator + bias -> activation (bf16 tile) and its argument (f16, tensor memory)
   auto forward = [&](const float* bias, uint32_t tile, uint32_t args) {
 #pragma unroll
-    for (int c0 = 0; c0 < 64; c0 += 16) {
-      const int c = 64 * half + c0;
+    for (int c0 = 0; c0 < 32; c0 += 16) {
+      const int c = 32 * part + c0;
       uint32_t v[16], s[8], a[8];
       umma::tmem_ld16_issue(tlane + kCAcc + c, v);
       umma::tmem_ld16_wait(v);
@@ -329,30 +344,27 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     umma::tmem_st_wait();
   };
   // dS = dA * act'(S) -> bf16 tile, and its column sums
-  auto backward = [&](uint32_t tile, uint32_t args, float* db) {
+  auto backward = [&](uint32_t tile, uint32_t args, float& db) {
+    const int c = 32 * part;
+    float d[32];
+    {
+      uint32_t v[32], s[16];
+      umma::tmem_ld32_issue(tlane + kCAcc + c, v);
+      umma::tmem_ld16_issue(tlane + args + c / 2, s);
+      umma::tmem_ld32_wait(v);
+      umma::tmem_ld16_wait(s);
 #pragma unroll
-    for (int b = 0; b < 2; b++) {
-      const int c = 64 * half + 32 * b;
-      float d[32];
-      {
-        uint32_t v[32], s[16];
-        umma::tmem_ld32_issue(tlane + kCAcc + c, v);
-        umma::tmem_ld16_issue(tlane + args + c / 2, s);
-        umma::tmem_ld32_wait(v);
-        umma::tmem_ld16_wait(s);
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-          const float2 g = train_grad<ACT>(s[i]);
-          d[2 * i] = __uint_as_float(v[2 * i]) * g.x;
-          d[2 * i + 1] = __uint_as_float(v[2 * i + 1]) * g.y;
-        }
+      for (int i = 0; i < 16; i++) {
+        const float2 g = train_grad<ACT>(s[i]);
+        d[2 * i] = __uint_as_float(v[2 * i]) * g.x;
+        d[2 * i + 1] = __uint_as_float(v[2 * i + 1]) * g.y;
       }
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-        *chunk(tile, c + 8 * i) = make_uint4(pack_bf16(d[8 * i], d[8 * i + 1]), pack_bf16(d[8 * i + 2], d[8 * i + 3]),
-                                             pack_bf16(d[8 * i + 4], d[8 * i + 5]), pack_bf16(d[8 * i + 6], d[8 * i + 7]));
-      db[b] += warp_colsum(d, lane);
     }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      *chunk(tile, c + 8 * i) = make_uint4(pack_bf16(d[8 * i], d[8 * i + 1]), pack_bf16(d[8 * i + 2], d[8 * i + 3]),
+                                           pack_bf16(d[8 * i + 4], d[8 * i + 5]), pack_bf16(d[8 * i + 6], d[8 * i + 7]));
+    db += warp_colsum(d, lane);
   };
   constexpr uint32_t id128 = umma::idesc_bf16(128, 128), id64 = umma::idesc_bf16(128, 64);
 
@@ -363,19 +375,16 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
       if (tid == kStorer) umma::bulk_store(image + at, sb + smem, bytes);
     };
     const int64_t b = (int64_t)tile * 128 + row;
-    float x[16];
-    const int k0 = 16 * half;
+    float x[8];
+    const int k0 = 8 * part;
 #pragma unroll
-    for (int k = 0; k < 16; k++) x[k] = k0 + k < kF ? X[b * kF + k0 + k] : 0.0f;
+    for (int k = 0; k < 8; k++) x[k] = k0 + k < kF ? X[b * kF + k0 + k] : 0.0f;
     const float yy = y[b];
     // 1. normalised bf16 inputs
 #pragma unroll
-    for (int k = 0; k < 16; k++)
+    for (int k = 0; k < 8; k++)
       if (k0 + k < kF) x[k] = (fminf(x[k], s_nrm[k0 + k]) - s_nrm[kF + k0 + k]) * s_nrm[2 * kF + k0 + k];
-#pragma unroll
-    for (int j = 0; j < 2; j++)
-      *chunk(kTX0, k0 + 8 * j) = make_uint4(pack_bf16(x[8 * j], x[8 * j + 1]), pack_bf16(x[8 * j + 2], x[8 * j + 3]),
-                                            pack_bf16(x[8 * j + 4], x[8 * j + 5]), pack_bf16(x[8 * j + 6], x[8 * j + 7]));
+    *chunk(kTX0, k0) = make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
     handoff();
     store(kTX0, kTX0, kAtom);
     // 2. layer 1 (K = 32)
@@ -411,57 +420,68 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
       umma::mma_commit(&bar);
     }
     if (!(ok = wait())) break;
-    // 5. output layer, loss, dS3 = dz w4 act'(S3).  Both threads of a row
-    //    form the whole dot product (in the order of a 32-lane exchange over
-    //    fma(a[l], w[l], a[l+32] w[l+32])); each forms its half of dS3.
+    // 5. output layer, loss, dS3 = dz w4 act'(S3).  The row's dot product is
+    //    summed in the order of a 32-lane exchange over
+    //    fma(a[l], w[l], a[l+32] w[l+32]): the quarters 2 and 3 hand their
+    //    products to 0 and 1, quarter 1 its sums to 0.
     {
-      float t[32], a3[32];
-      uint32_t s3[16];
+      const int c = 16 * part;
+      float a3[16];
+      uint32_t s3[8];
+      float* scr = reinterpret_cast<float*>(base + kTScr) + (part & 1) * 16 * 128 + row;
+      {
+        uint32_t v[16];
+        umma::tmem_ld16_issue(tlane + kCAcc + c, v);
+        umma::tmem_ld16_wait(v);
 #pragma unroll
-      for (int p = 1; p >= 0; p--)
-#pragma unroll
-        for (int c = 0; c < 32; c += 16) {
-          uint32_t v[16];
-          umma::tmem_ld16_issue(tlane + kCAcc + 32 * p + c, v);
-          umma::tmem_ld16_wait(v);
-#pragma unroll
-          for (int i = 0; i < 8; i++) {
-            const int n = 32 * p + c + 2 * i;
-            uint32_t s;
-            float2 f;
-            train_act<ACT>(__uint_as_float(v[2 * i]) + s_b3[n], __uint_as_float(v[2 * i + 1]) + s_b3[n + 1], &s, &f);
-            t[c + 2 * i] = p == 1 ? f.x * s_w4[n] : fmaf(f.x, s_w4[n], t[c + 2 * i]);
-            t[c + 2 * i + 1] = p == 1 ? f.y * s_w4[n + 1] : fmaf(f.y, s_w4[n + 1], t[c + 2 * i + 1]);
-            if (p == half) {
-              s3[(c + 2 * i) / 2] = s;
-              a3[c + 2 * i] = f.x;
-              a3[c + 2 * i + 1] = f.y;
-            }
-          }
+        for (int i = 0; i < 8; i++) {
+          float2 f;
+          train_act<ACT>(__uint_as_float(v[2 * i]) + s_b3[c + 2 * i], __uint_as_float(v[2 * i + 1]) + s_b3[c + 2 * i + 1], &s3[i], &f);
+          a3[2 * i] = f.x;
+          a3[2 * i + 1] = f.y;
         }
+      }
+      if (part >= 2)
 #pragma unroll
-      for (int o = 16; o; o >>= 1)
+        for (int i = 0; i < 16; i++) scr[i * 128] = a3[i] * s_w4[c + i];
+      __syncthreads();
+      float t[16];
+      if (part < 2)
 #pragma unroll
-        for (int i = 0; i < o; i++) t[i] += t[i + o];
-      const float z = t[0] + s_b4;
+        for (int i = 0; i < 16; i++) t[i] = fmaf(a3[i], s_w4[c + i], scr[i * 128]);
+      if (part == 1)
+#pragma unroll
+        for (int i = 0; i < 16; i++) scr[i * 128] = t[i];
+      __syncthreads();
+      if (part == 0) {
+#pragma unroll
+        for (int i = 0; i < 16; i++) t[i] += scr[(16 + i) * 128];
+#pragma unroll
+        for (int o = 8; o; o >>= 1)
+#pragma unroll
+          for (int i = 0; i < o; i++) t[i] += t[i + o];
+        s_z[row] = t[0] + s_b4;
+      }
+      __syncthreads();
+      const float z = s_z[row];
       const float prob = 1.0f / (1.0f + expf(-z));
       // BCE with logits, stable form
       const float l = fmaxf(z, 0.0f) - z * yy + log1pf(expf(-fabsf(z)));
       const float g = (prob - yy) / (float)B;
       loss += l / (float)B;
       db4 += g;
-      float d[32];
+      float d[16];
 #pragma unroll
-      for (int i = 0; i < 16; i++) {
+      for (int i = 0; i < 8; i++) {
         const float2 dg = train_grad<ACT>(s3[i]);
-        d[2 * i] = g * s_w4[32 * half + 2 * i] * dg.x;
-        d[2 * i + 1] = g * s_w4[32 * half + 2 * i + 1] * dg.y;
+        d[2 * i] = g * s_w4[c + 2 * i] * dg.x;
+        d[2 * i + 1] = g * s_w4[c + 2 * i + 1] * dg.y;
         a3[2 * i] *= g;
         a3[2 * i + 1] *= g;
       }
 #pragma unroll
-      for (int i = 0; i < 4; i++)
-        *chunk(kTD3, 32 * half + 8 * i) =
+      for (int i = 0; i < 2; i++)
+        *chunk(kTD3, c + 8 * i) =
             make_uint4(pack_bf16(d[8 * i], d[8 * i + 1]), pack_bf16(d[8 * i + 2], d[8 * i + 3]),
                        pack_bf16(d[8 * i + 4], d[8 * i + 5]), pack_bf16(d[8 * i + 6], d[8 * i + 7]));
       db3 += warp_colsum(d, lane);
@@ -500,15 +520,14 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     atomicExch(status, 1);
     umma::mbar_wait(&bar, phase ^ 1u, kWaitLimit);
   }
-  // the four warps of a half cover the tile's rows: their column sums added in order
-#pragma unroll
-  for (int i = 0; i < 2; i++) {
-    s_red[quad][64 * half + 32 * i + lane] = db1[i];
-    s_red[quad][kH1 + 64 * half + 32 * i + lane] = db2[i];
+  // the four warps of a quarter cover the tile's rows: their column sums added in order
+  s_red[quad][32 * part + lane] = db1;
+  s_red[quad][kH1 + 32 * part + lane] = db2;
+  if (lane < 16) {
+    s_red[quad][kH1 + kH2 + 16 * part + lane] = db3;
+    s_red[quad][kH1 + kH2 + kH3 + 16 * part + lane] = dw4;
   }
-  s_red[quad][kH1 + kH2 + 32 * half + lane] = db3;
-  s_red[quad][kH1 + kH2 + kH3 + 32 * half + lane] = dw4;
-  if (half == 0) {
+  if (part == 0) {
     for (int k = 16; k; k >>= 1) {
       db4 += __shfl_xor_sync(0xffffffffu, db4, k);
       loss += __shfl_xor_sync(0xffffffffu, loss, k);
@@ -552,6 +571,7 @@ __device__ __forceinline__ void finish_grad(const AdamStep& a, float* __restrict
 }
 
 constexpr int kWgradThreads = 128, kWgradStages = 6, kWgradBlocks = 8;
+constexpr int kSplitMin = 8, kSplitMax = 64;  // tiles of a batch whose chains are split
 constexpr uint32_t kStageBytes = 2 * kAtom;
 constexpr size_t kSmWgrad = 1024 + kWgradStages * kStageBytes;
 constexpr int kSumBlocks = (kSums + kWgradThreads - 1) / kWgradThreads;
@@ -559,14 +579,21 @@ constexpr int kSumBlocks = (kSums + kWgradThreads - 1) / kWgradThreads;
 // Blocks 0..7: a 64 x 64 block of a weight gradient each, D[m][n] = sum over
 // the samples of U[b][m] V[b][n] with U, V one 64-column atom of the stored
 // operands; the further blocks: the sums over the training kernel's CTAs.
-template <bool STEP>
+// The grid starts beside mlp_train_kernel's; what that stored is read, and the
+// parameters are written, only after its end.
+__device__ __forceinline__ void wait_for_train() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// SPLIT CTAs of a cluster take a quarter of the tiles of one block each; a
+// quarter of the block's columns is then summed in each, in sample order.
+template <bool STEP, int SPLIT>
 __global__ void __launch_bounds__(kWgradThreads, 1)
     mlp_wgrad_kernel(const unsigned char* __restrict__ images, int tiles, const float* __restrict__ sums, int ctas,
                      AdamStep a, float* __restrict__ grads, float* __restrict__ loss, int* __restrict__ status) {
-  const int r = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int r = blockIdx.x / SPLIT, part = blockIdx.x % SPLIT, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (r >= kWgradBlocks) {
-    const int i = (r - kWgradBlocks) * kWgradThreads + tid;
+    const int i = ((int)blockIdx.x - kWgradBlocks * SPLIT) * kWgradThreads + tid;
     if (i >= kSums) return;
+    wait_for_train();
     float g = 0.0f;
 #pragma unroll 8
     for (int c = 0; c < ctas; c++) g += sums[(size_t)c * kSums + i];
@@ -599,17 +626,19 @@ __global__ void __launch_bounds__(kWgradThreads, 1)
   umma::tc_fence_before();
   __syncthreads();
   umma::tc_fence_after();
+  wait_for_train();
   const uint32_t tm = tmem_base;
   const uint32_t u = r < 4 ? kID2 + (r & 1) * kAtom : r < 6 ? kTA2 + (r - 4) * kAtom : kID1 + (r - 6) * kAtom;
   const uint32_t v = r < 4 ? kTA1 + (r >> 1) * kAtom : r < 6 ? kTD3 : kTX0;
+  const int t0 = (int)((int64_t)tiles * part / SPLIT), nt = (int)((int64_t)tiles * (part + 1) / SPLIT) - t0;
   if (tid == 0) {  // producer
-    for (int t = 0; t < tiles; t++) {
+    for (int t = 0; t < nt; t++) {
       const int s = t % kWgradStages, n = t / kWgradStages;
       if (n > 0 && !umma::mbar_wait(&empty[s], (uint32_t)(n - 1) & 1u, kWaitLimit)) {
         s_fail = 1;
         break;
       }
-      const unsigned char* image = images + (size_t)t * kImage;
+      const unsigned char* image = images + (size_t)(t0 + t) * kImage;
       umma::mbar_expect_tx(&full[s], kStageBytes);
       umma::bulk_load(sb + s * kStageBytes, image + u, kAtom, &full[s]);
       umma::bulk_load(sb + s * kStageBytes + kAtom, image + v, kAtom, &full[s]);
@@ -617,7 +646,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1)
   } else if (tid == 32) {  // MMAs, in sample order
     constexpr uint32_t id = umma::idesc_bf16(64, 64) | umma::kTransposeA | umma::kTransposeB;
     bool ok = true;
-    for (int t = 0; t < tiles && ok; t++) {
+    for (int t = 0; t < nt && ok; t++) {
       const int s = t % kWgradStages, n = t / kWgradStages;
       ok = umma::mbar_wait(&full[s], (uint32_t)n & 1u, kWaitLimit);
       if (!ok) break;
@@ -638,22 +667,52 @@ __global__ void __launch_bounds__(kWgradThreads, 1)
     // record it and let the copies in flight land (bounded) before the CTA ends
     if (tid == 0) {
       atomicExch(status, 1);
-      for (int s = 0; s < kWgradStages && s < tiles; s++)
-        umma::mbar_wait(&full[s], (uint32_t)((tiles - 1 - s) / kWgradStages) & 1u, kWaitLimit);
+      for (int s = 0; s < kWgradStages && s < nt; s++)
+        umma::mbar_wait(&full[s], (uint32_t)((nt - 1 - s) / kWgradStages) & 1u, kWaitLimit);
     }
-  } else {
-    // row m of a 64-row accumulator: lane m % 16 of the tensor-memory quarter m / 16
-    const int m = 16 * warp + lane;
+  }
+  auto finish = [&](int m, int n, float g) {
+    if (r < 4) finish_grad<STEP>(a, grads, kOffW2 + (64 * (r & 1) + m) * kH1 + 64 * (r >> 1) + n, g);
+    else if (r < 6) finish_grad<STEP>(a, grads, kOffW3 + n * kH2 + 64 * (r - 4) + m, g);
+    else if (n < kF) finish_grad<STEP>(a, grads, kOffW1 + (64 * (r - 6) + m) * kF + n, g);
+  };
+  // row m of a 64-row accumulator: lane m % 16 of the tensor-memory quarter m / 16
+  const int m = 16 * warp + lane;
+  if (SPLIT > 1) {
+    // this CTA's sums as [column][row], in the ring that every MMA has read
+    float* own = reinterpret_cast<float*>(smem_raw + (sb - umma::smem_u32(smem_raw)));
+    if (!s_fail)
+      for (int c = 0; c < 64; c += 16) {
+        float g[16];
+        umma::tmem_ld16(tm + ((uint32_t)(warp * 32) << 16) + c, g);
+        if (lane < 16)
+#pragma unroll
+          for (int i = 0; i < 16; i++) own[(c + i) * 64 + m] = g[i];
+        __syncwarp();
+      }
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    cl.sync();
+    constexpr int kCols = 64 / SPLIT;
+    bool failed = false;  // any of the four
+#pragma unroll
+    for (int q = 0; q < SPLIT; q++) failed |= *cl.map_shared_rank(&s_fail, q) != 0;
+#pragma unroll
+    for (int i = tid; i < kCols * 64 && !failed; i += kWgradThreads) {
+      const int n = part * kCols + (i >> 6), k = i & 63;
+      float g = 0.0f;
+#pragma unroll
+      for (int q = 0; q < SPLIT; q++) g += cl.map_shared_rank(own, q)[n * 64 + k];
+      finish(k, n, g);
+    }
+    cl.sync();  // a CTA's shared memory is read by the others until here
+  } else if (!s_fail) {
     for (int c = 0; c < 64; c += 16) {
       float g[16];
       umma::tmem_ld16(tm + ((uint32_t)(warp * 32) << 16) + c, g);
       if (lane < 16) {
 #pragma unroll
         for (int i = 0; i < 16; i++) {
-          const int n = c + i;
-          if (r < 4) finish_grad<STEP>(a, grads, kOffW2 + (64 * (r & 1) + m) * kH1 + 64 * (r >> 1) + n, g[i]);
-          else if (r < 6) finish_grad<STEP>(a, grads, kOffW3 + n * kH2 + 64 * (r - 4) + m, g[i]);
-          else if (n < kF) finish_grad<STEP>(a, grads, kOffW1 + (64 * (r - 6) + m) * kF + n, g[i]);
+          finish(m, c + i, g[i]);
         }
       }
       __syncwarp();
@@ -681,18 +740,39 @@ size_t carve_mlp(cbmv_mlp* n, char* base) {
   return off + 256;
 }
 
+template <bool STEP, int SPLIT>
+int launch_wgrad(const cbmv_mlp* n, const AdamStep& a, float* grads, float* loss, cudaStream_t st) {
+  static_assert(kSumBlocks % SPLIT == 0 && 64 % SPLIT == 0, "whole clusters");
+  CBMV_CUDA(cudaFuncSetAttribute(mlp_wgrad_kernel<STEP, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmWgrad));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kWgradBlocks * SPLIT + kSumBlocks);
+  cfg.blockDim = dim3(kWgradThreads);
+  cfg.dynamicSmemBytes = kSmWgrad;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2] = {};
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = SPLIT;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
+  CBMV_CUDA(cudaLaunchKernelEx(&cfg, mlp_wgrad_kernel<STEP, SPLIT>, (const unsigned char*)n->images, n->B / 128,
+                               (const float*)n->sums, n->ctas, a, grads, loss, n->status));
+  return check_launch("mlp_wgrad");
+}
+
 // Forward and backward of one batch, then Adam (STEP) or the gradients.
 template <int ACT, bool STEP>
 int launch_train(const cbmv_mlp* n, const float* X, const float* y, const AdamStep& a, float* grads, float* loss,
                  cudaStream_t st) {
   CBMV_CUDA(cudaFuncSetAttribute(mlp_train_kernel<ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmTrain));
-  CBMV_CUDA(cudaFuncSetAttribute(mlp_wgrad_kernel<STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmWgrad));
   mlp_train_kernel<ACT><<<n->ctas, kTrainThreads, kSmTrain, st>>>(X, y, n->P, n->B, n->images, n->sums, n->status);
   int rc = check_launch("mlp_train");
   if (rc) return rc;
-  mlp_wgrad_kernel<STEP><<<kWgradBlocks + kSumBlocks, kWgradThreads, kSmWgrad, st>>>(n->images, n->B / 128, n->sums,
-                                                                                     n->ctas, a, grads, loss, n->status);
-  return check_launch("mlp_wgrad");
+  const int tiles = n->B / 128;
+  return tiles >= kSplitMin && tiles <= kSplitMax ? launch_wgrad<STEP, 4>(n, a, grads, loss, st)
+                                                  : launch_wgrad<STEP, 1>(n, a, grads, loss, st);
 }
 
 template <bool STEP>
