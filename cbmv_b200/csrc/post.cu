@@ -861,7 +861,20 @@ __global__ void __launch_bounds__(256) cbca_mask_build_kernel(const float* __res
 }
 
 // One CBCA pass from the precomputed supports (same tiling and summation
-// order as cbca_hwd_sep_kernel<kMaskHalo>).
+// order as cbca_hwd_sep_kernel<kMaskHalo>).  Bound by instruction issue (two
+// per tap, 22 taps) with too few warps to cover its loads, so what stands
+// between the loads is kept out: supports never leave the image, so columns
+// are clamped and rows outside skipped instead of tested per value; the eight
+// support words of a column step are read together; and the division is a
+// multiplication by the count's reciprocal with one correction (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000",
+// 1990), which rounds as the division does for every float32 significand and
+// every count (all checked) while no exponent nears its limits; a step that
+// holds any other value, or a copied one, is done again with the division.
+// 694x554 D=128: 192 us per pass (240 before), 901x600 D=192 403 (499),
+// 1482x994 D=256 1522 (1922).  Measured beside it: two disparities per lane
+// 208-253 us, a ring of row sums down taller tiles 283, the next row's values
+// loaded ahead 234.
 template <int CS_TY>
 __global__ void __launch_bounds__(256, 4) cbca_hwd_mask_kernel(const uint32_t* __restrict__ mask,
                                                                const float* __restrict__ in, int H, int W,
@@ -872,62 +885,87 @@ __global__ void __launch_bounds__(256, 4) cbca_hwd_mask_kernel(const uint32_t* _
   constexpr int G = 8;
   static_assert(CS_TX == 8 && CS_TY % G == 0, "one warp per tile column");
   extern __shared__ float sR[];  // [SR][CS_TX][CS_TD]
+  __shared__ float2 s_div[128];  // a count and its reciprocal
   const int ntd = (D + CS_TD - 1) / CS_TD, ntx = (W + CS_TX - 1) / CS_TX;
   const int64_t t = blockIdx.x;
   const int td = (int)(t % ntd), tx = (int)((t / ntd) % ntx), ty = (int)(t / ((int64_t)ntd * ntx));
   const int X0 = tx * CS_TX, Y0 = ty * CS_TY;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int d = td * CS_TD + lane;
-  const bool dok = d < D;
-  // 1. row sums over each (yy, x, d)'s support-row taps
-  for (int r = warp; r < SR; r += 8) {
-    const int yy = Y0 - HALO + r;
-    const bool rok = yy >= 0 && yy < H && dok;
-    const int64_t o = (int64_t)(rok ? yy : 0) * W;
-    const float* row = in + o * D + d;
-    const uint32_t* mrow = mask + o * D + d;
+  const int d = td * CS_TD + lane, dl = min(d, D - 1);  // a lane beyond D reads the last disparity
+  const int64_t WD = (int64_t)W * D;
+  if (threadIdx.x < 128) s_div[threadIdx.x] = make_float2((float)threadIdx.x, 1.0f / (float)threadIdx.x);
+  // 1. row sums over each (yy, x, d)'s support-row taps; what clamped columns
+  //    and skipped rows leave in the tile is never added below
+  const bool interior = X0 >= HALO && X0 + CS_TX + HALO <= W;
+  const int r1 = min(SR, H + HALO - Y0);
+  for (int r = warp + (Y0 < HALO ? (HALO - Y0 - warp + 7) / 8 * 8 : 0); r < r1; r += 8) {
+    const int64_t ro = (int64_t)(Y0 - HALO + r) * W * D + dl;
+    const float* row = in + ro;
     float v[NV];
+    if (interior) {
+      row += (int64_t)(X0 - HALO) * D;
 #pragma unroll
-    for (int j = 0; j < NV; j++) {
-      const int xx = X0 - HALO + j;
-      v[j] = (rok && xx >= 0 && xx < W) ? __ldg(row + (int64_t)xx * D) : 0.0f;
+      for (int j = 0; j < NV; j++, row += D) v[j] = __ldg(row);
+    } else {
+#pragma unroll
+      for (int j = 0; j < NV; j++) v[j] = __ldg(row + (int64_t)min(max(X0 - HALO + j, 0), W - 1) * D);
     }
+    const uint32_t* m = mask + ro + (int64_t)X0 * D;
 #pragma unroll
     for (int c = 0; c < CS_TX; c++) {
-      const int x = X0 + c;
-      const uint32_t hm = (rok && x < W) ? __ldg(mrow + (int64_t)x * D) : 0u;
+      const uint32_t hm = __ldg(m);
       float sum = 0.0f;
 #pragma unroll
-      for (int k = -HALO; k <= HALO; k++)
-        if (hm & (1u << (k + HALO))) sum += v[c + HALO + k];
+      for (int k = 0; k <= 2 * HALO; k++)
+        if (hm & (1u << k)) sum += v[c + k];
       sR[(r * CS_TX + c) * CS_TD + lane] = sum;
+      if (X0 + c + 1 < W) m += D;
     }
   }
   __syncthreads();
   // 2. column sums: warp c owns tile column c; G output rows at a time from
   //    a register window of G + 2*HALO row sums
   const int c = warp, x = X0 + c;
-  if (x >= W || !dok) return;
+  if (x >= W || d >= D) return;
 #pragma unroll 1
   for (int g0 = 0; g0 < CS_TY; g0 += G) {
+    const int n = min(G, H - (Y0 + g0));
+    if (n <= 0) break;
+    const int64_t o = (Y0 + g0) * WD + (int64_t)x * D + d;
+    uint32_t w[G];
+    const uint32_t* m = mask + o;
+#pragma unroll
+    for (int cy = 0; cy < G; cy++) {
+      w[cy] = __ldg(m);
+      if (cy + 1 < n) m += WD;
+    }
     float wr[G + 2 * HALO];
 #pragma unroll
     for (int j = 0; j < G + 2 * HALO; j++) wr[j] = sR[((g0 + j) * CS_TX + c) * CS_TD + lane];
-#pragma unroll
-    for (int cy = 0; cy < G; cy++) {
-      const int y = Y0 + g0 + cy;
-      if (y >= H) break;
-      const int64_t id = ((int64_t)y * W + x) * D + d;
-      const uint32_t w = __ldg(mask + id);
-      if (w & kMaskCopy) {
-        out[id] = __ldg(in + id);
-        continue;
-      }
+    auto column = [&](int cy) {
       float sum = 0.0f;
 #pragma unroll
-      for (int k = -HALO; k <= HALO; k++)
-        if (w & (1u << (k + HALO + 11))) sum += wr[cy + HALO + k];
-      out[id] = sum / (float)((w >> 22) & 0x7Fu);
+      for (int k = 0; k <= 2 * HALO; k++)
+        if (w[cy] & (1u << (k + 11))) sum += wr[cy + k];
+      return sum;
+    };
+    float* dst = out + o;
+    bool again = false;
+#pragma unroll
+    for (int cy = 0; cy < G; cy++, dst += WD) {
+      const float sum = column(cy);
+      const float2 div = s_div[(w[cy] >> 22) & 0x7Fu];
+      const float q = sum * div.y, res = fmaf(fmaf(-q, div.x, sum), div.y, q);
+      again |= !(fabsf(res) <= 0x1p100f) || (fabsf(sum) < 0x1p-90f && sum != 0.0f) || (w[cy] & kMaskCopy);
+      if (cy < n) *dst = res;
+    }
+    if (again) {
+      dst = out + o;
+#pragma unroll
+      for (int cy = 0; cy < G; cy++, dst += WD) {
+        if (cy >= n) break;
+        *dst = w[cy] & kMaskCopy ? __ldg(in + o + cy * WD) : column(cy) / (float)((w[cy] >> 22) & 0x7Fu);
+      }
     }
   }
 }
@@ -1404,9 +1442,9 @@ int launch_cbca_sep(const float* lc, const float* rc, const float* in, int64_t H
 
 // Tiles of the separable CBCA's kernels with `rows` rows each.  A tile's
 // halo costs 10 rows, so 32 rows are the least work (a pass at 694x554 D=128:
-// 238 us); below kCbcaFull tiles (two per SM) they leave SMs idle and each
+// 192 us, 24 rows 205); below kCbcaFull tiles (two per SM) they leave SMs idle and each
 // tile is a longer chain: 96x64 D=16, 24 tiles of 32 rows 19.6 us, 96 of 8
-// rows 6.8 (the support build 26.0 and 20.1 us).
+// rows 5.3 (the support build 26.0 and 20.1 us).
 static unsigned cbca_tiles(int64_t H, int64_t W, int D, int rows) {
   return (unsigned)(((W + CS_TX - 1) / CS_TX) * ((H + rows - 1) / rows) * ((D + CS_TD - 1) / CS_TD));
 }
