@@ -114,6 +114,7 @@ struct Work {
   float *volA, *volB;
   float* volC;  // the right view's cost of the _interp post (else null)
   float *imL, *imR, *crossL, *crossR, *dtmp, *dtmp2, *dright, *outlier;
+  uint32_t* arm_words;  // both views' cross arms as tap words (L1 <= 6)
   void* codes;  // SGM image classes
   uint32_t* masks;  // CBCA support words, 4 B per (p,d), live beside the SGM volumes
   bool prepped = false;  // the post's image terms were launched on the side stream (prep_ev)
@@ -148,6 +149,7 @@ Work carve(void* base, int64_t H, int64_t W, int D, size_t* bytes, bool f32, boo
   w.imR = c.take<float>(HW);
   w.crossL = c.take<float>(4 * HW);
   w.crossR = c.take<float>(4 * HW);
+  w.arm_words = c.take<uint32_t>(2 * HW);
   w.dtmp = c.take<float>(HW);
   w.dtmp2 = c.take<float>(HW);
   w.dright = c.take<float>(HW);
@@ -291,14 +293,16 @@ static int cost_chain(cbmv_ctx* c, const cbmv_params* p, Work& w, int64_t H, int
   // the first pass
   const bool masked = !p->exact_cbca && p->L1 - 1 <= kCbcaMaskMaxHalo;
   uint32_t* masks = w.masks;
+  const uint32_t* wordsA = w.arm_words + (crossA == w.crossR ? HW : 0);
+  const uint32_t* wordsB = w.arm_words + (crossB == w.crossR ? HW : 0);
   const bool beside = masked && p->cbca_i1 == 0 && p->cbca_i2 > 0 && p->sgm_i > 0;
   if (beside) {
     CBMV_CUDA(cudaEventRecord(c->fork_ev, st));
     CBMV_CUDA(cudaStreamWaitEvent(c->side, c->fork_ev, 0));
-    RC(launch_cbca_mask_build(crossA, crossB, H, W, D, direction, masks, c->side));
+    RC(launch_cbca_mask_build(wordsA, wordsB, H, W, D, direction, masks, c->side));
     CBMV_CUDA(cudaEventRecord(c->join_ev, c->side));
   } else if (masked && p->cbca_i1 + p->cbca_i2 > 0) {
-    RC(launch_cbca_mask_build(crossA, crossB, H, W, D, direction, masks, st));
+    RC(launch_cbca_mask_build(wordsA, wordsB, H, W, D, direction, masks, st));
   }
   auto cbca = [&](const float* in, float* out) {
     if (p->exact_cbca)
@@ -344,7 +348,8 @@ static int cost_chain(cbmv_ctx* c, const cbmv_params* p, Work& w, int64_t H, int
 // the call, beside the matchers.
 static int post_prep(const cbmv_params* p, const uint8_t* L, const uint8_t* R, int64_t H, int64_t W, Work& w,
                      cudaStream_t s) {
-  RC(launch_normalise_cross(L, R, H, W, w.mom, p->L1, p->tau1, w.imL, w.imR, w.crossL, w.crossR, s));
+  RC(launch_normalise_cross(L, R, H, W, w.mom, p->L1, p->tau1, w.imL, w.imR, w.crossL, w.crossR,
+                            w.arm_words, s));
   if (p->sgm_i > 0) RC(launch_sgm_codes(w.imL, w.imR, H, W, p->tau_so, sgm_codes_at(w.codes, H, W), s));
   return CBMV_OK;
 }

@@ -618,16 +618,9 @@ int launch_cbca_sep_h(const float* lc, const float* rc, const float* in, int64_t
 constexpr int kMaskHalo = kCbcaMaskMaxHalo;
 constexpr uint32_t kMaskCopy = 1u << 31;
 
-// Relative arms of one pixel packed as four int8: arm a minus the pixel's
-// x (arms 0, 1) or y (arms 2, 3).  cross_kernel's arms lie within L1 of
-// their pixel; anything beyond 127 is clamped (the taps stop at +-5 anyway).
+// A pixel's relative arms as four packed int8: arm a minus the pixel's x
+// (arms 0, 1) or y (arms 2, 3), clamped.
 __device__ __forceinline__ int clamp_i8(int v) { return min(max(v, -128), 127); }
-__device__ __forceinline__ uint32_t pack_rel_arms(const float* __restrict__ c, int64_t HW, int64_t o, int x, int y) {
-  const int a0 = clamp_i8((int)__ldg(c + o) - x), a1 = clamp_i8((int)__ldg(c + HW + o) - x);
-  const int a2 = clamp_i8((int)__ldg(c + 2 * HW + o) - y), a3 = clamp_i8((int)__ldg(c + 3 * HW + o) - y);
-  return (uint32_t)(a0 & 0xFF) | ((uint32_t)(a1 & 0xFF) << 8) | ((uint32_t)(a2 & 0xFF) << 16) |
-         ((uint32_t)(a3 & 0xFF) << 24);
-}
 template <int B>
 __device__ __forceinline__ int rel_arm(uint32_t w) {
   return (int)((int32_t)(w << (24 - 8 * B)) >> 24);
@@ -647,9 +640,9 @@ __device__ __forceinline__ int rel_arm(uint32_t w) {
 // thread per output walking its support (cbca_kernel).
 constexpr int CD_X = 32, CD_Y = 16, CD_D = 8, CD_G = 4, CD_HALO = 5;
 
-// The arms of one pixel packed as pack_rel_arms does, without conversions
-// (an arm below 2^22 is read off its sum with 1.5 * 2^23); *odd: one of them
-// is no whole number, or too large for that.
+// The relative arms of one pixel, packed without conversions (an arm below
+// 2^22 is read off its sum with 1.5 * 2^23); *odd: one of them is no whole
+// number, or too large for that.
 __device__ __forceinline__ uint32_t pack_whole_arms(const float* __restrict__ c, int64_t HW, int64_t o, int x, int y,
                                                     bool* odd) {
   constexpr float kMagic = 12582912.0f;
@@ -761,102 +754,76 @@ __global__ void __launch_bounds__(32 * CD_D) cbca_dhw_kernel(const float* __rest
   }
 }
 
+// The cross arms of one pixel as the taps they allow: bits 0..10 of its row
+// (tap k at bit k + 5), bits 11..21 of its column; from the reach (0..5
+// pixels) to the left, right, up and down.
+__device__ __forceinline__ uint32_t arm_word(int l, int r, int u, int d) {
+  return ((1u << (l + r + 1)) - 1u) << (kMaskHalo - l) | ((1u << (u + d + 1)) - 1u) << (11 + kMaskHalo - u);
+}
+
+__global__ void arm_words_kernel(const float* __restrict__ lc, const float* __restrict__ rc, int64_t H, int64_t W,
+                                 uint32_t* __restrict__ words) {
+  const int64_t n = H * W;
+  const float* __restrict__ arms = blockIdx.y ? rc : lc;
+  GRID_STRIDE(p, n) {
+    const int y = (int)(p / W), x = (int)(p - y * W);
+    auto reach = [&](int v) { return min(max(v - 1, 0), kMaskHalo); };
+    words[blockIdx.y * n + p] = arm_word(reach(x - (int)arms[p]), reach((int)arms[n + p] - x),
+                                         reach(y - (int)arms[2 * n + p]), reach((int)arms[3 * n + p] - y));
+  }
+}
+
+// The support words from the arm words of the volume's own view (wl) and of
+// the matching view (wr): both arms allow a tap where both words do, so a
+// support is one AND; a support row's length is its number of taps, and the
+// count the difference of two prefix sums of those down the tile's column,
+// which a warp walks once (column = warp, disparity = lane).  Bound by
+// instruction issue, 4 B written per word: 694x554 D=128 89 us (238 from the
+// arms' coordinates), 901x600 D=192 179 (481).
 template <int CS_TY>
-__global__ void __launch_bounds__(256) cbca_mask_build_kernel(const float* __restrict__ lc,
-                                                              const float* __restrict__ rc, int H, int W, int D,
+__global__ void __launch_bounds__(256) cbca_mask_build_kernel(const uint32_t* __restrict__ wl,
+                                                              const uint32_t* __restrict__ wr, int H, int W, int D,
                                                               int direction, uint32_t* __restrict__ mask) {
-  constexpr int HALO = kMaskHalo;
-  constexpr int SR = CS_TY + 2 * HALO;
+  constexpr int HALO = kMaskHalo, SR = CS_TY + 2 * HALO;
   constexpr int NXM = CS_TX + CS_TD - 1;  // matching columns x + d * direction of the tile
-  // support-row lengths of rows 0..SR-1 in sP[1..SR], then (in place)
-  // their prefix sums over the rows: sP[r] = lengths of rows 0..r-1
-  __shared__ uint16_t sP[SR + 1][CS_TX][CS_TD];
-  __shared__ uint16_t sH[CS_TY][CS_TX][CS_TD];  // support-row taps of the tile's own rows
-  __shared__ uint32_t sAL[SR][CS_TX];           // packed relative arms, left view at (yy, x)
-  __shared__ uint32_t sAR[SR][NXM];             // right view at (yy, xm)
+  __shared__ uint16_t sP[SR + 1][CS_TX][CS_TD];  // taps of the rows above, per column and disparity
+  __shared__ uint32_t sL[SR][CS_TX], sR[SR][NXM];
   const int ntd = (D + CS_TD - 1) / CS_TD, ntx = (W + CS_TX - 1) / CS_TX;
   const int64_t t = blockIdx.x;
   const int td = (int)(t % ntd), tx = (int)((t / ntd) % ntx), ty = (int)(t / ((int64_t)ntd * ntx));
   const int X0 = tx * CS_TX, Y0 = ty * CS_TY;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int d = td * CS_TD + lane, dd = d * direction;
-  const bool dok = d < D;
-  const int64_t HW = (int64_t)H * W;
-  // the tile's matching columns: X0 + d * direction over its disparities
+  const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
   const int xm_lo = direction > 0 ? X0 + td * CS_TD : X0 - (td * CS_TD + CS_TD - 1);
-  // 0. the arms the tile needs, converted once per pixel (rows and columns
-  //    outside the image are never read back)
   for (int q = threadIdx.x; q < SR * (CS_TX + NXM); q += blockDim.x) {
     const int r = q / (CS_TX + NXM), j = q - r * (CS_TX + NXM);
-    const int yy = Y0 - HALO + r;
-    if (yy < 0 || yy >= H) continue;
-    if (j < CS_TX) {
-      const int x = X0 + j;
-      if (x < W) sAL[r][j] = pack_rel_arms(lc, HW, (int64_t)yy * W + x, x, yy);
-    } else {
-      const int xm = xm_lo + (j - CS_TX);
-      if (xm >= 0 && xm < W) sAR[r][j - CS_TX] = pack_rel_arms(rc, HW, (int64_t)yy * W + xm, xm, yy);
-    }
+    const int yy = Y0 - HALO + r, xx = j < CS_TX ? X0 + j : xm_lo + j - CS_TX;
+    const bool in = yy >= 0 && yy < H && xx >= 0 && xx < W;
+    if (j < CS_TX) sL[r][j] = in ? __ldg(wl + (int64_t)yy * W + xx) : 0u;
+    else sR[r][j - CS_TX] = in ? __ldg(wr + (int64_t)yy * W + xx) : 0u;
   }
   __syncthreads();
-  // 1. support rows of the tile's rows and HALO rows above and below
-  for (int r = warp; r < SR; r += 8) {
-    const int yy = Y0 - HALO + r;
-    const bool rok = yy >= 0 && yy < H && dok;
-#pragma unroll
-    for (int c = 0; c < CS_TX; c++) {
-      const int x = X0 + c, xm = x + dd;
-      int cnt = 0;
-      uint32_t hm = 0;
-      if (rok && x < W && xm >= 0 && xm < W) {
-        const uint32_t wl = sAL[r][c], wr = sAR[r][xm - xm_lo];
-        // max(lc0[x], rc0[xm] - dd) - x and min(lc1[x], rc1[xm] - dd) - x
-        const int ks = max(rel_arm<0>(wl), rel_arm<0>(wr));
-        const int kt = min(rel_arm<1>(wl), rel_arm<1>(wr));
-        cnt = max(kt - ks - 1, 0);
-        const int lo = max(ks + 1, -HALO), hi = min(kt - 1, HALO);
-        if (hi >= lo) hm = ((1u << (hi - lo + 1)) - 1u) << (lo + HALO);
-      }
-      sP[r + 1][c][lane] = (uint16_t)cnt;
-      if (r >= HALO && r < HALO + CS_TY) sH[r - HALO][c][lane] = (uint16_t)hm;
-    }
-  }
-  __syncthreads();
-  // 2. support columns: warp c owns tile column c; the thread first forms
-  //    the prefix sums of its (column, disparity)'s support-row lengths, so
-  //    a support of rows lo..hi counts sP[hi + 1] - sP[lo] pixels (exact
-  //    integers, the same count as adding them row by row)
-  const int c = warp, x = X0 + c, xm = x + dd;
-  {
-    uint32_t run = 0;
-    sP[0][c][lane] = 0;
-    for (int r = 1; r <= SR; r++) {
-      run += sP[r][c][lane];
-      sP[r][c][lane] = (uint16_t)run;
-    }
-  }
-  if (x >= W || !dok) return;
+  const int d = td * CS_TD + lane, x = X0 + c, xm = x + d * direction;
+  if (x >= W || d >= D) return;
+  const int j = c + (direction > 0 ? lane : CS_TD - 1 - lane);
   const bool xok = xm >= 0 && xm < W;
-  for (int cy = 0; cy < CS_TY; cy++) {
-    const int y = Y0 + cy;
-    if (y >= H) break;
-    const int64_t id = ((int64_t)y * W + x) * D + d;
-    if (!xok) {
-      mask[id] = kMaskCopy;
-      continue;
-    }
-    const uint32_t wl = sAL[cy + HALO][c], wr = sAR[cy + HALO][xm - xm_lo];
-    // max(lc2[x], rc2[xm]) - y and min(lc3[x], rc3[xm]) - y: the support
-    // rows are the taps k with ks < k < kt, within +-HALO
-    const int ks = max(rel_arm<2>(wl), rel_arm<2>(wr));
-    const int kt = min(rel_arm<3>(wl), rel_arm<3>(wr));
-    const int lo = max(ks + 1, -HALO), hi = min(kt - 1, HALO);
-    uint32_t vm = 0, cnt = 0;
-    if (hi >= lo) {
-      vm = ((1u << (hi - lo + 1)) - 1u) << (lo + HALO);
-      cnt = (uint32_t)sP[cy + HALO + hi + 1][c][lane] - (uint32_t)sP[cy + HALO + lo][c][lane];
-    }
-    mask[id] = (uint32_t)sH[cy][c][lane] | (vm << 11) | ((cnt & 0x7Fu) << 22);
+  uint32_t run = 0;
+  sP[0][c][lane] = 0;
+  auto add_row = [&](int r) {
+    run += __popc(sL[r][c] & sR[r][j] & 0x7FFu);
+    sP[r + 1][c][lane] = (uint16_t)run;
+  };
+#pragma unroll
+  for (int r = 0; r < 2 * HALO; r++) add_row(r);
+  uint32_t* dst = mask + ((int64_t)Y0 * W + x) * D + d;
+  const int n = min(CS_TY, H - Y0);
+#pragma unroll 4
+  for (int cy = 0; cy < n; cy++, dst += (int64_t)W * D) {
+    add_row(cy + 2 * HALO);
+    const int r = cy + HALO;
+    const uint32_t w = sL[r][c] & sR[r][j];
+    const int up = __popc(w & (0x1Fu << 11)), down = __popc(w & (0x1Fu << 17));
+    const uint32_t cnt = (uint32_t)sP[r + down + 1][c][lane] - (uint32_t)sP[r - up][c][lane];
+    *dst = xok ? w | cnt << 22 : kMaskCopy;
   }
 }
 
@@ -1304,14 +1271,16 @@ __global__ void __launch_bounds__(256) moments_kernel(const uint8_t* __restrict_
 // population std, as test.py:489-492 does with numpy on the float32 image,
 // and the cross arms of the result (cross_kernel's).  An 8-bit image has 256
 // normalised values: each block divides them once, and a pixel's neighbours
-// are looked up instead of read from the image the same launch writes.  Bound
+// are looked up instead of read from the image the same launch writes.
+// words (or null): both images' arm_word, for L1 - 1 <= kMaskHalo.  Bound
 // by the arms' chain of dependent reads; both images of 694x554 24 us (77 us
 // as four launches), 96x64 5.9 us (19).
 __global__ void __launch_bounds__(256) normalise_cross_kernel(const uint8_t* __restrict__ L, const uint8_t* __restrict__ R,
                                                             int64_t H, int64_t W,
                                                             const unsigned long long* __restrict__ mom, int L1, float tau1,
                                                             float* __restrict__ imL, float* __restrict__ imR,
-                                                            float* __restrict__ crossL, float* __restrict__ crossR) {
+                                                            float* __restrict__ crossL, float* __restrict__ crossR,
+                                                            uint32_t* __restrict__ words) {
   __shared__ float value[256];
   const int64_t n = H * W;
   const uint8_t* __restrict__ img = blockIdx.y ? R : L;
@@ -1325,6 +1294,7 @@ __global__ void __launch_bounds__(256) normalise_cross_kernel(const uint8_t* __r
     const int64_t y = p / W, x = p - y * W;
     const float c = value[img[p]];
     out[p] = c;
+    int reach[4];
 #pragma unroll
     for (int dir = 0; dir < 4; dir++) {
       // steps to the image's edge, and the pixel offset of one
@@ -1337,7 +1307,9 @@ __global__ void __launch_bounds__(256) normalise_cross_kernel(const uint8_t* __r
         if (k >= L1) break;                                              // rule 2
       }
       arms[dir * n + p] = (float)((dir <= 1 ? x : y) + ((dir & 1) ? k : -k));
+      reach[dir] = (int)k - 1;
     }
+    if (words) words[blockIdx.y * n + p] = arm_word(reach[0], reach[1], reach[2], reach[3]);
   }
 }
 
@@ -1442,23 +1414,23 @@ int launch_cbca_sep(const float* lc, const float* rc, const float* in, int64_t H
 
 // Tiles of the separable CBCA's kernels with `rows` rows each.  A tile's
 // halo costs 10 rows, so 32 rows are the least work (a pass at 694x554 D=128:
-// 192 us, 24 rows 205); below kCbcaFull tiles (two per SM) they leave SMs idle and each
-// tile is a longer chain: 96x64 D=16, 24 tiles of 32 rows 19.6 us, 96 of 8
-// rows 5.3 (the support build 26.0 and 20.1 us).
+// 192 us, 24 rows 205); below kCbcaFull tiles (two per SM) they leave SMs
+// idle and each tile is a longer chain: a pass at 96x64 D=16 with 24 tiles of
+// 32 rows 19.6 us, with 96 of 8 rows 5.3.
 static unsigned cbca_tiles(int64_t H, int64_t W, int D, int rows) {
   return (unsigned)(((W + CS_TX - 1) / CS_TX) * ((H + rows - 1) / rows) * ((D + CS_TD - 1) / CS_TD));
 }
 constexpr unsigned kCbcaFull = 296;
 
-int launch_cbca_mask_build(const float* lc, const float* rc, int64_t H, int64_t W, int D, int direction,
+int launch_cbca_mask_build(const uint32_t* wl, const uint32_t* wr, int64_t H, int64_t W, int D, int direction,
                            uint32_t* mask, cudaStream_t st) {
   CBMV_REQUIRE(H < (1 << 30) && W < (1 << 30) &&
                    (int64_t)((W + CS_TX - 1) / CS_TX) * ((H + 15) / 16) * ((D + CS_TD - 1) / CS_TD) <
                        ((int64_t)1 << 31),
                CBMV_ERANGE, "cbca: volume too large");
   const unsigned tiles32 = cbca_tiles(H, W, D, 32), tiles8 = cbca_tiles(H, W, D, 8);
-  if (tiles32 >= kCbcaFull) cbca_mask_build_kernel<32><<<tiles32, 256, 0, st>>>(lc, rc, (int)H, (int)W, D, direction, mask);
-  else cbca_mask_build_kernel<8><<<tiles8, 256, 0, st>>>(lc, rc, (int)H, (int)W, D, direction, mask);
+  if (tiles32 >= kCbcaFull) cbca_mask_build_kernel<32><<<tiles32, 256, 0, st>>>(wl, wr, (int)H, (int)W, D, direction, mask);
+  else cbca_mask_build_kernel<8><<<tiles8, 256, 0, st>>>(wl, wr, (int)H, (int)W, D, direction, mask);
   return check_launch("cbca_mask_build");
 }
 
@@ -1499,12 +1471,13 @@ int launch_mean2d(const float* in, int64_t H, int64_t W, const float* kernel, in
 }
 
 int launch_normalise_cross(const uint8_t* L, const uint8_t* R, int64_t H, int64_t W, double* mom, int L1, float tau1,
-                           float* imL, float* imR, float* crossL, float* crossR, cudaStream_t st) {
+                           float* imL, float* imR, float* crossL, float* crossR, uint32_t* words, cudaStream_t st) {
   unsigned long long* m = reinterpret_cast<unsigned long long*>(mom);
   const int64_t n = H * W;
   CBMV_CUDA(cudaMemsetAsync(m, 0, 4 * sizeof(unsigned long long), st));
   moments_kernel<<<dim3(grid_for(n / 16 + 1, 256), 2), 256, 0, st>>>(L, R, n, m);
-  normalise_cross_kernel<<<dim3(grid_for(n, 256), 2), 256, 0, st>>>(L, R, H, W, m, L1, tau1, imL, imR, crossL, crossR);
+  normalise_cross_kernel<<<dim3(grid_for(n, 256), 2), 256, 0, st>>>(L, R, H, W, m, L1, tau1, imL, imR, crossL, crossR,
+                                                                         L1 - 1 <= kMaskHalo ? words : nullptr);
   return check_launch("normalise_cross");
 }
 
@@ -1633,8 +1606,11 @@ extern "C" int cbmv_cbca_separable(const float* crossL, const float* crossR, con
   if (L1 - 1 > kCbcaMaskMaxHalo) return launch_cbca_sep(crossL, crossR, in, H, W, D, direction, out, st, L1 - 1);
   // the pipeline's form: supports precomputed into a stream-ordered scratch buffer
   uint32_t* mask = nullptr;
-  CBMV_CUDA(cudaMallocAsync(&mask, sizeof(uint32_t) * H * W * D, st));
-  int rc = launch_cbca_mask_build(crossL, crossR, H, W, D, direction, mask, st);
+  CBMV_CUDA(cudaMallocAsync(&mask, sizeof(uint32_t) * H * W * (D + 2), st));
+  uint32_t* words = mask + H * W * D;
+  arm_words_kernel<<<dim3(grid_for(H * W, kBlock), 2), kBlock, 0, st>>>(crossL, crossR, H, W, words);
+  int rc = check_launch("arm_words");
+  if (rc == CBMV_OK) rc = launch_cbca_mask_build(words, words + H * W, H, W, D, direction, mask, st);
   if (rc == CBMV_OK) rc = launch_cbca_masked(mask, in, H, W, D, out, st);
   CBMV_CUDA(cudaFreeAsync(mask, st));
   return rc;

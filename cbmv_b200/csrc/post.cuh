@@ -49,7 +49,7 @@ int launch_cbca_sep(const float* lc, const float* rc, const float* in, int64_t H
 // the separable cbca with its supports precomputed (arms of at most 5
 // pixels, L1 <= 6): one 32-bit word per (p,d) in `mask`, built once per
 // cross, then any number of passes; bit-identical to launch_cbca_sep
-int launch_cbca_mask_build(const float* lc, const float* rc, int64_t H, int64_t W, int D, int direction,
+int launch_cbca_mask_build(const uint32_t* wl, const uint32_t* wr, int64_t H, int64_t W, int D, int direction,
                            uint32_t* mask, cudaStream_t st);
 int launch_cbca_masked(const uint32_t* mask, const float* in, int64_t H, int64_t W, int D, float* out,
                        cudaStream_t st, int rows = 0);
@@ -59,9 +59,10 @@ int launch_wta_subpixel(const float* cost, int64_t H, int64_t W, int D, float* d
 int launch_median(const float* in, int64_t H, int64_t W, int k, float* out, cudaStream_t st);
 int launch_mean2d(const float* in, int64_t H, int64_t W, const float* kernel, int ks, float alpha2,
                   float* out, cudaStream_t st);
-// do_post's normalisation (test.py:485-504) of both images and their cross arms; mom: 4 doubles of scratch
+// do_post's normalisation (test.py:485-504) of both images, their cross arms and (L1 - 1 <= kCbcaMaskMaxHalo) the
+// arms as tap words, left view's [H, W] then right view's; mom: 4 doubles of scratch
 int launch_normalise_cross(const uint8_t* L, const uint8_t* R, int64_t H, int64_t W, double* mom, int L1, float tau1,
-                           float* imL, float* imR, float* crossL, float* crossR, cudaStream_t st);
+                           float* imL, float* imR, float* crossL, float* crossR, uint32_t* words, cudaStream_t st);
 // get_right_cost of a float32 [H,W,D] volume (the _interp post's right view)
 int launch_right_cost_f32(const float* in, int64_t H, int64_t W, int D, float* out, cudaStream_t st);
 int launch_outlier(const float* d0, const float* d1, int64_t H, int64_t W, int disp_max, float* out,
