@@ -272,6 +272,12 @@ static int ensure_gaussian(cbmv_ctx* c, float sigma) {
     if (rc_) return rc_;      \
   } while (0)
 
+// Whether a caller's cost volume is used where it lies: the classifier writes
+// it and the chain's first pass reads it there (a copy of a 694x554 D=128
+// volume takes 64 us).  One that is not 16-byte aligned is copied, so that
+// the passes keep their vector accesses.
+static bool in_place(const float* volume) { return volume && (uintptr_t)volume % 16 == 0; }
+
 // The cost-optimisation chain of Testing.__postprocessing_mem
 // (test.py:355-405) on one float32 [H,W,D] cost volume held in `cur`:
 // cbca_i1 CBCA passes, sgm_i SGM iterations (each the mean of the four
@@ -279,11 +285,13 @@ static int ensure_gaussian(cbmv_ctx* c, float sigma) {
 // are the arms of the volume's own view and of the matching view: the left
 // view's chain passes (left, right, direction); the right view's chain of
 // the _interp post (test.py:176-251) passes (right, left, -direction), and
-// its SGM keeps the images in their order (test.py:203-207).  `oth` is a
-// second volume; *result receives the buffer holding the result.
+// its SGM keeps the images in their order (test.py:203-207).  The first pass
+// reads `cur` and writes `oth`; from then on `oth` and `spare` alternate, so
+// `cur` is left as it is unless it is `spare` as well.  *result receives the
+// buffer holding the result.
 static int cost_chain(cbmv_ctx* c, const cbmv_params* p, Work& w, int64_t H, int64_t W, int D,
-                      const float* crossA, const float* crossB, int direction, float* cur, float* oth,
-                      float** result) {
+                      const float* crossA, const float* crossB, int direction, const float* cur, float* oth,
+                      float* spare, const float** result) {
   cudaStream_t st = c->stream;
   const int64_t HW = H * W;
   // the separable form's supports, built once for all the chain's passes
@@ -310,9 +318,14 @@ static int cost_chain(cbmv_ctx* c, const cbmv_params* p, Work& w, int64_t H, int
     if (masked) return launch_cbca_masked(masks, in, H, W, D, out, st, p->cbca_rows);
     return launch_cbca_sep(crossA, crossB, in, H, W, D, direction, out, st, p->L1 - 1, p->cbca_rows == 16 ? 16 : 32);
   };
+  auto swap = [&]() {  // `oth` holds the newest volume
+    cur = oth;
+    oth = spare;
+    spare = const_cast<float*>(cur);
+  };
   for (int i = 0; i < p->cbca_i1; i++) {
     RC(cbca(cur, oth));
-    float* t = cur; cur = oth; oth = t;
+    swap();
   }
   SgmParams sp{p->pi1, p->pi2, p->tau_so, p->alpha1, p->sgm_q1, p->sgm_q2, direction};
   const SgmCodes g = sgm_codes_at(w.codes, H, W);
@@ -324,18 +337,18 @@ static int cost_chain(cbmv_ctx* c, const cbmv_params* p, Work& w, int64_t H, int
     // out = ((L0 + L1 + L2) + L3) / 4   (test.py:379-383)
     RC(launch_sgm4(g, cur, H, W, D, sp, so, st));
     RC(launch_sgm_combine(so, V, nullptr, 0.25f, oth, st));
-    float* t = cur; cur = oth; oth = t;
+    swap();
   }
   if (beside) CBMV_CUDA(cudaStreamWaitEvent(st, c->join_ev, 0));
   for (int i = 0; i < p->cbca_i2; i++) {
     RC(cbca(cur, oth));
-    float* t = cur; cur = oth; oth = t;
+    swap();
   }
   *result = cur;
   return CBMV_OK;
 }
 
-// Step 5 of the header comment on the float32 volume in w.volA; the
+// Step 5 of the header comment on the float32 volume `cost` (read only unless it is w.volA); the
 // disparity lands in `disp`.  p->interpolate = 0: the _mem post
 // (test.py:341-449); 1: the _interp post (test.py:153-338), which first runs
 // the right view's chain on get_right_cost of the cost (its winner-take-all
@@ -355,21 +368,21 @@ static int post_prep(const cbmv_params* p, const uint8_t* L, const uint8_t* R, i
 }
 
 static int run_post(cbmv_ctx* c, const cbmv_params* p, const uint8_t* L, const uint8_t* R,
-                    int64_t H, int64_t W, int D, Work& w, float* disp) {
+                    int64_t H, int64_t W, int D, Work& w, const float* cost, float* disp) {
   cudaStream_t st = c->stream;
   RC(ensure_gaussian(c, p->blur_sigma));
   if (w.prepped)
     CBMV_CUDA(cudaStreamWaitEvent(st, c->prep_ev, 0));
   else
     RC(post_prep(p, L, R, H, W, w, st));
-  float* res = nullptr;
+  const float* res = nullptr;
   if (p->interpolate) {
     // right view (test.py:154, 176-255): its cost, its chain, its argmin
-    RC(launch_right_cost_f32(w.volA, H, W, D, w.volC, st));
-    RC(cost_chain(c, p, w, H, W, D, w.crossR, w.crossL, -p->direction, w.volC, w.volB, &res));
+    RC(launch_right_cost_f32(cost, H, W, D, w.volC, st));
+    RC(cost_chain(c, p, w, H, W, D, w.crossR, w.crossL, -p->direction, w.volC, w.volB, w.volC, &res));
     RC(launch_wta_subpixel(res, H, W, D, w.dright, nullptr, st));
   }
-  RC(cost_chain(c, p, w, H, W, D, w.crossL, w.crossR, p->direction, w.volA, w.volB, &res));
+  RC(cost_chain(c, p, w, H, W, D, w.crossL, w.crossR, p->direction, cost, w.volB, w.volA, &res));
   float* d0 = w.dtmp;
   float* d1 = w.dtmp2;
   if (p->interpolate) {
@@ -481,11 +494,12 @@ extern "C" int cbmv_run_rf(cbmv_ctx* c, const cbmv_forest* f, const cbmv_params*
   RC(run_front(c, p, L, R, H, W, D, &w, false, true));
   cudaStream_t st = c->stream;
   const double* vols[4] = {w.vol[0], w.vol[1], w.vol[2], w.vol[3]};
-  RC(launch_features_rf(vols, w.stats, H, W, D, f, w.volA, st));
-  if (prob0)
-    CBMV_CUDA(cudaMemcpyAsync(prob0, w.volA, sizeof(float) * H * W * D, cudaMemcpyDeviceToDevice, st));
+  float* cost = in_place(prob0) ? prob0 : w.volA;
+  RC(launch_features_rf(vols, w.stats, H, W, D, f, cost, st));
+  if (prob0 && cost != prob0)
+    CBMV_CUDA(cudaMemcpyAsync(prob0, cost, sizeof(float) * H * W * D, cudaMemcpyDeviceToDevice, st));
   CBMV_CUDA(cudaEventRecord(c->ev[3], st));
-  RC(run_post(c, p, L, R, H, W, D, w, disp));
+  RC(run_post(c, p, L, R, H, W, D, w, cost, disp));
   CBMV_CUDA(cudaEventRecord(c->ev[4], st));
   return CBMV_OK;
 }
@@ -499,11 +513,12 @@ extern "C" int cbmv_run_mlp(cbmv_ctx* c, const cbmv_mlp* m, const cbmv_params* p
   RC(run_front(c, p, L, R, H, W, D, &w, true, true));
   cudaStream_t st = c->stream;
   const float* vols[4] = {(float*)w.vol[0], (float*)w.vol[1], (float*)w.vol[2], (float*)w.vol[3]};
-  RC(launch_features_mlp(vols, w.statsf, H, W, D, m, w.volA, st, p->mlp_ctas));
-  if (prob0)
-    CBMV_CUDA(cudaMemcpyAsync(prob0, w.volA, sizeof(float) * H * W * D, cudaMemcpyDeviceToDevice, st));
+  float* cost = in_place(prob0) ? prob0 : w.volA;
+  RC(launch_features_mlp(vols, w.statsf, H, W, D, m, cost, st, p->mlp_ctas));
+  if (prob0 && cost != prob0)
+    CBMV_CUDA(cudaMemcpyAsync(prob0, cost, sizeof(float) * H * W * D, cudaMemcpyDeviceToDevice, st));
   CBMV_CUDA(cudaEventRecord(c->ev[3], st));
-  RC(run_post(c, p, L, R, H, W, D, w, disp));
+  RC(run_post(c, p, L, R, H, W, D, w, cost, disp));
   CBMV_CUDA(cudaEventRecord(c->ev[4], st));
   return CBMV_OK;
 }
@@ -574,8 +589,11 @@ extern "C" int cbmv_run_post(cbmv_ctx* c, const cbmv_params* p, const uint8_t* L
   Work w = carve(c->ws, H, W, D, &bytes, true, p->interpolate != 0);
   cudaStream_t st = c->stream;
   for (int i = 0; i < 4; i++) CBMV_CUDA(cudaEventRecord(c->ev[i], st));
-  CBMV_CUDA(cudaMemcpyAsync(w.volA, cost, sizeof(float) * H * W * D, cudaMemcpyDeviceToDevice, st));
-  RC(run_post(c, p, L, R, H, W, D, w, disp));
+  if (!in_place(cost)) {
+    CBMV_CUDA(cudaMemcpyAsync(w.volA, cost, sizeof(float) * H * W * D, cudaMemcpyDeviceToDevice, st));
+    cost = w.volA;
+  }
+  RC(run_post(c, p, L, R, H, W, D, w, cost, disp));
   CBMV_CUDA(cudaEventRecord(c->ev[4], st));
   return CBMV_OK;
 }
