@@ -364,6 +364,86 @@ __global__ void stats_f32_left_kernel(VolsF vols, int64_t HW, int D, float2* __r
   }
 }
 
+// view 0 for rows that a warp holds in registers: K vectors of V costs per
+// lane, PX pixels at a time, so that their loads are in flight together; the
+// minimum is a `redux`, and the sums of PX pixels are exchanged in one tree
+// whose additions are those of stats_f32_left_kernel.  Bound by memory:
+// 451x319 D=70 74 us (142 with one pixel per warp, its row read twice),
+// 1482x994 D=256 1043 (1464).
+template <int V, int K>
+__global__ void __launch_bounds__(256) stats_f32_left_r_kernel(VolsF vols, int64_t HW, int D,
+                                                               float2* __restrict__ statsf) {
+  constexpr int PX = V * K <= 4 ? 4 : V * K <= 8 ? 2 : 1;
+  const int m = blockIdx.y;
+  const float* __restrict__ vol = vols.v[m];
+  const float inv_sigma = kInvSigmaF32[m];
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t p0 = PX * (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); p0 < HW; p0 += PX * nw) {
+    float v[PX][K][V], mn[PX], den[PX];
+#pragma unroll
+    for (int i = 0; i < PX; i++) {
+      const float* r = vol + (p0 + i < HW ? p0 + i : p0) * D;
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const int d = V * (lane + 32 * k);
+        if constexpr (V == 4) {
+          const float4 q = d < D ? __ldg(reinterpret_cast<const float4*>(r + d))
+                                 : make_float4(kRandMaxF, kRandMaxF, kRandMaxF, kRandMaxF);
+          v[i][k][0] = q.x, v[i][k][1] = q.y, v[i][k][2] = q.z, v[i][k][3] = q.w;
+        } else {
+          v[i][k][0] = d < D ? __ldg(r + d) : kRandMaxF;
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < PX; i++) {
+      mn[i] = kRandMaxF;
+#pragma unroll
+      for (int k = 0; k < K; k++)
+#pragma unroll
+        for (int j = 0; j < V; j++) mn[i] = fminf(mn[i], v[i][k][j]);
+      asm volatile("redux.sync.min.f32 %0, %0, 0xffffffff;" : "+f"(mn[i]));
+      den[i] = 0.0f;
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        if (V * (lane + 32 * k) < D) {
+          float e[V];
+#pragma unroll
+          for (int j = 0; j < V; j++) {
+            const float t = v[i][k][j] - mn[i];
+            e[j] = __expf(-(t * t) * inv_sigma);
+          }
+          if constexpr (V == 4) den[i] += (e[0] + e[1]) + (e[2] + e[3]);
+          else den[i] += e[0];
+        }
+      }
+    }
+    // lane l keeps the sum and minimum of pixel `mine`
+    float sum = den[0], low = mn[0];
+    int mine = 0, o = 16;
+    if constexpr (PX == 4) {
+      const bool up = lane & 16;
+      const float a = (up ? den[2] : den[0]) + __shfl_xor_sync(0xffffffffu, up ? den[0] : den[2], 16);
+      const float b = (up ? den[3] : den[1]) + __shfl_xor_sync(0xffffffffu, up ? den[1] : den[3], 16);
+      const bool odd = lane & 8;
+      sum = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+      mine = (up ? 2 : 0) + (odd ? 1 : 0);
+      low = up ? (odd ? mn[3] : mn[2]) : (odd ? mn[1] : mn[0]);
+      o = 4;
+    } else if constexpr (PX == 2) {
+      const bool up = lane & 16;
+      sum = (up ? den[1] : den[0]) + __shfl_xor_sync(0xffffffffu, up ? den[0] : den[1], 16);
+      mine = up ? 1 : 0;
+      low = up ? mn[1] : mn[0];
+      o = 8;
+    }
+    constexpr int kLanes = 32 / PX;
+    for (; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane % kLanes == 0 && p0 + mine < HW) statsf[(int64_t)(m * 2) * HW + p0 + mine] = stats_pair(m, low, sum);
+  }
+}
+
 // view 1: right pixel x' of row y sees C[y, x' + d, d] (the fill C[0,0,0]
 // where x' + d >= W, featextract.cpp:115-152).  A CTA owns RS_PIX right
 // pixels of one row; for each 32-wide disparity chunk it stages the
@@ -387,14 +467,11 @@ __global__ void __launch_bounds__(RS_PIX) stats_f32_right_kernel(VolsF vols, int
   for (int pass = 0; pass < 2; pass++) {
     for (int d0 = 0; d0 < D; d0 += 32) {
       __syncthreads();
-      for (int q = tid; q < (RS_PIX + 32) * 32; q += RS_PIX) {
-        const int i = q >> 5, j = q & 31;
-        const int64_t x = X0 + d0 + i;
-        const int d = d0 + j;
-        float v = fill;
-        if (x < W && d < D) v = __ldg(vol + (y * W + x) * D + d);
-        tile[i * 33 + j] = v;
-      }
+      const int j = tid & 31, last = d0 + j < D ? (int)min(W - X0 - d0, (int64_t)RS_PIX + 32) : 0;
+      const float* src = vol + (y * W + X0 + d0 + (tid >> 5)) * D + d0 + j;
+#pragma unroll 9
+      for (int i = tid >> 5; i < RS_PIX + 32; i += RS_PIX / 32, src += (RS_PIX / 32) * (int64_t)D)
+        tile[i * 33 + j] = i < last ? __ldg(src) : fill;
       __syncthreads();
       if (xr < W) {
         const int nj = D - d0 < 32 ? D - d0 : 32;
@@ -540,6 +617,12 @@ __global__ void __launch_bounds__(RS_PIX) stats_f32_right_q_kernel(VolsF vols, i
   if (xr < Wi) statsf[(int64_t)(m * 2 + 1) * H * W + y * W + xr] = stats_pair(m, mn, den);
 }
 
+template <int V, int K>
+static void launch_stats_left_r(const VolsF& v, int64_t HW, int D, float2* statsf, cudaStream_t st) {
+  const int64_t blocks = (HW + 15) / 16;  // 8 warps per block, two pixels each (a warp of fewer or more strides)
+  stats_f32_left_r_kernel<V, K><<<dim3((unsigned)(blocks < 65535 * 16 ? blocks : 65535 * 16), 4), 256, 0, st>>>(v, HW, D, statsf);
+}
+
 int launch_feature_stats_f32(const float* const* vols, int64_t H, int64_t W, int D, float2* statsf,
                              cudaStream_t st) {
   const VolsF v = {{vols[0], vols[1], vols[2], vols[3]}};
@@ -554,6 +637,16 @@ int launch_feature_stats_f32(const float* const* vols, int64_t H, int64_t W, int
     const int64_t qblocks = (HW + 15) / 16;  // 8 warps per block, two pixels each
     stats_f32_left_q_kernel<<<dim3((unsigned)(qblocks < 65535 * 16 ? qblocks : 65535 * 16), 4), 256, 0, st>>>(
         v, HW, D, statsf);
+  } else if (q && D <= 512) {
+    if (D <= 256) launch_stats_left_r<4, 2>(v, HW, D, statsf, st);
+    else if (D <= 384) launch_stats_left_r<4, 3>(v, HW, D, statsf, st);
+    else launch_stats_left_r<4, 4>(v, HW, D, statsf, st);
+  } else if (D % 4 != 0 && D <= 256) {
+#define LEFT_R(K) case K: launch_stats_left_r<1, K>(v, HW, D, statsf, st); break;
+    switch ((D + 31) / 32) {
+      LEFT_R(1) LEFT_R(2) LEFT_R(3) LEFT_R(4) LEFT_R(5) LEFT_R(6) LEFT_R(7) LEFT_R(8)
+    }
+#undef LEFT_R
   } else {
     stats_f32_left_kernel<<<dim3((unsigned)(lblocks < 65535 * 16 ? lblocks : 65535 * 16), 4), 256, 0, st>>>(
         v, HW, D, statsf);
