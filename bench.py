@@ -382,8 +382,8 @@ def run_cbmv(a, ws, rank, local):
         rf_achieved = visits * units / t_rf
         sm_count = torch.cuda.get_device_properties(dev).multi_processor_count
         mhz = clk_max_mhz()
-        # L1 sector bound of the walk: each lane's next 32-byte node block (two tree
-        # levels) is a different sector; an SM's L1 returns 4 sectors (128 B) per clock
+        # L1 sector bound of the walk: each lane's next 16-byte entry (two tree
+        # levels) is in a different sector; an SM's L1 returns 4 sectors (128 B) per clock
         rf_peak = sm_count * 4 * 2 * mhz * 1e6
         res["rf"]["roofline"] = {
             "bound": "l1", "kernel": "features_rf_tiled", "achieved": rf_achieved, "peak": rf_peak,
@@ -391,8 +391,8 @@ def run_cbmv(a, ws, rank, local):
             "traffic": traffic.get("features_rf_kernel"), "peak_kind": "derived (L1 sectors/clock)",
             "visits_per_unit": visits,
             "note": "node visits = comparisons per (pixel,d) summed over the 50 trees (mean over 65,536 "
-                    "sampled (p,d) of this pair); peak = SMs x 4 sectors/clock x 2 levels per 32-byte "
-                    "block x max SM clock; HBM: %.0f GB/s of %.0f for 4 B/(p,d)"
+                    "sampled (p,d) of this pair); peak = SMs x 4 sectors/clock x 2 levels per 16-byte "
+                    "entry x max SM clock; HBM: %.0f GB/s of %.0f for 4 B/(p,d)"
                     % (BYTES_PER_UNIT_FUSED * units / t_rf / 1e9, hbm)}
     if "mlp" in res:
         mlp_tflops = FLOPS_PER_UNIT_MLP * units / (res["mlp"]["stage_ms"]["classify"] / 1e3) / 1e12

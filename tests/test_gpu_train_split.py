@@ -61,3 +61,21 @@ def test_split_equals_the_mean_of_single_tiles(gpu, tiles):
         a, b = g[o:o + s], want[o:o + s]
         assert np.abs(a - b).max() <= 3e-4 * np.abs(b).max(), (o, s)
         o += s
+
+
+@pytest.mark.parametrize("tiles", [2, 64])
+def test_gradients_under_capture(gpu, tiles):
+    """Both launches (the second set up beside the first) in a CUDA graph."""
+    from cbmv_b200.mlp import MlpTrainer
+    net, X, y = _net_and_batch("gelu", tiles)
+    tr = MlpTrainer(net, batch=len(X))
+    Xt, yt = torch.from_numpy(X).cuda(), torch.from_numpy(y).cuda()
+    want = tr.gradients(Xt, yt)[0].clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got, _ = tr.gradients(Xt, yt)
+    for _ in range(2):
+        got.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
