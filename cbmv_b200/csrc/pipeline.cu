@@ -416,7 +416,7 @@ static int run_post(cbmv_ctx* c, const cbmv_params* p, const uint8_t* L, const u
 // and of the training samples); f32 = true: float32 volumes (in the first
 // half of each float64 buffer) and float32 statistics only, for the network.
 static int run_front(cbmv_ctx* c, const cbmv_params* p, const uint8_t* L, const uint8_t* R,
-                     int64_t H, int64_t W, int D, Work* wout, bool f32 = false, bool prep = false) {
+                     int64_t H, int64_t W, int D, Work* wout, bool f32 = false, bool prep = false, bool stats = true) {
   RC(check_params(p));
   CBMV_REQUIRE(H > p->censw && W > p->censw, CBMV_EINVAL, "image %lldx%lld smaller than the census window",
                (long long)W, (long long)H);
@@ -471,7 +471,7 @@ static int run_front(cbmv_ctx* c, const cbmv_params* p, const uint8_t* L, const 
   RC(launch_zsad_cost<double>(L, R, w.muL, w.muR, H, W, D, p->sadw, CBMV_HWD, w.vol[3], st));
   CBMV_CUDA(cudaEventRecord(c->ev[1], st));
   const double* vols[4] = {w.vol[0], w.vol[1], w.vol[2], w.vol[3]};
-  RC(launch_feature_stats(vols, H, W, D, w.stats, st));
+  if (stats) RC(launch_feature_stats(vols, H, W, D, w.stats, st));
   CBMV_CUDA(cudaEventRecord(c->ev[2], st));
   *wout = w;
   return CBMV_OK;
@@ -619,9 +619,10 @@ extern "C" int cbmv_ctx_features_at(cbmv_ctx* c, const cbmv_params* p, const uin
   cbmv_params def;
   p = params_or_default(p, &def);
   Work w;
-  RC(run_front(c, p, L, R, H, W, D, &w));
+  const bool rows = features_gather_rows(H, W, n);
+  RC(run_front(c, p, L, R, H, W, D, &w, false, false, !rows));
   const double* vols[4] = {w.vol[0], w.vol[1], w.vol[2], w.vol[3]};
-  return launch_features_gather(vols, w.stats, H, W, D, idx, n, out, c->stream);
+  return launch_features_gather(vols, rows ? nullptr : w.stats, H, W, D, idx, n, out, c->stream);
 }
 
 extern "C" int cbmv_ctx_features_f32_at(cbmv_ctx* c, const cbmv_params* p, const uint8_t* L,

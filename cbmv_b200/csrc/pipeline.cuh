@@ -55,6 +55,9 @@ int launch_features_mlp(const float* const* vols, const float2* statsf, int64_t 
 int launch_features_f32_gather(const float* const* vols, const float2* statsf, int64_t H, int64_t W, int D,
                                const int64_t* idx, int64_t n, float* out, cudaStream_t st);
 // The 20 features (float32) of the samples idx[i] = (y*W + x)*D + d.
+// n samples' features from the whole image's statistics, or (stats null) from
+// those of their own rows; the second where features_gather_rows says so
+bool features_gather_rows(int64_t H, int64_t W, int64_t n);
 int launch_features_gather(const double* const* vols, const double* stats, int64_t H, int64_t W,
                            int D, const int64_t* idx, int64_t n, float* out, cudaStream_t st);
 int launch_features_rf(const double* const* vols, const double* stats, int64_t H, int64_t W,
