@@ -5,6 +5,7 @@
 // divided by the tree count, as predict_proba does with one job.
 #include <string.h>
 
+#include <unordered_map>
 #include <vector>
 
 #include "common.cuh"
@@ -58,31 +59,57 @@ __global__ void __launch_bounds__(kBlock, kPerSm)
 
 // The device layout of rf.cuh from validated two-level blocks: one segment
 // per tree, breadth-first; a group that its segment can no longer number
-// starts a segment of its own, reached by a jump.
-static void rf_entries(const uint32_t* blocks, const double* leaf_value, const int32_t* tree_offsets, int n_trees,
-                       uint32_t max_group, std::vector<uint32_t>* entries, std::vector<uint32_t>* roots) {
+// starts a segment of its own, reached by a jump, and so does a block that
+// several slots name as their child (laid out once, however many reach it).
+// Every block begins at most one segment and forms at most one group, so
+// there are at most 8 entries per block.
+static void rf_entries(const uint32_t* blocks, int64_t n_blocks, const double* leaf_value, const int32_t* tree_offsets,
+                       int n_trees, uint32_t max_group, std::vector<uint32_t>* entries, std::vector<uint32_t>* roots) {
   std::vector<uint32_t>& E = *entries;
+  // the child block or leaf (kLeafFlag) in slot j of a block's child n
+  auto child_of = [](const uint32_t* w, int n, int j) {
+    return ((w[3] >> (8 * n)) & 0xFFu) == kLeafFeature ? w[2 + 2 * n] | kLeafFlag : w[2 + 2 * n + j];
+  };
   auto leaf = [&](uint32_t at, uint32_t id) {
     memcpy(&E[4 * (size_t)at], &leaf_value[2 * (size_t)id], sizeof(double));
     E[4 * (size_t)at + 2] = id;
     E[4 * (size_t)at + 3] = kRfLeaf;
   };
+  constexpr uint32_t kNone = 0xFFFFFFFFu;
+  std::vector<uint8_t> named(n_blocks, 0);  // slots that name the block, at most 2
+  for (int64_t k = 0; k < n_blocks; k++) {
+    const uint32_t* w = blocks + 8 * (size_t)k;
+    if ((w[3] & 0xFFu) == kLeafFeature) continue;
+    for (int s = 0; s < 4; s++) {
+      const uint32_t c = child_of(w, 1 + s / 2, s % 2);
+      if (!(c & kLeafFlag) && named[c] < 2) named[c]++;
+    }
+  }
+  std::unordered_map<uint32_t, uint32_t> shared;  // a block named twice -> its segment
   struct Item {
     uint32_t block, at;
   };
   for (int t = 0; t < n_trees; t++) {
-    std::vector<Item> starts = {{(uint32_t)tree_offsets[t], 0u}};  // block, the jump leading to it
+    std::vector<Item> starts = {{(uint32_t)tree_offsets[t], kNone}};  // block, the jump leading to it
     for (size_t i = 0; i < starts.size(); i++) {
-      const uint32_t seg = (uint32_t)(E.size() / 4);
-      E.resize(E.size() + 16, 0u);
-      if (i == 0) {
+      const Item start = starts[i];
+      uint32_t seg = (uint32_t)(E.size() / 4);
+      bool laid = false;
+      if (named[start.block] > 1) {
+        const auto put = shared.emplace(start.block, seg);
+        laid = !put.second;
+        seg = put.first->second;
+      }
+      if (start.at == kNone) {
         roots->push_back(seg);
       } else {
-        E[4 * (size_t)starts[i].at] = seg;
-        E[4 * (size_t)starts[i].at + 3] = kRfJump;
+        E[4 * (size_t)start.at] = seg;
+        E[4 * (size_t)start.at + 3] = kRfJump;
       }
+      if (laid) continue;
+      E.resize(E.size() + 16, 0u);
       uint32_t group = 1;
-      std::vector<Item> queue = {{starts[i].block, seg}};
+      std::vector<Item> queue = {{start.block, seg}};
       for (size_t q = 0; q < queue.size(); q++) {
         const uint32_t at = queue[q].at;
         const uint32_t* w = blocks + 8 * (size_t)queue[q].block;
@@ -100,13 +127,11 @@ static void rf_entries(const uint32_t* blocks, const double* leaf_value, const i
         uint32_t* e = &E[4 * (size_t)at];
         for (int n = 0; n < 3; n++) e[n] = f[n] == kLeafFeature ? 0u : w[n];
         e[3] = group++ | f[0] << 17 | (f[1] == kLeafFeature ? 0u : f[1]) << 22 | (f[2] == kLeafFeature ? 0u : f[2]) << 27;
-        for (int n = 1; n <= 2; n++)
-          for (int j = 0; j < 2; j++) {
-            const uint32_t c = f[n] == kLeafFeature ? w[2 + 2 * n] | kLeafFlag : w[2 + 2 * n + j];
-            const uint32_t to = child + 2 * (n - 1) + j;
-            if (c & kLeafFlag) leaf(to, c & ~kLeafFlag);
-            else queue.push_back({c, to});
-          }
+        for (int s = 0; s < 4; s++) {
+          const uint32_t c = child_of(w, 1 + s / 2, s % 2), to = child + s;
+          if (c & kLeafFlag) leaf(to, c & ~kLeafFlag);
+          else (named[c] > 1 ? starts : queue).push_back({c, to});
+        }
       }
     }
   }
@@ -171,7 +196,7 @@ extern "C" int cbmv_forest_create(const uint32_t* blocks, int64_t n_blocks, cons
   }
   std::vector<uint32_t> entries, roots;
   entries.reserve(16 * (size_t)(n_blocks + n_trees));
-  rf_entries(blocks, leaf_value, tree_offsets, n_trees, kRfMaxGroup, &entries, &roots);
+  rf_entries(blocks, n_blocks, leaf_value, tree_offsets, n_trees, kRfMaxGroup, &entries, &roots);
   std::vector<double> p1((size_t)n_leaves);
   for (int64_t i = 0; i < n_leaves; i++) p1[i] = leaf_value[2 * i + 1];
   cbmv_forest* f = new cbmv_forest();

@@ -17,7 +17,8 @@
 // Four sibling entries form a 64-byte group, numbered from their segment's
 // first entry; a child that is itself a leaf fills both of its slots.  A
 // tree is one segment, its root the first entry; where it has more groups
-// than 17 bits count, a jump leads to a subtree in a segment of its own.
+// than 17 bits count, a jump leads to a subtree in a segment of its own, and
+// so it does to a block that several slots name as their child.
 //
 // A walk step is one 16-byte load and descends two levels, and the leaf's
 // value is in the entry that ends the walk.  (The 32-byte blocks took two
