@@ -5,6 +5,7 @@
 // divided by the tree count, as predict_proba does with one job.
 #include <string.h>
 
+#include <new>
 #include <unordered_map>
 #include <vector>
 
@@ -195,11 +196,17 @@ extern "C" int cbmv_forest_create(const uint32_t* blocks, int64_t n_blocks, cons
     }
   }
   std::vector<uint32_t> entries, roots;
-  entries.reserve(16 * (size_t)(n_blocks + n_trees));
-  rf_entries(blocks, n_blocks, leaf_value, tree_offsets, n_trees, kRfMaxGroup, &entries, &roots);
-  std::vector<double> p1((size_t)n_leaves);
+  std::vector<double> p1;
+  cbmv_forest* f = nullptr;
+  try {
+    entries.reserve(16 * (size_t)(n_blocks + n_trees));
+    rf_entries(blocks, n_blocks, leaf_value, tree_offsets, n_trees, kRfMaxGroup, &entries, &roots);
+    p1.resize((size_t)n_leaves);
+    f = new cbmv_forest();
+  } catch (const std::bad_alloc&) {
+    return set_error(CBMV_ENOMEM, "forest layout: out of host memory");
+  }
   for (int64_t i = 0; i < n_leaves; i++) p1[i] = leaf_value[2 * i + 1];
-  cbmv_forest* f = new cbmv_forest();
   auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t eb = up(entries.size() * 4), lb = up((size_t)n_leaves * sizeof(double)), rb = roots.size() * 4;
   cudaError_t e = cudaMalloc(&f->mem, eb + lb + rb);

@@ -47,7 +47,7 @@ enum cbmv_status {
   CBMV_OK = 0,
   CBMV_EINVAL = -1,  /* bad argument (null pointer, size, window, dtype ...) */
   CBMV_ECUDA = -2,   /* a CUDA runtime call failed                          */
-  CBMV_ENOMEM = -3,  /* device allocation failed                            */
+  CBMV_ENOMEM = -3,  /* device (or a forest's host) allocation failed       */
   CBMV_ERANGE = -4,  /* size beyond a documented limit                      */
   CBMV_ESTATE = -5   /* object used in the wrong state                       */
 };

@@ -73,6 +73,31 @@ def test_a_shared_block_is_laid_out_once():
     subprocess.run([sys.executable, "-c", CHILD % (ROOT, os.path.join(ROOT, "tests"))], check=True, timeout=120, env=env)
 
 
+NO_MEMORY = """
+import ctypes, resource, sys
+import numpy as np
+sys.path.insert(0, %r)
+from cbmv_b200 import _lib
+L = _lib.lib()
+n = 1 << 20
+k = np.arange(n, dtype=np.int64)
+blocks = np.zeros((n, 8), np.uint32)
+blocks[:, 4:8] = np.where(4 * k[:, None] + np.arange(1, 5) < n, 4 * k[:, None] + np.arange(1, 5), 0x80000000)
+leafv, offs, h = np.zeros((1, 2)), np.array([0, n], np.int32), ctypes.c_void_p()
+data = sum(int(f.split()[1]) << 10 for f in open("/proc/self/status") if f.startswith("VmData"))
+resource.setrlimit(resource.RLIMIT_DATA, (data + (16 << 20), data + (16 << 20)))
+rc = L.cbmv_forest_create(blocks.ctypes.data, n, leafv.ctypes.data, 1, offs.ctypes.data, 1, 20, ctypes.byref(h))
+assert rc == -3 and b"host memory" in L.cbmv_last_error(), (rc, L.cbmv_last_error())
+"""
+
+
+def test_exhausted_host_memory_is_an_error_code():
+    """A million blocks (64 MB of entries) with 16 MB left: CBMV_ENOMEM, no
+    C++ exception through the C boundary."""
+    env = dict(os.environ, CUDA_VISIBLE_DEVICES="")
+    subprocess.run([sys.executable, "-c", NO_MEMORY % ROOT], check=True, timeout=120, env=env)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("make", [lambda: _chain(12), lambda: _random_dag(40, 9, 1), lambda: _random_dag(700, 60, 2)])
 def test_walk_over_shared_blocks(gpu, make):
