@@ -761,15 +761,60 @@ __device__ __forceinline__ uint32_t arm_word(int l, int r, int u, int d) {
   return ((1u << (l + r + 1)) - 1u) << (kMaskHalo - l) | ((1u << (u + d + 1)) - 1u) << (11 + kMaskHalo - u);
 }
 
+// *odd (zeroed by the caller) is set where an arm is none that cross_kernel
+// gives: one that excludes its pixel, or is longer than a word's taps.
 __global__ void arm_words_kernel(const float* __restrict__ lc, const float* __restrict__ rc, int64_t H, int64_t W,
-                                 uint32_t* __restrict__ words) {
+                                 uint32_t* __restrict__ words, uint32_t* __restrict__ odd) {
   const int64_t n = H * W;
   const float* __restrict__ arms = blockIdx.y ? rc : lc;
   GRID_STRIDE(p, n) {
     const int y = (int)(p / W), x = (int)(p - y * W);
-    auto reach = [&](int v) { return min(max(v - 1, 0), kMaskHalo); };
+    bool ok = true;
+    auto reach = [&](int v) {
+      ok &= v >= 1 && v <= kMaskHalo + 1;
+      return min(max(v - 1, 0), kMaskHalo);
+    };
     words[blockIdx.y * n + p] = arm_word(reach(x - (int)arms[p]), reach((int)arms[n + p] - x),
                                          reach(y - (int)arms[2 * n + p]), reach((int)arms[3 * n + p] - y));
+    if (!ok) *odd = 1u;
+  }
+}
+
+// The support words of any arms, one thread per word, where *odd says that
+// the arm words do not hold them: the taps of a support within five pixels
+// and inside the image, and the pixels of its rows at their whole length.
+__global__ void cbca_mask_any_kernel(const float* __restrict__ lc, const float* __restrict__ rc, int64_t H, int64_t W,
+                                     int D, int direction, const uint32_t* __restrict__ odd, uint32_t* __restrict__ mask) {
+  if (*odd == 0u) return;
+  const int64_t n = H * W;
+  GRID_STRIDE(id, n * D) {
+    const int64_t p = id / D, y = p / W, x = p - y * W;
+    const int64_t xm = x + (id - p * D) * direction;
+    if (xm < 0 || xm >= W) {
+      mask[id] = kMaskCopy;
+      continue;
+    }
+    // taps lo..hi that arms a and a + 1 of row yy allow
+    auto taps = [&](int a, int64_t yy, int* lo, int* hi) {
+      const int64_t l = a * n + yy * W + x, r = a * n + yy * W + xm;
+      const int ol = (int)(a < 2 ? x : yy), orr = (int)(a < 2 ? xm : yy);
+      *lo = max(clamp_i8((int)lc[l] - ol), clamp_i8((int)rc[r] - orr)) + 1;
+      *hi = min(clamp_i8((int)lc[l + n] - ol), clamp_i8((int)rc[r + n] - orr)) - 1;
+    };
+    int lo, hi;
+    uint32_t w = 0, cnt = 0;
+    taps(0, y, &lo, &hi);
+    for (int k = max(lo, -kMaskHalo); k <= min(hi, kMaskHalo); k++)
+      if (x + k >= 0 && x + k < W) w |= 1u << (k + kMaskHalo);
+    taps(2, y, &lo, &hi);
+    for (int k = max(lo, -kMaskHalo); k <= min(hi, kMaskHalo); k++)
+      if (y + k >= 0 && y + k < H) {
+        w |= 1u << (11 + k + kMaskHalo);
+        int from, to;
+        taps(0, y + k, &from, &to);
+        cnt += (uint32_t)max(to - from + 1, 0);
+      }
+    mask[id] = w | (cnt & 0x7Fu) << 22;
   }
 }
 
@@ -1643,11 +1688,16 @@ extern "C" int cbmv_cbca_separable(const float* crossL, const float* crossR, con
   if (L1 - 1 > kCbcaMaskMaxHalo) return launch_cbca_sep(crossL, crossR, in, H, W, D, direction, out, st, L1 - 1);
   // the pipeline's form: supports precomputed into a stream-ordered scratch buffer
   uint32_t* mask = nullptr;
-  CBMV_CUDA(cudaMallocAsync(&mask, sizeof(uint32_t) * H * W * (D + 2), st));
-  uint32_t* words = mask + H * W * D;
-  arm_words_kernel<<<dim3(grid_for(H * W, kBlock), 2), kBlock, 0, st>>>(crossL, crossR, H, W, words);
+  CBMV_CUDA(cudaMallocAsync(&mask, sizeof(uint32_t) * (H * W * (D + 2) + 1), st));
+  uint32_t *words = mask + H * W * D, *odd = words + 2 * H * W;
+  cudaMemsetAsync(odd, 0, sizeof(uint32_t), st);
+  arm_words_kernel<<<dim3(grid_for(H * W, kBlock), 2), kBlock, 0, st>>>(crossL, crossR, H, W, words, odd);
   int rc = check_launch("arm_words");
   if (rc == CBMV_OK) rc = launch_cbca_mask_build(words, words + H * W, H, W, D, direction, mask, st);
+  if (rc == CBMV_OK) {
+    cbca_mask_any_kernel<<<grid_for(H * W * D, kBlock), kBlock, 0, st>>>(crossL, crossR, H, W, D, direction, odd, mask);
+    rc = check_launch("cbca_mask_any");
+  }
   if (rc == CBMV_OK) rc = launch_cbca_masked(mask, in, H, W, D, out, st);
   CBMV_CUDA(cudaFreeAsync(mask, st));
   return rc;
