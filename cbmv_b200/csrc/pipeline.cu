@@ -16,6 +16,7 @@
 // The reference's per-row batching of the classifier (test.py:608-623) only
 // bounds its host memory; every feature is row-local, so one launch covers
 // the whole image with identical results.
+#include <cuda.h>
 #include <math.h>
 #include <string.h>
 
@@ -275,8 +276,45 @@ static int ensure_gaussian(cbmv_ctx* c, float sigma) {
 // Whether a caller's cost volume is used where it lies: the classifier writes
 // it and the chain's first pass reads it there (a copy of a 694x554 D=128
 // volume takes 64 us).  One that is not 16-byte aligned is copied, so that
-// the passes keep their vector accesses.
-static bool in_place(const float* volume) { return volume && (uintptr_t)volume % 16 == 0; }
+// the passes keep their vector accesses; so is one that is not wholly device
+// memory of this GPU as far as the driver knows, because a copy turns a bad
+// pointer or size into an error and a kernel would fault on it.
+static bool in_place(const float* volume, int64_t elements) {
+  typedef CUresult (*Range)(CUdeviceptr*, size_t*, CUdeviceptr);
+  static const Range address_range = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    cudaGetLastError();
+    return reinterpret_cast<Range>(f);
+  }();
+  if (!volume || (uintptr_t)volume % 16 != 0 || !address_range) return false;
+  cudaPointerAttributes at;
+  int dev = 0;
+  if (cudaPointerGetAttributes(&at, volume) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  return at.type == cudaMemoryTypeDevice && at.device == dev &&
+         address_range(&base, &size, (CUdeviceptr)volume) == CUDA_SUCCESS &&
+         (CUdeviceptr)volume + elements * sizeof(float) <= base + size;
+}
+
+// A volume in pageable host memory, where the device cannot read that, is
+// refused before any work is launched.
+static int check_volume(const float* volume) {
+  cudaPointerAttributes at;
+  int dev = 0, pageable = 0;
+  CBMV_CUDA(cudaGetDevice(&dev));
+  CBMV_CUDA(cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, dev));
+  CBMV_CUDA(cudaPointerGetAttributes(&at, volume));
+  CBMV_REQUIRE(pageable || at.type != cudaMemoryTypeUnregistered, CBMV_EINVAL, "the cost volume is pageable host memory");
+  return CBMV_OK;
+}
 
 // The cost-optimisation chain of Testing.__postprocessing_mem
 // (test.py:355-405) on one float32 [H,W,D] cost volume held in `cur`:
@@ -490,11 +528,12 @@ extern "C" int cbmv_run_rf(cbmv_ctx* c, const cbmv_forest* f, const cbmv_params*
   cbmv_params def;
   p = params_or_default(p, &def);
   CBMV_REQUIRE(forest_view(f)->n_features == 20, CBMV_EINVAL, "the forest must take the 20 CBMV features");
+  if (prob0) RC(check_volume(prob0));
   Work w;
   RC(run_front(c, p, L, R, H, W, D, &w, false, true));
   cudaStream_t st = c->stream;
   const double* vols[4] = {w.vol[0], w.vol[1], w.vol[2], w.vol[3]};
-  float* cost = in_place(prob0) ? prob0 : w.volA;
+  float* cost = in_place(prob0, H * W * D) ? prob0 : w.volA;
   RC(launch_features_rf(vols, w.stats, H, W, D, f, cost, st));
   if (prob0 && cost != prob0)
     CBMV_CUDA(cudaMemcpyAsync(prob0, cost, sizeof(float) * H * W * D, cudaMemcpyDeviceToDevice, st));
@@ -509,11 +548,12 @@ extern "C" int cbmv_run_mlp(cbmv_ctx* c, const cbmv_mlp* m, const cbmv_params* p
   CBMV_REQUIRE(c && m && L && R && disp, CBMV_EINVAL, "null pointer argument");
   cbmv_params def;
   p = params_or_default(p, &def);
+  if (prob0) RC(check_volume(prob0));
   Work w;
   RC(run_front(c, p, L, R, H, W, D, &w, true, true));
   cudaStream_t st = c->stream;
   const float* vols[4] = {(float*)w.vol[0], (float*)w.vol[1], (float*)w.vol[2], (float*)w.vol[3]};
-  float* cost = in_place(prob0) ? prob0 : w.volA;
+  float* cost = in_place(prob0, H * W * D) ? prob0 : w.volA;
   RC(launch_features_mlp(vols, w.statsf, H, W, D, m, cost, st, p->mlp_ctas));
   if (prob0 && cost != prob0)
     CBMV_CUDA(cudaMemcpyAsync(prob0, cost, sizeof(float) * H * W * D, cudaMemcpyDeviceToDevice, st));
@@ -583,13 +623,14 @@ extern "C" int cbmv_run_post(cbmv_ctx* c, const cbmv_params* p, const uint8_t* L
   CBMV_REQUIRE(H > p->censw && W > p->censw, CBMV_EINVAL, "image %lldx%lld smaller than the census window",
                (long long)W, (long long)H);
   CBMV_REQUIRE(H <= 65535 && D >= 1 && D <= 1024, CBMV_ERANGE, "H must be <= 65535 and D in 1..1024");
+  RC(check_volume(cost));
   size_t bytes = 0;
   carve(nullptr, H, W, D, &bytes, true, p->interpolate != 0);
   RC(ensure_workspace(c, bytes));
   Work w = carve(c->ws, H, W, D, &bytes, true, p->interpolate != 0);
   cudaStream_t st = c->stream;
   for (int i = 0; i < 4; i++) CBMV_CUDA(cudaEventRecord(c->ev[i], st));
-  if (!in_place(cost)) {
+  if (!in_place(cost, H * W * D)) {
     CBMV_CUDA(cudaMemcpyAsync(w.volA, cost, sizeof(float) * H * W * D, cudaMemcpyDeviceToDevice, st));
     cost = w.volA;
   }
