@@ -36,6 +36,27 @@ def to_device(a, dtype):
     return t.to("cuda", non_blocking=False).contiguous(), True
 
 
+def lend(stream, pairs):
+    """Device copies made on torch's current stream for a call on `stream` (a
+    cudaStream_t): that stream waits for them to be made, and the allocator
+    keeps their memory until it has passed the call.  `pairs` holds (what the
+    caller gave, its device tensor); a tensor of the caller's own is left to
+    the caller, as its life is."""
+    cur = torch.cuda.current_stream()
+    if (stream or 0) == cur.cuda_stream:
+        return
+    made = [t for a, t in pairs if not (is_device(a) and a.data_ptr() == t.data_ptr())]
+    if made:
+        on = stream_object(stream)
+        on.wait_stream(cur)
+        for t in made:
+            t.record_stream(on)
+
+
+def stream_object(stream):
+    return torch.cuda.ExternalStream(stream) if stream else torch.cuda.default_stream()
+
+
 def is_host(a):
     """True for numpy arrays and CPU tensors (pinned or not)."""
     return isinstance(a, np.ndarray) or (isinstance(a, torch.Tensor) and not a.is_cuda)
@@ -70,8 +91,12 @@ def zeros(shape, dtype):
     return torch.zeros(tuple(int(s) for s in shape), dtype=_NP2T[np.dtype(dtype)], device="cuda")
 
 
-def result(t, host):
-    """Returns `t` as numpy when the call's input came from the host."""
+def result(t, host, stream=None):
+    """Returns `t`, written on `stream` (None: torch's current one), as numpy
+    when the call's input came from the host."""
     if host:
+        cur = torch.cuda.current_stream()
+        if stream is not None and stream != cur.cuda_stream:
+            cur.wait_stream(stream_object(stream))
         return t.cpu().numpy()
     return t

@@ -22,8 +22,8 @@ class StereoPipeline:
         self.forest = forest
         self.params = params if params is not None else _lib.default_params()
         h = ctypes.c_void_p()
-        self._stream = stream
-        _lib.call("cbmv_ctx_create", stream if stream is not None else _dev.stream_ptr(), ctypes.byref(h))
+        self._stream = stream if stream is not None else _dev.stream_ptr()
+        _lib.call("cbmv_ctx_create", self._stream, ctypes.byref(h))
         self.ctx = h
 
     def close(self):
@@ -62,12 +62,13 @@ class StereoPipeline:
             return self._run_host("cbmv_run_rf_host", self.forest.handle, left, right, ndisp, disp_out)
         l, host = _dev.to_device(left, np.uint8)
         r, _ = _dev.to_device(right, np.uint8)
+        _dev.lend(self._stream, [(left, l), (right, r)])
         H, W = l.shape
         disp = disp_out if disp_out is not None else _dev.empty((H, W), np.float32)
         _lib.call("cbmv_run_rf", self.ctx, self.forest.handle, ctypes.byref(self.params), l.data_ptr(),
                   r.data_ptr(), H, W, int(ndisp), disp.data_ptr(),
                   prob_out.data_ptr() if prob_out is not None else None)
-        return _dev.result(disp, host)
+        return _dev.result(disp, host, self._stream)
 
     def run_mlp(self, net, left, right, ndisp, disp_out=None, prob_out=None):
         """The same path with the learned classifier (cbmv_b200.mlp.GpuMlp)."""
@@ -75,12 +76,13 @@ class StereoPipeline:
             return self._run_host("cbmv_run_mlp_host", net.h, left, right, ndisp, disp_out)
         l, host = _dev.to_device(left, np.uint8)
         r, _ = _dev.to_device(right, np.uint8)
+        _dev.lend(self._stream, [(left, l), (right, r)])
         H, W = l.shape
         disp = disp_out if disp_out is not None else _dev.empty((H, W), np.float32)
         _lib.call("cbmv_run_mlp", self.ctx, net.h, ctypes.byref(self.params), l.data_ptr(), r.data_ptr(),
                   H, W, int(ndisp), disp.data_ptr(),
                   prob_out.data_ptr() if prob_out is not None else None)
-        return _dev.result(disp, host)
+        return _dev.result(disp, host, self._stream)
 
     def run_classified(self, left, right, ndisp, net=None, disp_out=None, prob_out=None):
         """The learned classifier with the random forest as its fallback:
@@ -105,13 +107,14 @@ class StereoPipeline:
         l, host = _dev.to_device(left, np.uint8)
         r, _ = _dev.to_device(right, np.uint8)
         c, _ = _dev.to_device(cost, np.float32)
+        _dev.lend(self._stream, [(left, l), (right, r), (cost, c)])
         H, W = l.shape
         if c.dim() != 3 or tuple(c.shape[:2]) != (H, W):
             raise ValueError("cost must be [H,W,D] for images of %dx%d" % (W, H))
         disp = disp_out if disp_out is not None else _dev.empty((H, W), np.float32)
         _lib.call("cbmv_run_post", self.ctx, ctypes.byref(self.params), l.data_ptr(), r.data_ptr(), H, W,
-                  int(c.shape[2]), c.contiguous().data_ptr(), disp.data_ptr())
-        return _dev.result(disp, host)
+                  int(c.shape[2]), c.data_ptr(), disp.data_ptr())
+        return _dev.result(disp, host, self._stream)
 
     def volumes_f32(self, left, right, ndisp):
         """The learned path's four float32 matcher volumes (census, NCC,
@@ -119,6 +122,7 @@ class StereoPipeline:
         import torch
         l, _ = _dev.to_device(left, np.uint8)
         r, _ = _dev.to_device(right, np.uint8)
+        _dev.lend(self._stream, [(left, l), (right, r)])
         H, W = l.shape
         out = torch.empty((4, H, W, int(ndisp)), dtype=torch.float32, device="cuda")
         _lib.call("cbmv_ctx_volumes_f32", self.ctx, ctypes.byref(self.params), l.data_ptr(), r.data_ptr(),
@@ -135,6 +139,7 @@ class StereoPipeline:
         r, _ = _dev.to_device(right, np.uint8)
         H, W = l.shape
         ix, _ = _dev.to_device(idx, np.int64)
+        _dev.lend(self._stream, [(left, l), (right, r), (idx, ix)])
         if ix.numel() and (int(ix.min()) < 0 or int(ix.max()) >= H * W * int(ndisp)):
             raise ValueError("sample index outside the H*W*D volume")
         out = torch.empty((ix.numel(), 20), dtype=torch.float32, device="cuda")

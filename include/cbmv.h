@@ -381,7 +381,9 @@ int cbmv_ctx_destroy(cbmv_ctx* c);
  * interpolate=False): matchers -> features -> random forest -> P(class 0)
  * -> post (_mem chain, test.py:341-449) -> disparity.  L, R uint8 [H,W],
  * disp float32 [H,W], all device memory.  prob0 (optional, may be NULL)
- * receives the float32 [H,W,D] matching-cost volume P(class 0). */
+ * receives the float32 [H,W,D] matching-cost volume P(class 0); the post
+ * reads it there, so it stays valid, and is not written by other work, until
+ * `stream` has passed the call (two contexts in flight take two volumes). */
 int cbmv_run_rf(cbmv_ctx* c, const cbmv_forest* f, const cbmv_params* p, const uint8_t* L,
                 const uint8_t* R, int64_t H, int64_t W, int D, float* disp, float* prob0);
 
@@ -410,7 +412,8 @@ int cbmv_run_mlp_host(cbmv_ctx* c, const cbmv_mlp* m, const cbmv_params* p, cons
  * test.py:143-149, 341-449) on a given matching cost: cost float32 [H,W,D]
  * (low = good, e.g. a saved P(class 0) volume, main.py:56-67), the images L,
  * R uint8 [H,W] for the cross arms and SGM, disp float32 [H,W]; device
- * memory.  `cost` is not modified. */
+ * memory.  `cost` is not modified; it is read throughout the call, and stays
+ * valid and unchanged until `stream` has passed it. */
 int cbmv_run_post(cbmv_ctx* c, const cbmv_params* p, const uint8_t* L, const uint8_t* R, int64_t H,
                   int64_t W, int D, const float* cost, float* disp);
 
