@@ -642,7 +642,8 @@ constexpr int CD_X = 32, CD_Y = 16, CD_D = 8, CD_G = 4, CD_HALO = 5;
 
 // The relative arms of one pixel, packed without conversions (an arm below
 // 2^22 is read off its sum with 1.5 * 2^23); *odd: one of them is no whole
-// number, or too large for that.
+// number, or too large for that, or so far on the other side of its pixel
+// that an interval of two such arms may lie beyond what a byte holds.
 __device__ __forceinline__ uint32_t pack_whole_arms(const float* __restrict__ c, int64_t HW, int64_t o, int x, int y,
                                                     bool* odd) {
   constexpr float kMagic = 12582912.0f;
@@ -650,8 +651,9 @@ __device__ __forceinline__ uint32_t pack_whole_arms(const float* __restrict__ c,
 #pragma unroll
   for (int a = 0; a < 4; a++) {
     const float v = __ldg(c + a * HW + o), t = __fadd_rn(v, kMagic);
-    *odd |= !(__fsub_rn(t, kMagic) == v && fabsf(v) < 4194304.0f);
-    w |= (uint32_t)(clamp_i8(__float_as_int(t) - __float_as_int(kMagic) - (a < 2 ? x : y)) & 0xFF) << (8 * a);
+    const int rel = __float_as_int(t) - __float_as_int(kMagic) - (a < 2 ? x : y);
+    *odd |= !(__fsub_rn(t, kMagic) == v && fabsf(v) < 4194304.0f) || (a & 1 ? rel < -120 : rel > 120);
+    w |= (uint32_t)(clamp_i8(rel) & 0xFF) << (8 * a);
   }
   return w;
 }

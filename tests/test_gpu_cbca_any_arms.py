@@ -53,6 +53,29 @@ def _separable(lc, rc, v, direction):
 
 
 @pytest.mark.parametrize("direction", [-1, 1])
+@pytest.mark.parametrize("H,W,D,shift", [(9, 17, 5, 2), (7, 430, 2, 200), (310, 9, 2, 150)])
+def test_dhw_with_any_arms(gpu, H, W, D, shift, direction):
+    """The reference-order sums of [D,H,W] volumes; the supports of a shift of
+    150 pixels and more lie beyond the byte that holds a relative arm."""
+    from cbmv_b200 import _lib
+    from test_gpu_cbca_dhw import _reference
+    rng = np.random.default_rng(H + W)
+    y, x = np.mgrid[0:H, 0:W]
+    lo = np.clip(x + shift + rng.integers(-2, 3, (H, W)), 0, W - 1)
+    up = np.clip(y - shift + rng.integers(-2, 3, (H, W)), 0, H - 1)
+    lc, rc = (np.stack([lo - 1, np.minimum(lo + rng.integers(2, 7, (H, W)), W), up - 1,
+                        np.minimum(up + rng.integers(2, 7, (H, W)), H)]).astype(F) for _ in range(2))
+    v = rng.random((D, H, W)).astype(F)
+    with np.errstate(all="ignore"):
+        want = _reference(lc, rc, v, direction)
+    tl, tr, tv = (torch.from_numpy(a).cuda() for a in (lc, rc, v))
+    got = torch.empty_like(tv)
+    _lib.call("cbmv_cbca", tl.data_ptr(), tr.data_ptr(), tv.data_ptr(), H, W, D, _lib.DHW, direction, got.data_ptr(),
+              None)
+    assert np.array_equal(got.cpu().numpy(), want, equal_nan=True)
+
+
+@pytest.mark.parametrize("direction", [-1, 1])
 @pytest.mark.parametrize("H,W,D,shift", [(9, 17, 5, 1), (14, 35, 3, 3), (11, 40, 2, 9)])
 def test_separable_with_any_arms(gpu, H, W, D, shift, direction):
     from cbmv_b200 import _lib
