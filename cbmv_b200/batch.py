@@ -94,9 +94,10 @@ def tune_batch(shapes, net, lefts, rights, streams=CANDIDATE_STREAMS, mlp_ctas=(
     """Pick the batch's launch shape by timing it: the number of concurrent
     contexts and the classifier kernel's CTA cap (0 = every SM, None = the
     SM count divided by the number of contexts), then (tile_search) the
-    kernel tile shapes, one at a time from the best: rows per CBCA tile
-    (32, 16) and SGM prefetch depth (default, 1, 4).  None of these change
-    the results.  Each candidate is captured, run once untimed and `iters`
+    kernel tile shapes, one at a time from the best: rows per CBCA tile (at
+    most 32 or 16; small volumes take fewer either way) and SGM prefetch depth
+    (default, 1, 4; the scan has one depth, so these time the same launches).
+    None of these change the results.  Each candidate is captured, run once untimed and `iters`
     times timed (graph span, CUDA events); the fastest is cached per (GPU,
     batch shapes) in a JSON file.  Returns {"streams", "mlp_ctas",
     "cbca_rows", "sgm_prefetch", "ms", "tried": [...]}."""

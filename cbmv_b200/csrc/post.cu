@@ -1495,15 +1495,15 @@ int launch_cbca_mask_build(const uint32_t* wl, const uint32_t* wr, int64_t H, in
   return check_launch("cbca_mask_build");
 }
 
-// tile rows 16 or 32, 0: by the volume (the results do not depend on them)
+// at most 16 or 32 tile rows (0: 32), fewer where the volume is too small for
+// them to fill the GPU (the results do not depend on them)
 int launch_cbca_masked(const uint32_t* mask, const float* in, int64_t H, int64_t W, int D, float* out,
                        cudaStream_t st, int rows) {
   CBMV_REQUIRE(H < (1 << 30) && W < (1 << 30) &&
                    (int64_t)((W + CS_TX - 1) / CS_TX) * ((H + 15) / 16) * ((D + CS_TD - 1) / CS_TD) <
                        ((int64_t)1 << 31),
                CBMV_ERANGE, "cbca: volume too large");
-  if (rows == 0)
-    rows = cbca_tiles(H, W, D, 32) >= kCbcaFull ? 32 : cbca_tiles(H, W, D, 16) >= kCbcaFull ? 16 : 8;
+  rows = rows != 16 && cbca_tiles(H, W, D, 32) >= kCbcaFull ? 32 : cbca_tiles(H, W, D, 16) >= kCbcaFull ? 16 : 8;
   if (rows == 8) return launch_cbca_masked_t<8>(mask, in, H, W, D, out, st);
   if (rows == 16) return launch_cbca_masked_t<16>(mask, in, H, W, D, out, st);
   return launch_cbca_masked_t<32>(mask, in, H, W, D, out, st);

@@ -347,9 +347,10 @@ typedef struct cbmv_params {
    * (cbmv_batch). */
   int mlp_ctas;
   /* Launch shapes that do not change the results (picked by the batch
-   * autotuner): rows per CBCA tile, 16 or 32 (0 = by the volume's size); SGM
-   * steps loaded ahead, 0, 1, 2 or 4: no longer a choice (the scan's ring in shared
-   * memory has a depth fixed by the disparity count), still checked. */
+   * autotuner): rows per CBCA tile, at most 16 or 32 (0 = 32; a volume
+   * too small to fill the GPU with them takes fewer); SGM steps loaded
+   * ahead, 0, 1, 2 or 4: no longer a choice (the scan's ring in shared memory
+   * has a depth fixed by the disparity count), still checked. */
   int cbca_rows, sgm_prefetch;
   /* Post-processing chain, Testing.eval_prob's `interpolate` (main.py:70,
    * test.py:143-149): 0 (default) the _mem post (test.py:341-449); 1 the
