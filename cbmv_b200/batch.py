@@ -77,11 +77,14 @@ class StereoBatch:
 
 # ----------------------------------------------------------------- autotuner
 CANDIDATE_STREAMS = (1, 2, 4, 8)
+# raised when the kernels change what a launch shape costs: choices timed on
+# other kernels are not taken from the cache
+LAUNCH_SHAPES = 2
 
 
 def _signature(shapes):
     import torch
-    key = json.dumps([torch.cuda.get_device_name(), sorted(shapes)])
+    key = json.dumps([torch.cuda.get_device_name(), LAUNCH_SHAPES, sorted(shapes)])
     return hashlib.sha1(key.encode()).hexdigest()[:16]
 
 
@@ -99,7 +102,7 @@ def tune_batch(shapes, net, lefts, rights, streams=CANDIDATE_STREAMS, mlp_ctas=(
     (default, 1, 4; the scan has one depth, so these time the same launches).
     None of these change the results.  Each candidate is captured, run once untimed and `iters`
     times timed (graph span, CUDA events); the fastest is cached per (GPU,
-    batch shapes) in a JSON file.  Returns {"streams", "mlp_ctas",
+    kernels, batch shapes) in a JSON file.  Returns {"streams", "mlp_ctas",
     "cbca_rows", "sgm_prefetch", "ms", "tried": [...]}."""
     import torch
     shapes = [tuple(int(v) for v in s) for s in shapes]
