@@ -12,6 +12,7 @@ SO = os.path.join(HERE, "libcbmv.so")
 F32, F64 = 0, 1
 ACT_RELU, ACT_GELU = 0, 1
 HWD, DHW = 0, 1
+ECUDA = -2  # CBMV_ECUDA
 
 _i64 = ctypes.c_int64
 _int = ctypes.c_int

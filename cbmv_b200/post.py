@@ -79,7 +79,10 @@ def sgm(left, right, in_cost, out_cost, tmp, pi1, pi2, tau_so, alpha1, sgm_q1, s
     torch's caching allocator, on the stream the call runs on."""
     H, W, D = in_cost.ins
     need = _lib.lib().cbmv_sgm_scratch_bytes(H, W, D)
-    scratch = torch.empty(max(need, 16), dtype=torch.uint8, device="cuda")
+    try:
+        scratch = torch.empty(max(need, 16), dtype=torch.uint8, device="cuda")
+    except torch.OutOfMemoryError as e:  # as cbmv_sgm reports its own scratch
+        raise _lib.CbmvError("cbmv_sgm", _lib.ECUDA, str(e)) from e
     _lib.call("cbmv_sgm_scratch", left.ptr, right.ptr, in_cost.ptr, H, W, D, float(pi1), float(pi2),
               float(tau_so), float(alpha1), float(sgm_q1), float(sgm_q2), int(direction),
               out_cost.ptr, scratch.data_ptr(), _s())
