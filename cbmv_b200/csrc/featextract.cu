@@ -19,10 +19,9 @@ constexpr int kBlock = 256;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += (int64_t)gridDim.x * blockDim.x)
 
 // [rows, cols] -> [cols, rows] of float64 through 32 x 32 shared-memory
-// tiles, both sides coalesced: bound by its traffic (a thread per element
-// with one strided side took 400 us for the 49.2 M elements of a 694x554
-// D=128 volume, 787 MB; now 129 us).  Tiles are numbered along one grid axis: either
-// side may be H*W.
+// tiles, both sides coalesced: bound by its traffic (787 MB for a 694x554
+// D=128 volume).  Tiles are numbered along one grid axis: either side may be
+// H*W.
 __global__ void __launch_bounds__(256) transpose_f64_kernel(const double* __restrict__ in, int64_t rows, int64_t cols,
                                                             double* __restrict__ out) {
   __shared__ double tile[32][33];
@@ -41,10 +40,80 @@ __global__ void __launch_bounds__(256) transpose_f64_kernel(const double* __rest
   }
 }
 
-int launch_transpose_f64(const double* in, int64_t rows, int64_t cols, double* out, cudaStream_t st) {
-  const int64_t tiles = ((rows + 31) / 32) * ((cols + 31) / 32);
-  transpose_f64_kernel<<<(unsigned)(tiles < 1 << 30 ? tiles : 1 << 30), 256, 0, st>>>(in, rows, cols, out);
+// [D, H*W] -> [H*W, D] with the disparities of 32 pixels in one tile (64 of
+// them where D has more), so that a run of `out` is written by one CTA: with
+// D % 4 != 0 the runs of the 32 x 32 tiles share 32-byte sectors.
+constexpr int kSwapD = 64;
+
+__global__ void __launch_bounds__(256) swap_runs_kernel(const double* __restrict__ in, int64_t HW, int D, int dt,
+                                                      double* __restrict__ out) {
+  __shared__ double tile[kSwapD][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nd = (D + dt - 1) / dt;
+  const int64_t tiles = (HW + 31) / 32 * nd;
+  for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const int64_t p0 = t / nd * 32;
+    const int d0 = (int)(t % nd) * dt, n = min(dt, D - d0), np = (int)min((int64_t)32, HW - p0);
+    const double* src = in + (d0 + warp) * HW + p0 + lane;
+    if (lane < np) {
+#pragma unroll 8
+      for (int d = warp; d < n; d += 8, src += 8 * HW) tile[d][lane] = __ldg(src);
+    }
+    __syncthreads();
+    double* dst = out + (p0 + warp) * D + d0 + lane;
+#pragma unroll 4
+    for (int p = warp; p < np; p += 8, dst += 8 * (int64_t)D)
+#pragma unroll
+      for (int d = 0; d < kSwapD; d += 32)
+        if (d + lane < n) dst[d] = tile[d + lane][p];
+    __syncthreads();
+  }
+}
+
+// A few disparities fill no tile: [D, H*W] -> [H*W, D] with a thread per value
+// of `out`, and back with one per pixel.
+__global__ void swap_few_kernel(const double* __restrict__ in, int64_t HW, int D, double* __restrict__ out) {
+  GRID_STRIDE(t, D * HW) {
+    const int64_t p = t / D, d = t - p * D;
+    out[t] = in[d * HW + p];
+  }
+}
+__global__ void swap_back_few_kernel(const double* __restrict__ in, int64_t HW, int D, double* __restrict__ out) {
+  GRID_STRIDE(p, HW) {
+#pragma unroll 4
+    for (int d = 0; d < D; d++) out[d * HW + p] = __ldg(in + p * D + d);
+  }
+}
+
+static unsigned tile_grid(int64_t tiles) { return (unsigned)(tiles < 1 << 30 ? tiles : 1 << 30); }
+
+// us at 694x554: a few disparities' kernel, 32 x 32 tiles, whole runs
+//   D     swap_axes          swap_axes_back
+//     1     7 /  24            5 / 21
+//    12    20 /  25           15 / 23
+//    16    30 /  27
+//    33    56 /  59 /  52
+//    65   102 / 130 /  95
+//    97   253 / 196 / 134
+//   128   313 / 130 / 128
+// Whole runs pay where the volume leaves L2 (450x375 D=50, 67 MB: 38 / 29 /
+// 36; 1482x994 D=33, 389 MB: 307 / 230 / 179) and where the tiles' runs are
+// unaligned (D=36 at 694x554: 56 with tiles).
+int launch_swap_axes(const double* in, int64_t D, int64_t HW, double* out, cudaStream_t st) {
+  if (D < 15) {
+    swap_few_kernel<<<grid_for(D * HW, kBlock), kBlock, 0, st>>>(in, HW, (int)D, out);
+  } else if (D % 4 != 0 && D > 32 && D < (1 << 20) && D * HW >= 12500000) {  // 100 MB
+    const int64_t n = (D + kSwapD - 1) / kSwapD, dt = (D + n - 1) / n;
+    swap_runs_kernel<<<tile_grid((HW + 31) / 32 * n), 256, 0, st>>>(in, HW, (int)D, (int)dt, out);
+  } else {
+    transpose_f64_kernel<<<tile_grid(((D + 31) / 32) * ((HW + 31) / 32)), 256, 0, st>>>(in, D, HW, out);
+  }
   return check_launch("swap_axes");
+}
+
+int launch_swap_axes_back(const double* in, int64_t HW, int64_t D, double* out, cudaStream_t st) {
+  if (D < 14) swap_back_few_kernel<<<grid_for(HW, kBlock), kBlock, 0, st>>>(in, HW, (int)D, out);
+  else transpose_f64_kernel<<<tile_grid(((D + 31) / 32) * ((HW + 31) / 32)), 256, 0, st>>>(in, HW, D, out);
+  return check_launch("swap_axes_back");
 }
 
 __global__ void get_cost_kernel(const double* __restrict__ in, int64_t n, int64_t K,
@@ -755,14 +824,14 @@ extern "C" int cbmv_swap_axes(const double* in, int64_t D, int64_t H, int64_t W,
                               void* stream) {
   CHECK_VOL(in, out);
   CBMV_REQUIRE(D > 0 && H > 0 && W > 0, CBMV_EINVAL, "bad size");
-  return launch_transpose_f64(in, D, H * W, out, as_stream(stream));
+  return launch_swap_axes(in, D, H * W, out, as_stream(stream));
 }
 
 extern "C" int cbmv_swap_axes_back(const double* in, int64_t H, int64_t W, int64_t D, double* out,
                                    void* stream) {
   CHECK_VOL(in, out);
   CBMV_REQUIRE(D > 0 && H > 0 && W > 0, CBMV_EINVAL, "bad size");
-  return launch_transpose_f64(in, H * W, D, out, as_stream(stream));
+  return launch_swap_axes_back(in, H * W, D, out, as_stream(stream));
 }
 
 extern "C" int cbmv_get_cost(const double* in, int64_t H, int64_t W, int64_t D, int64_t K,
