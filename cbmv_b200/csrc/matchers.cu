@@ -572,6 +572,23 @@ static dim3 strip_grid(const StripArgs& a, int xs) {
   return dim3((unsigned)((units + kStripWarps - 1) / kStripWarps), (unsigned)a.H);
 }
 
+// A strip's lanes are disparities: below 32 of them its time stays what it is
+// at 32, and for a few the general kernels' thread per value is quicker; so it
+// is for NCC volumes that fill neither.  us, general against strip, the last
+// size of the general kernel and the next measured (census is quicker in
+// strips from D = 1 on):
+//   NCC        [H,W,D]  694x554 D=4   42 / 49     D=6   53 / 49
+//   NCC        [D,H,W]  694x554 D=10  71 / 68-74  D=12  82 / 69-74
+//   NCC                 320x240 D=6   22 / 24     D=8   25 / 24;  80x60 D=33 17 / 20
+//   SAD-Sobel           694x554 D=3   38 / 38-42  D=4   44 / 38-43
+//   ZSAD f64   [H,W,D]  694x554 D=10 100 / 114    D=12 116 / 114
+//   ZSAD f64   [D,H,W]  694x554 D=12 114 / 120    D=14 129 / 120
+static bool strip_is_quicker(int mode, int layout, int64_t H, int64_t W, int D) {
+  const bool hwd = layout == CBMV_HWD;
+  if (mode == kStripNcc && H * W * D <= 500000) return false;
+  return D > (mode == kStripNcc ? (hwd ? 5 : 10) : mode == kStripSadSob ? 3 : mode == kStripZsad ? (hwd ? 11 : 13) : 0);
+}
+
 template <int MODE, class T, int XS>
 static int launch_strip(const StripArgs& a, int layout, T* out, cudaStream_t st) {
   const dim3 grid = strip_grid(a, XS);
@@ -605,7 +622,7 @@ template <class T>
 int launch_ncc_cost(const uint8_t* L, const uint8_t* R, const uint32_t* Al, const uint32_t* Ar,
                     const double* Cl, const double* Cr, int64_t H, int64_t W, int D, int w,
                     int layout, T* out, cudaStream_t st) {
-  if (w == 3) {
+  if (w == 3 && strip_is_quicker(kStripNcc, layout, H, W, D)) {
     const StripArgs a{L, R, Al, Ar, Cl, Cr, nullptr, nullptr, H, W, D, w};
     return launch_strip<kStripNcc, T, 32>(a, layout, out, st);
   }
@@ -617,7 +634,7 @@ int launch_ncc_cost(const uint8_t* L, const uint8_t* R, const uint32_t* Al, cons
 template <class T>
 int launch_sadsob_cost(const int32_t* SL, const int32_t* SR, int64_t H, int64_t W, int D, int w,
                        int layout, T* out, cudaStream_t st) {
-  if (w == 5) {
+  if (w == 5 && strip_is_quicker(kStripSadSob, layout, H, W, D)) {
     const StripArgs a{SL, SR, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, H, W, D, w};
     return launch_strip<kStripSadSob, T, 32>(a, layout, out, st);
   }
@@ -647,7 +664,7 @@ static int launch_zsad_general(const uint8_t* L, const uint8_t* R, const double*
 template <class T>
 int launch_zsad_cost(const uint8_t* L, const uint8_t* R, const double* ml, const double* mr,
                      int64_t H, int64_t W, int D, int w, int layout, T* out, cudaStream_t st) {
-  if (w == 5 && std::is_same<T, double>::value) {
+  if (w == 5 && std::is_same<T, double>::value && strip_is_quicker(kStripZsad, layout, H, W, D)) {
     const StripArgs a{L, R, nullptr, nullptr, nullptr, nullptr, ml, mr, H, W, D, w};
     return launch_strip<kStripZsad, double, 16>(a, layout, reinterpret_cast<double*>(out), st);
   }
@@ -716,7 +733,7 @@ extern "C" int cbmv_ncc(const uint8_t* L, const uint8_t* R, int64_t H, int64_t W
   double* Cr = Cl + n;
   uint32_t* Al = (uint32_t*)(Cr + n);
   uint32_t* Ar = Al + n;
-  if (wsize == 3) {
+  if (wsize == 3 && strip_is_quicker(kStripNcc, layout, H, W, D)) {  // else two launches of the 9 values alone: 3 us less
     MatchTerms t{{L, R}};
     t.A[0] = Al, t.A[1] = Ar, t.C[0] = Cl, t.C[1] = Cr;
     rc = launch_match_terms(t, H, W, st);
