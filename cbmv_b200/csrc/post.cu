@@ -1446,7 +1446,12 @@ int launch_cbca(const float* lc, const float* rc, const float* in, int64_t H, in
     return check_launch("cbca_tiled");
   }
   const int64_t dhw_tiles = ((W + CD_X - 1) / CD_X) * ((H + CD_Y - 1) / CD_Y) * ((D + CD_D - 1) / CD_D);
-  if (layout == CBMV_DHW && H < (1 << 30) && W < (1 << 30) && dhw_tiles < ((int64_t)1 << 31)) {
+  // A tile takes 30 us however few the tiles are, and its warps are
+  // disparities.  us, a thread per output against tiles: 80x60 D=33 13 / 31;
+  // 320x240 D=9 34 / 39, D=11 40 / 39, D=16 57 / 41; 694x554 D=3 57 / 63, D=4
+  // 74 / 64; 1482x994 D=1 94 / 147, D=2 151 / 152.
+  const bool few = H * W * D <= 800000 || (D <= 3 && H * W * D <= 1500000);
+  if (layout == CBMV_DHW && !few && H < (1 << 30) && W < (1 << 30) && dhw_tiles < ((int64_t)1 << 31)) {
     cbca_dhw_kernel<<<(unsigned)dhw_tiles, 32 * CD_D, 0, st>>>(lc, rc, in, (int)H, (int)W, D, direction, out);
     return check_launch("cbca_dhw");
   }
