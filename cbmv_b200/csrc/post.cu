@@ -997,10 +997,12 @@ int launch_cbca_masked_t(const uint32_t* mask, const float* in, int64_t H, int64
 // Winner-take-all (first minimum, as np.argmin) and the subpixel parabola
 // (post.cu:453-483).  One warp per pixel on [H,W,D] volumes.
 // A warp takes four pixels at a time, so that their loads are in flight
-// together; lane l reads V consecutive disparities from V l on (V = 4 where D
-// and the volume's alignment allow it).  Bound by memory: 901x600 D=192 70 us
-// (128 one pixel at a time with single loads), 694x554 D=128 38 (58).
-template <int V>
+// together; lane l reads four consecutive disparities (V = 4, where D and the
+// volume's alignment allow it) or N single ones 32 apart, as many as a row of
+// up to 128 has.  Bound by memory.  us, one pixel at a time with single loads
+// against this: 901x600 D=192 128 / 70; 694x554 D=128 58 / 36, D=127 45 / 37
+// (50 with one single load per pixel), D=65 41 / 33, D=33 37 / 26.
+template <int V, int N>
 __global__ void __launch_bounds__(256) wta_subpixel_hwd_kernel(const float* __restrict__ c, int64_t HW, int D,
                                                                float* __restrict__ disp_int, float* __restrict__ disp) {
   constexpr int PX = 4;
@@ -1014,8 +1016,9 @@ __global__ void __launch_bounds__(256) wta_subpixel_hwd_kernel(const float* __re
     int bd[PX];
 #pragma unroll
     for (int k = 0; k < PX; k++) bv[k] = inf, bd[k] = 0x7fffffff;
-    for (int d = V * lane; d < D; d += 32 * V) {
-      float v[PX][V];
+    constexpr int S = V == 4 ? 1 : 32;  // between a lane's N disparities
+    for (int d = V * lane; d < D; d += 32 * N) {
+      float v[PX][N];
 #pragma unroll
       for (int k = 0; k < PX; k++) {
         const float* r = c + (p0 + (k < n ? k : 0)) * D + d;
@@ -1023,14 +1026,15 @@ __global__ void __launch_bounds__(256) wta_subpixel_hwd_kernel(const float* __re
           const float4 q = __ldg(reinterpret_cast<const float4*>(r));
           v[k][0] = q.x, v[k][1] = q.y, v[k][2] = q.z, v[k][3] = q.w;
         } else {
-          v[k][0] = __ldg(r);
+#pragma unroll
+          for (int i = 0; i < N; i++) v[k][i] = i == 0 || d + S * i < D ? __ldg(r + S * i) : inf;
         }
       }
 #pragma unroll
       for (int k = 0; k < PX; k++)
 #pragma unroll
-        for (int i = 0; i < V; i++)
-          if (v[k][i] < bv[k]) { bv[k] = v[k][i]; bd[k] = d + i; }
+        for (int i = 0; i < N; i++)
+          if (v[k][i] < bv[k]) { bv[k] = v[k][i]; bd[k] = d + S * i; }
     }
     // the lowest d among the lanes that hold the warp's minimum; lane k keeps pixel k's
     int mine = 0;
@@ -1516,10 +1520,11 @@ int launch_cbca_masked(const uint32_t* mask, const float* in, int64_t H, int64_t
 
 int launch_wta_subpixel(const float* cost, int64_t H, int64_t W, int D, float* disp_int,
                         float* disp, cudaStream_t st) {
-  if (D % 4 == 0 && (uintptr_t)cost % 16 == 0)
-    wta_subpixel_hwd_kernel<4><<<grid_for((H * W + 3) / 4 * 32, 256), 256, 0, st>>>(cost, H * W, D, disp_int, disp);
-  else
-    wta_subpixel_hwd_kernel<1><<<grid_for((H * W + 3) / 4 * 32, 256), 256, 0, st>>>(cost, H * W, D, disp_int, disp);
+  const unsigned grid = grid_for((H * W + 3) / 4 * 32, 256);
+  if (D % 4 == 0 && (uintptr_t)cost % 16 == 0) wta_subpixel_hwd_kernel<4, 4><<<grid, 256, 0, st>>>(cost, H * W, D, disp_int, disp);
+  else if (D <= 32) wta_subpixel_hwd_kernel<1, 1><<<grid, 256, 0, st>>>(cost, H * W, D, disp_int, disp);
+  else if (D <= 64) wta_subpixel_hwd_kernel<1, 2><<<grid, 256, 0, st>>>(cost, H * W, D, disp_int, disp);
+  else wta_subpixel_hwd_kernel<1, 4><<<grid, 256, 0, st>>>(cost, H * W, D, disp_int, disp);
   return check_launch("wta_subpixel");
 }
 
