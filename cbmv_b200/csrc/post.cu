@@ -640,18 +640,21 @@ __device__ __forceinline__ int rel_arm(uint32_t w) {
 // reads and masks each row of its tile once (eleven taps, those outside the
 // interval as 0: adding 0 changes no sum) and adds the eleven values to the
 // running sum of every one of four output rows whose support has the row --
-// the rows ascend, so each sum runs in the reference's order.  A support
-// that reaches beyond five pixels (cross arms of L1 > 6) is summed by
-// cbca_one.  Bound by instruction issue (the masks of a row are formed for
+// the rows ascend, so each sum runs in the reference's order.  Bound by instruction issue (the masks of a row are formed for
 // every four outputs, 14 rows; eight outputs at once need 79 registers and
-// were slower, 613 us).  694x320 D=128: 533 us a pass, 1380 us with a
+// were slower, 613 us).  694x554 D=128: 800 us a pass, 2420 us with a
 // thread per output walking its support (cbca_kernel).
+// A tile whose arms may reach beyond the taps (cross arms of L1 > 6), or are
+// no whole numbers, is left to cbca_dhw_left_kernel.
 constexpr int CD_X = 32, CD_Y = 16, CD_D = 8, CD_G = 4, CD_HALO = 5;
+constexpr int CD_LEFT = 24;  // at most, blocks of cbca_dhw_left_kernel per SM
+constexpr uint32_t kCbcaLeft = 0x7FA5C3E1u;  // the mark of a run that is left, its first value: a NaN that no sum gives
 
 // The relative arms of one pixel, packed without conversions (an arm below
 // 2^22 is read off its sum with 1.5 * 2^23); *odd: one of them is no whole
-// number, or too large for that, or so far on the other side of its pixel
-// that an interval of two such arms may lie beyond what a byte holds.
+// number, or too large for that, or reaches beyond the taps, or lies so far
+// on the other side of its pixel that an interval of two such arms may lie
+// beyond what a byte holds.
 __device__ __forceinline__ uint32_t pack_whole_arms(const float* __restrict__ c, int64_t HW, int64_t o, int x, int y,
                                                     bool* odd) {
   constexpr float kMagic = 12582912.0f;
@@ -660,7 +663,7 @@ __device__ __forceinline__ uint32_t pack_whole_arms(const float* __restrict__ c,
   for (int a = 0; a < 4; a++) {
     const float v = __ldg(c + a * HW + o), t = __fadd_rn(v, kMagic);
     const int rel = __float_as_int(t) - __float_as_int(kMagic) - (a < 2 ? x : y);
-    *odd |= !(__fsub_rn(t, kMagic) == v && fabsf(v) < 4194304.0f) || (a & 1 ? rel < -120 : rel > 120);
+    *odd |= !(__fsub_rn(t, kMagic) == v && fabsf(v) < 4194304.0f) || (a & 1 ? rel < -120 || rel > CD_HALO + 1 : rel > 120 || rel < -CD_HALO - 1);
     w |= (uint32_t)(clamp_i8(rel) & 0xFF) << (8 * a);
   }
   return w;
@@ -685,18 +688,30 @@ __global__ void __launch_bounds__(32 * CD_D) cbca_dhw_kernel(const float* __rest
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t HW = (int64_t)H * W;
   const int xm_lo = direction > 0 ? X0 + D0 : X0 - (D0 + CD_D - 1);
-  bool odd = false;  // an arm that is no whole number: the sums are left to cbca_one
+  bool odd = false;
+  auto leave = [&]() {  // whether the tile is cbca_dhw_left_kernel's; its runs are marked then
+    if (!__syncthreads_or(odd)) return false;
+    if (lane < CD_Y && Y0 + lane < H && D0 + warp < D)
+      out[(int64_t)(D0 + warp) * HW + (int64_t)(Y0 + lane) * W + X0] = __uint_as_float(kCbcaLeft);
+    return true;
+  };
   for (int r = warp; r < SR; r += CD_D) {
     const int yy = Y0 - CD_HALO + r;
     const bool rok = yy >= 0 && yy < H;  // outside the image: an empty interval
     const int64_t o = (int64_t)yy * W;
     sAL[r][lane] = rok && X0 + lane < W ? pack_whole_arms(lc, HW, o + X0 + lane, X0 + lane, yy, &odd) : 0u;
+  }
+  if (leave()) return;
+  for (int r = warp; r < SR; r += CD_D) {
+    const int yy = Y0 - CD_HALO + r;
+    const bool rok = yy >= 0 && yy < H;
+    const int64_t o = (int64_t)yy * W;
     for (int j = lane; j < NXM; j += 32) {
       const int xm = xm_lo + j;
       sAR[r][j] = rok && xm >= 0 && xm < W ? pack_whole_arms(rc, HW, o + xm, xm, yy, &odd) : 0u;
     }
   }
-  odd = __syncthreads_or(odd);
+  if (leave()) return;
   const int x = X0 + lane;
   float(*tile)[SX] = tiles[warp];
   const int xa = X0 - CD_HALO + lane, xb = xa + 32;
@@ -719,8 +734,7 @@ __global__ void __launch_bounds__(32 * CD_D) cbca_dhw_kernel(const float* __rest
   float* dst = out + (int64_t)d * HW + x;
 #pragma unroll 1
   for (int g = 0; g < CD_Y && Y0 + g < H; g += CD_G) {
-    // the rows of every output's support as taps; its sum; its pixels, and from bit 16 up the
-    // rows (or the support itself) that reach beyond the taps
+    // the rows of every output's support as taps; its sum; its pixels
     uint32_t vm[CD_G];
     float sum[CD_G];
     int cnt[CD_G];
@@ -729,7 +743,7 @@ __global__ void __launch_bounds__(32 * CD_D) cbca_dhw_kernel(const float* __rest
       const uint32_t wl = sAL[g + j + CD_HALO][lane], wr = sAR[g + j + CD_HALO][jr];
       const int lo = max(rel_arm<2>(wl), rel_arm<2>(wr)) + 1, hi = min(rel_arm<3>(wl), rel_arm<3>(wr)) - 1;
       vm[j] = tap_mask(lo, hi);
-      cnt[j] = odd || (hi >= lo && (lo < -CD_HALO || hi > CD_HALO)) ? 1 << 16 : 0;
+      cnt[j] = 0;
       sum[j] = 0.0f;
     }
 #pragma unroll
@@ -737,8 +751,7 @@ __global__ void __launch_bounds__(32 * CD_D) cbca_dhw_kernel(const float* __rest
       const uint32_t wl = sAL[g + r][lane], wr = sAR[g + r][jr];
       const int lo = max(rel_arm<0>(wl), rel_arm<0>(wr)) + 1, hi = min(rel_arm<1>(wl), rel_arm<1>(wr)) - 1;
       const uint32_t hm = tap_mask(lo, hi);
-      int len = hi - lo + 1;
-      len = len <= 0 ? 0 : lo < -CD_HALO || hi > CD_HALO ? 1 << 16 : len;
+      const int len = max(hi - lo + 1, 0);
       float v[NT];
 #pragma unroll
       for (int k = 0; k < NT; k++) {
@@ -757,9 +770,35 @@ __global__ void __launch_bounds__(32 * CD_D) cbca_dhw_kernel(const float* __rest
     for (int j = 0; j < CD_G; j++) {
       const int y = Y0 + g + j;
       if (y >= H) break;
-      float v = match ? sum[j] / (float)cnt[j] : tile[g + j + CD_HALO][lane + CD_HALO];
-      if (match && cnt[j] >= 1 << 16) v = cbca_one(lc, rc, in, H, W, D, CBMV_DHW, direction, y, x, d);
-      dst[(int64_t)y * W] = v;
+      dst[(int64_t)y * W] = match ? sum[j] / (float)cnt[j] : tile[g + j + CD_HALO][lane + CD_HALO];
+    }
+  }
+}
+
+// The runs of up to 32 outputs that cbca_dhw_kernel left, by cbca_one: a warp
+// reads the marks of 32 runs at once and walks those that are marked.  A mark
+// may also be the bits of a result: that run is formed again, to the same
+// values.  Bound by the latency of the supports' loads, so what counts is
+// that every output has a thread and runs of large supports are spread over
+// the SMs: with the long supports summed by the tiles' own warps, 16 outputs
+// one after the other, beside the taps of the others, L1=9 took at 694x554
+// D=128 3390 us (cbca_kernel alone 2840, now 2440), at 320x240 D=16 262 (82,
+// 81).  Launched beside the tiles' last wave (programmatic launch) its
+// blocks keep the tiles' split of L1 and shared memory: 3570 us.  Where no run is
+// marked the launch takes 2 to 4 us.
+__global__ void __launch_bounds__(256) cbca_dhw_left_kernel(const float* __restrict__ lc, const float* __restrict__ rc,
+                                                          const float* __restrict__ in, int H, int W, int D,
+                                                          int direction, float* out) {
+  const int ntx = (W + CD_X - 1) / CD_X, lane = threadIdx.x & 31;
+  const int64_t runs = (int64_t)ntx * H * D, nw = (int64_t)gridDim.x * 8, w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  for (int64_t r0 = w; r0 < runs; r0 += 32 * nw) {
+    const int64_t r = r0 + lane * nw, row = r / ntx;
+    const bool left = r < runs && __float_as_uint(out[row * W + (r - row * ntx) * CD_X]) == kCbcaLeft;
+    uint32_t marked = __ballot_sync(0xffffffffu, left);
+    for (; marked; marked &= marked - 1) {
+      const int64_t q = r0 + (__ffs(marked) - 1) * nw, qrow = q / ntx;  // row qrow % H of disparity qrow / H
+      const int d = (int)(qrow / H), y = (int)(qrow - (int64_t)d * H), x = (int)(q - qrow * ntx) * CD_X + lane;
+      if (x < W) out[qrow * W + x] = cbca_one(lc, rc, in, H, W, D, CBMV_DHW, direction, y, x, d);
     }
   }
 }
@@ -1465,7 +1504,15 @@ int launch_cbca(const float* lc, const float* rc, const float* in, int64_t H, in
   const bool few = H * W * D <= 800000 || (D <= 3 && H * W * D <= 1500000);
   if (layout == CBMV_DHW && !few && H < (1 << 30) && W < (1 << 30) && dhw_tiles < ((int64_t)1 << 31)) {
     cbca_dhw_kernel<<<(unsigned)dhw_tiles, 32 * CD_D, 0, st>>>(lc, rc, in, (int)H, (int)W, D, direction, out);
-    return check_launch("cbca_dhw");
+    if (const int rc_ = check_launch("cbca_dhw")) return rc_;
+    int dev = 0, sms = 0;
+    CBMV_CUDA(cudaGetDevice(&dev));
+    CBMV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // two runs per warp at least: an empty launch costs by its blocks (320x240 D=16, a pass with
+    // arms of L1 = 6 and 9: a run per warp 44.5 and 80 us, two 43.4 and 91, three 42.2 and 93)
+    const int64_t need = ((W + CD_X - 1) / CD_X * H * D + 15) / 16, blocks = (int64_t)sms * CD_LEFT;
+    cbca_dhw_left_kernel<<<(unsigned)(need < blocks ? need : blocks), 256, 0, st>>>(lc, rc, in, (int)H, (int)W, D, direction, out);
+    return check_launch("cbca_dhw_left");
   }
   cbca_kernel<<<grid_for(H * W * D, kBlock), kBlock, 0, st>>>(lc, rc, in, H, W, D, layout, direction,
                                                              out);
