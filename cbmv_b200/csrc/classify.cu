@@ -17,7 +17,7 @@
 //  - 48 warps per SM with two trees each in flight hide the L2 latency of
 //    the lower levels; the leaf values are added in tree order, as
 //    predict_proba does.
-// 694x554 D=128, 50 trees: 33.2 ms (67.3 ms with 32-byte blocks, 16 warps,
+// 694x554 D=128, 50 trees: 32.6 ms (67.3 ms with 32-byte blocks, 16 warps,
 // four trees each).  Measured beside it: 32 warps 34.6-36.9 ms, one or four
 // trees in flight 34.1-35.6, other warp shapes 32.8-34.1.
 #include "common.cuh"

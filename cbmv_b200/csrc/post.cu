@@ -119,9 +119,10 @@ __global__ void __launch_bounds__(128) sgm_codes_kernel(const float* __restrict_
 // the scan waited for them (380 to 450 us per launch at 694x554 D=128
 // against 240 without any).
 // Per launch, us (before: loads in registers, float differences, lanes
-// strided by 32 where D % 4 != 0): 694x554 D=128 242 (382), at 5.9 TB/s of
-// its 1.42 GB; 451x319 D=70 98 (262); 901x600 D=192 554 (990); 1482x994
-// D=256 1990 (2673).  A ring of eight steps, blocks of 4 to 16 lines, and a
+// strided by 32 where D % 4 != 0): 694x554 D=128 240 (382), at 5.9 TB/s of
+// its 1.42 GB; 451x319 D=70 98 (262); 901x600 D=192 558 (990); 1482x994
+// D=256 1923 (2673).  A whole post with two of them, ms: 694x554 D=400 6.7
+// (9.9), D=512 7.7 (11.2), D=694 10.7 (17.8), 1482x994 D=400 24.2 (36.6).  A ring of eight steps, blocks of 4 to 16 lines, and a
 // cap on registers for more resident lines changed nothing; two steps lose
 // 60 us at D=128.
 template <int KPL>
@@ -783,9 +784,10 @@ __global__ void __launch_bounds__(32 * CD_D) cbca_dhw_kernel(const float* __rest
 // the SMs: with the long supports summed by the tiles' own warps, 16 outputs
 // one after the other, beside the taps of the others, L1=9 took at 694x554
 // D=128 3390 us (cbca_kernel alone 2840, now 2440), at 320x240 D=16 262 (82,
-// 81).  Launched beside the tiles' last wave (programmatic launch) its
+// 91).  Launched beside the tiles' last wave (programmatic launch) its
 // blocks keep the tiles' split of L1 and shared memory: 3570 us.  Where no run is
-// marked the launch takes 2 to 4 us.
+// marked the launch takes 2 us at 320x240 D=16 and 19 at 694x320 D=128, for
+// the marks' sectors.
 __global__ void __launch_bounds__(256) cbca_dhw_left_kernel(const float* __restrict__ lc, const float* __restrict__ rc,
                                                           const float* __restrict__ in, int H, int W, int D,
                                                           int direction, float* out) {
