@@ -641,10 +641,11 @@ __device__ __forceinline__ int rel_arm(uint32_t w) {
 // reads and masks each row of its tile once (eleven taps, those outside the
 // interval as 0: adding 0 changes no sum) and adds the eleven values to the
 // running sum of every one of four output rows whose support has the row --
-// the rows ascend, so each sum runs in the reference's order.  Bound by instruction issue (the masks of a row are formed for
-// every four outputs, 14 rows; eight outputs at once need 79 registers and
-// were slower, 613 us).  694x554 D=128: 800 us a pass, 2420 us with a
-// thread per output walking its support (cbca_kernel).
+// the rows ascend, so each sum runs in the reference's order.  Bound by
+// instruction issue (the masks of a row are formed for every four outputs, 14
+// rows; eight outputs at once need 79 registers: 613 us where four took 533).
+// Now 694x320 D=128 458 us, 694x554 800; with a thread per output walking its
+// support (cbca_kernel) 1380 and 2420.
 // A tile whose arms may reach beyond the taps (cross arms of L1 > 6), or are
 // no whole numbers, is left to cbca_dhw_left_kernel.
 constexpr int CD_X = 32, CD_Y = 16, CD_D = 8, CD_G = 4, CD_HALO = 5;
